@@ -40,7 +40,7 @@ int fail(int code, const char* fmt, ...) {
   } while (0)
 
 // reference physics constants (src/config.c:82-90)
-constexpr double kGamma = 5.0 / 3.0, kCfl = 0.3, kCa = 10.0, kPdmb = 1.0;
+constexpr double kGamma = 5.0 / 3.0, kCfl = 0.3, kCa = 10.0;
 constexpr double kRhoFloor = 0.00316227, kPFloor = 0.000316227;
 
 // Dense 5x5 LU with partial pivoting and solve (the scheme of
@@ -185,7 +185,7 @@ void build_tables(const gop_desc& d, Tables& T) {
     if (a == 1) return -(std::cos(xs[1][f + 1]) - std::cos(xs[1][f]));
     return dxv[2][f];
   };
-  const double e = 1.0 / (2 * kPdmb + 1.0);
+  const double e = 1.0 / (2 * PDMB + 1.0);
   static const double fac[7] = {-1.0 / 140.0, 5.0 / 84.0, -101.0 / 420.0, 319.0 / 420.0,
                                 107.0 / 210.0, -19.0 / 210.0, 1.0 / 105.0};
   static const double f8[8] = {-3.0 / 840, 29.0 / 840, -139.0 / 840, 533.0 / 840,
@@ -532,8 +532,6 @@ int gop_create(const gop_desc* desc, gop_instance** out) {
   P.ca2 = d.ca * d.ca;
   P.rho_floor = d.rho_floor;
   P.p_floor = d.p_floor;
-  P.pdm_a1 = kPdmb / (kPdmb + 1.0);
-  P.pdm_a2 = 1.0 - P.pdm_a1;
   P.inv_gm1 = 1.0 / P.gm1;
   P.q_ca = 0.25 / d.ca;
 

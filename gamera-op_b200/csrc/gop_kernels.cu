@@ -283,7 +283,6 @@ __device__ __forceinline__ void c2c_body(const Params& P, const Work<R>& wk, Pos
   const R* __restrict__ W = lim_w<R>(P, wk) + x;
   FaceWeights<R> Wt;
   load_face_weights<p, R>(wk.tab, wk.fw, P.tmax, f, Wt);
-  const R a1h = (R)(0.5 * P.pdm_a1), a2 = (R)P.pdm_a2;
 #pragma unroll
   for (int cc = 0; cc < 2; cc++) {
     const int comp = cc == 0 ? p : q;
@@ -291,7 +290,7 @@ __device__ __forceinline__ void c2c_body(const Params& P, const Work<R>& wk, Pos
     line8<R, R>(wk.Wh + (size_t)(V1 + comp) * fs + x, s, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = W[(V1 + comp) * fs + (u - 2) * s];
-    recon_lr<R>(v, lim, Wt, a1h, a2, L, Rr);
+    recon_lr(v, lim, Wt, L, Rr);
     wk.V[x + (size_t)(2 * D + cc) * fs] = R(0.5) * (L + Rr);
   }
 }
@@ -312,7 +311,6 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
   const long long x = lin(P, i, j, k), sp = sd<p>(P), sq = sd<q>(P);
   const size_t fs = P.fs;
   const R* __restrict__ B = lim_b<R>(P, wk) + x;
-  const R a1h = (R)(0.5 * P.pdm_a1), a2 = (R)P.pdm_a2;
   R vav[2], bpl, bpr, bql, bqr;
   {
     FaceWeights<R> Wt;
@@ -323,7 +321,7 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
       line8<R, R>(wk.V + (size_t)(2 * D + cc) * fs + x, sq, v);
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = v[u + 2];
-      recon_lr<R>(v, lim, Wt, a1h, a2, L, Rr);
+      recon_lr(v, lim, Wt, L, Rr);
       vav[cc] = R(0.5) * (L + Rr);
     }
     // B_p along q
@@ -331,7 +329,7 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
     line8<R, R>(wk.Bh + (size_t)p * fs + x, sq, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = B[p * fs + (u - 2) * sq];
-    recon_lr<R>(v, lim, Wt, a1h, a2, bpl, bpr);
+    recon_lr(v, lim, Wt, bpl, bpr);
   }
   {
     // B_q along p
@@ -341,7 +339,7 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
     line8<R, R>(wk.Bh + (size_t)q * fs + x, sp, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = B[q * fs + (u - 2) * sp];
-    recon_lr<R>(v, lim, Wt, a1h, a2, bql, bqr);
+    recon_lr(v, lim, Wt, bql, bqr);
   }
   R b0p = R(0), b0q = R(0);
   if constexpr (BG) {  // B0 averaged along the edge (B0Aedge*)
@@ -373,7 +371,6 @@ __device__ __forceinline__ void flux_body(const Params& P, const Work<R>& wk, Po
   const R* __restrict__ W = lim_w<R>(P, wk) + x;
   FaceWeights<R> Wt;
   load_face_weights<D, R>(wk.tab, wk.fw, P.tmax, f, Wt);
-  const R a1h = (R)(0.5 * P.pdm_a1), a2 = (R)P.pdm_a2;
   R L[6], Rt[6], mL[3], mR[3];
   // PSL false: p_S is identically zero (Params::ps_live), its face states
   // are zero and flux_out's zero path gives the zero entropy flux that
@@ -386,7 +383,7 @@ __device__ __forceinline__ void flux_body(const Params& P, const Work<R>& wk, Po
     line8<R, R>(wk.Wh + (size_t)m * fs + x, s, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = W[m * fs + (u - 2) * s];
-    recon_lr<R>(v, lim, Wt, a1h, a2, L[m], Rt[m]);
+    recon_lr(v, lim, Wt, L[m], Rt[m]);
   }
 #pragma unroll
   for (int a = 0; a < 3; a++) {
@@ -395,7 +392,7 @@ __device__ __forceinline__ void flux_body(const Params& P, const Work<R>& wk, Po
     const R* ms = wk.Ms + (size_t)a * fs + x;
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = ms[(u - 2) * s];
-    recon_lr<R>(v, lim, Wt, a1h, a2, mL[a], mR[a]);
+    recon_lr(v, lim, Wt, mL[a], mR[a]);
   }
   flux_out<R, D, BG, PSL>(P, wk, x, L, Rt, mL, mR, lim_b<R>(P, wk)[x + D * fs]);
 }

@@ -144,10 +144,7 @@ __device__ __forceinline__ void load_tap(const R* w, FaceWeights<R>& W) {
     W.wl[u] = w[u * X];
     W.wr[u] = w[(7 + u) * X];
   }
-  W.cl1 = w[14 * X];
-  W.cl2 = w[15 * X];
-  W.cr1 = w[16 * X];
-  W.cr2 = w[17 * X];
+  W.set_limiter(w[14 * X], w[15 * X], w[16 * X], w[17 * X]);
 }
 
 // ------------------------------------------------------------------ flux
@@ -279,7 +276,6 @@ struct FluxStage {
     if constexpr (D == 0) load_tap<32>(s + F::OFF_W + col, Wt);
     else load_fw_smem(s + F::OFF_W + row * FW, Wt);
     const R bn = s[F::OFF_BN + row * F::BN.x + col];
-    const R a1h = (R)(0.5 * P.pdm_a1), a2 = (R)P.pdm_a2;
     R L[6], Rt[6], mL[3], mR[3];
     L[PS] = Rt[PS] = R(0);
 #pragma unroll
@@ -289,7 +285,7 @@ struct FluxStage {
       for (int u = 0; u < 8; u++) v[u] = wh[f * F::SB + u * TS];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = wl[f * F::LB + u * TS];
-      recon_lr<R>(v, lim, Wt, a1h, a2, L[f], Rt[f]);
+      recon_lr(v, lim, Wt, L[f], Rt[f]);
     }
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -298,7 +294,7 @@ struct FluxStage {
       for (int u = 0; u < 8; u++) v[u] = msh[a * F::SB + u * TS];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = ms[a * F::LB + u * TS];
-      recon_lr<R>(v, lim, Wt, a1h, a2, mL[a], mR[a]);
+      recon_lr(v, lim, Wt, mL[a], mR[a]);
     }
     flux_out<R, D, BG, false>(P, wk, lin(P, i, j, k), L, Rt, mL, mR, bn);
   }
@@ -431,7 +427,6 @@ struct EmfStage {
     const int i = T.x0 + lane, j = T.y0 + (D == 2 ? warp : 0), k = T.z0 + (D == 2 ? 0 : warp);
     if (!(i < NGH + P.n[0] + (D != 0) && j < NGH + P.n[1] + (D != 1) && k < NGH + P.n[2] + (D != 2)))
       return;
-    const R a1h = (R)(0.5 * P.pdm_a1), a2 = (R)P.pdm_a2;
     // stencil bases and tap strides of the windows along q and along p (the
     // boxes whose rows run along i on i faces are 40 wide)
     const R *v0, *bp, *bpl, *bq, *bql;
@@ -483,7 +478,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = v0[cc * E::VF + u * tq];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = v[u + 2];
-      recon_lr<R>(v, lim, Wq, a1h, a2, L, Rr);
+      recon_lr(v, lim, Wq, L, Rr);
       vav[cc] = R(0.5) * (L + Rr);
     }
     {  // B_p along q
@@ -492,7 +487,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = bp[u * tq];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = bpl[u * tq];
-      recon_lr<R>(v, lim, Wq, a1h, a2, bpL, bpR);
+      recon_lr(v, lim, Wq, bpL, bpR);
     }
     {  // B_q along p
       R v[8], lim[4];
@@ -500,7 +495,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = bq[u * tp];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = bql[u * tp];
-      recon_lr<R>(v, lim, Wp, a1h, a2, bqL, bqR);
+      recon_lr(v, lim, Wp, bqL, bqR);
     }
     const long long x = lin(P, i, j, k);
     const size_t fs = P.fs;

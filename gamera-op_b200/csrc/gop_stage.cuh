@@ -31,10 +31,12 @@ __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double max2(double a, double b) { return a > b || b != b ? a : b; }
 
 // sqrt(n / d) for d > 0 as n rsqrt(n d): one special function where the
-// division and the root take two of about 25 instructions each
+// division and the root take two of about 25 instructions each.  Not a number
+// for n or d below zero (a negative density, say), both included.
 __device__ __forceinline__ double sqrt_ratio(double n, double d) {
   const double r = n * rsqrt(n * d);
-  return n == 0.0 ? 0.0 : r;
+  const int nan_bits = (__double2hiint(d) >> 31) & 0x7ff80000;
+  return n == 0.0 ? 0.0 : __hiloint2double(__double2hiint(r) | nan_bits, __double2loint(r));
 }
 
 // Fast magnetosonic speed sqrt(cs^2 + va^2) with the Boris-limited Alfven

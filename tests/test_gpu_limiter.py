@@ -71,3 +71,24 @@ def test_ties_match_the_checker(oracle_mod, n, coord, sweep):
             s = list(act)
             s[c] = slice(NG, NG + n[c] + 1)
             assert rel_l1(d["face_b"][c][tuple(s)], r["B"][c][tuple(s)]) <= TOL, f"B{c}"
+
+
+@pytest.mark.parametrize("b", [0.0, 5.0, 30.0])
+def test_negative_density_is_reported(b):
+    """Faces between cells of negative density have no signal speed, however
+    strong the field (b^2 below and above ca^2 |rho|): the step reports it."""
+    import gop
+
+    n = (16, 12, 8)
+    xs = [gop.grid_uniform(m, 0.0, 1.0) for m in n]
+    N = tuple(m + 2 * NG + 1 for m in n)
+    W, B = np.zeros((6,) + N), np.zeros((3,) + N)
+    W[0], W[4], B[0] = 1.0, 1.0, b
+    W[0, NG + 4:NG + 8, NG + 4:NG + 8, NG + 2:NG + 6] = -1.0
+    inst = gop.Instance(n, *xs)
+    inst.upload(W, B)
+    inst.prepare()
+    with pytest.raises(gop.GopError) as e:
+        inst.step(2)
+    assert e.value.code == -34
+    inst.close()

@@ -374,6 +374,8 @@ struct gop_instance {
   Params P;
   cudaStream_t own = nullptr;  // the instance's own non-blocking stream
   cudaStream_t st = nullptr;   // where its work goes (own, or the caller's)
+  cudaStream_t copy = nullptr; // host copies of gop_upload and gop_download (made at first use)
+  cudaEvent_t field_ev[6] = {};  // the last use of each staging slot
   double* state = nullptr;   // 2 x (6 + 3) fields
   void* work = nullptr;      // WORK_FIELDS x R
   double* tab = nullptr;
@@ -405,6 +407,77 @@ struct gop_instance {
   double prof_ms[NGROUP] = {};
   int64_t prof_n[NGROUP] = {};
 };
+
+// Fields travel through the staging buffer's six slots.  Large ones are copied
+// one by one on a stream of their own, beside the layout kernels of the others
+// (one copy of all fields before or behind the kernels leaves the link idle
+// meanwhile); below kFieldBytes a field the events cost more than that gains.
+// Download to pinned memory on B200, one copy / field by field: 64^3 (3 MB a
+// field) 568 / 577 us, 128^3 (20 MB) 3.47 / 3.35 ms, 256^3 25.5 / 23.6 ms.
+constexpr size_t kFieldBytes = 8 << 20;
+static int copy_stream(gop_instance* h) {
+  if (h->copy) return GOP_OK;
+  for (cudaEvent_t& e : h->field_ev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  CK(cudaStreamCreateWithFlags(&h->copy, cudaStreamNonBlocking));
+  return GOP_OK;
+}
+// nf <= 6 fields from the host; ends with the kernels enqueued on h->st
+static int upload_fields(gop_instance* h, int nf, const double* host, double* dev) {
+  const Params& P = h->P;
+  const size_t ref = (size_t)P.N[0] * P.N[1] * P.N[2], bytes = ref * sizeof(double);
+  const bool single = bytes < kFieldBytes;
+  if (single) {
+    CK(cudaMemcpyAsync(h->staging, host, nf * bytes, cudaMemcpyHostToDevice, h->st));
+  } else {
+    const int rc = copy_stream(h);
+    if (rc) return rc;
+  }
+  for (int f = 0; f < nf; f++) {
+    double* slot = h->staging + f * ref;
+    if (!single) {
+      CK(cudaStreamWaitEvent(h->copy, h->field_ev[f], 0));
+      CK(cudaMemcpyAsync(slot, host + f * ref, bytes, cudaMemcpyHostToDevice, h->copy));
+      CK(cudaEventRecord(h->field_ev[f], h->copy));
+      CK(cudaStreamWaitEvent(h->st, h->field_ev[f], 0));
+    }
+    launch_from_ref(P, slot, dev + (size_t)f * P.fs, h->st);
+    if (!single) CK(cudaEventRecord(h->field_ev[f], h->st));
+  }
+  return GOP_OK;
+}
+// nf <= 6 fields to the host; ends with the copies enqueued (wait_fields)
+static int download_fields(gop_instance* h, int nf, const double* dev, double* host) {
+  const Params& P = h->P;
+  const size_t ref = (size_t)P.N[0] * P.N[1] * P.N[2], bytes = ref * sizeof(double);
+  const bool single = bytes < kFieldBytes;
+  if (!single) {
+    const int rc = copy_stream(h);
+    if (rc) return rc;
+  }
+  for (int f = 0; f < nf; f++) {
+    if (!single) CK(cudaStreamWaitEvent(h->st, h->field_ev[f], 0));
+    launch_to_ref(P, dev + (size_t)f * P.fs, h->staging + f * ref, h->st);
+    if (!single) CK(cudaEventRecord(h->field_ev[f], h->st));
+  }
+  if (single) {
+    CK(cudaMemcpyAsync(host, h->staging, nf * bytes, cudaMemcpyDeviceToHost, h->st));
+    return GOP_OK;
+  }
+  // (a copy to pageable memory holds the host up: after all the launches)
+  for (int f = 0; f < nf; f++) {
+    CK(cudaStreamWaitEvent(h->copy, h->field_ev[f], 0));
+    CK(cudaMemcpyAsync(host + f * ref, h->staging + f * ref, bytes, cudaMemcpyDeviceToHost, h->copy));
+    CK(cudaEventRecord(h->field_ev[f], h->copy));
+  }
+  return GOP_OK;
+}
+// the copies of download_fields have ended
+static int wait_fields(gop_instance* h) {
+  if (h->copy) CK(cudaStreamSynchronize(h->copy));
+  CK(cudaStreamSynchronize(h->st));
+  return GOP_OK;
+}
 
 // the background block (BG_NF fields of doubles), allocated at first use and
 // zeroed
@@ -646,6 +719,9 @@ int gop_destroy(gop_instance* h) {
                   (void*)h->staging, (void*)h->bg, (void*)h->ringtab})
     if (p) cudaFreeAsync(p, h->st);
   if (h->own) cudaStreamDestroy(h->own);  // released once the frees have run
+  if (h->copy) cudaStreamDestroy(h->copy);
+  for (cudaEvent_t e : h->field_ev)
+    if (e) cudaEventDestroy(e);
   sweep_destroy(h->sweep);
   delete[] h->hscal;
   prof_collect(h);
@@ -667,18 +743,12 @@ int gop_upload(gop_instance* h, const double* gas, const double* face_b, const d
   if ((gas_p == nullptr) != (face_b_p == nullptr))
     return fail(GOP_EINVAL, "gas_p and face_b_p go together");
   const Params& P = h->P;
-  size_t ref = (size_t)P.N[0] * P.N[1] * P.N[2];
   // the current state goes to buffer 0, the history to buffer 1
-  CK(cudaMemcpyAsync(h->staging, gas, 6 * ref * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  launch_from_ref(P, 6, h->staging, P.Wbuf[0], h->st);
-  CK(cudaMemcpyAsync(h->staging, face_b, 3 * ref * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  launch_from_ref(P, 3, h->staging, P.Bbuf[0], h->st);
-  if (gas_p) {
-    CK(cudaMemcpyAsync(h->staging, gas_p, 6 * ref * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    launch_from_ref(P, 6, h->staging, P.Wbuf[1], h->st);
-    CK(cudaMemcpyAsync(h->staging, face_b_p, 3 * ref * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    launch_from_ref(P, 3, h->staging, P.Bbuf[1], h->st);
-  }
+  int rc = upload_fields(h, 6, gas, P.Wbuf[0]);
+  if (!rc) rc = upload_fields(h, 3, face_b, P.Bbuf[0]);
+  if (!rc && gas_p) rc = upload_fields(h, 6, gas_p, P.Wbuf[1]);
+  if (!rc && gas_p) rc = upload_fields(h, 3, face_b_p, P.Bbuf[1]);
+  if (rc) return rc;
   double* s = h->hscal;
   CK(cudaStreamSynchronize(h->st));
   for (int t = 0; t < NSCAL; t++) s[t] = 0.0;
@@ -709,14 +779,13 @@ int gop_set_background(gop_instance* h, const double* b0, const double* lorentz,
   int rc = alloc_background(h);
   if (rc) return rc;
   const size_t ref = (size_t)P.N[0] * P.N[1] * P.N[2];
-  // through the staging buffer (6 fields) in groups of 3
   const double* src[8] = {b0, lorentz, b0_face, b0_face + 3 * ref, b0_face + 6 * ref,
                           b0_edge, b0_edge + 3 * ref, b0_edge + 6 * ref};
   const int dst[8] = {BG_B0, BG_LOR, BG_FACE, BG_FACE + 3, BG_FACE + 6,
                       BG_EDGE, BG_EDGE + 3, BG_EDGE + 6};
   for (int g = 0; g < 8; g++) {
-    CK(cudaMemcpyAsync(h->staging, src[g], 3 * ref * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    launch_from_ref(P, 3, h->staging, h->bg + (size_t)dst[g] * P.fs, h->st);
+    rc = upload_fields(h, 3, src[g], h->bg + (size_t)dst[g] * P.fs);
+    if (rc) return rc;
   }
   CK(cudaStreamSynchronize(h->st));
   CK(cudaGetLastError());
@@ -755,11 +824,10 @@ int gop_get_background(gop_instance* h, double* b0, double* lorentz, double* b0_
                       BG_EDGE, BG_EDGE + 3, BG_EDGE + 6};
   for (int g = 0; g < 8; g++) {
     if (!dst[g]) continue;
-    launch_to_ref(P, 3, h->bg + (size_t)src[g] * P.fs, h->staging, h->st);
-    CK(cudaMemcpyAsync(dst[g], h->staging, 3 * ref * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+    const int rc = download_fields(h, 3, h->bg + (size_t)src[g] * P.fs, dst[g]);
+    if (rc) return rc;
   }
-  CK(cudaStreamSynchronize(h->st));
-  return GOP_OK;
+  return wait_fields(h);
 }
 
 int gop_problem_init_device(gop_instance* h, const gop_problem* p) {
@@ -952,13 +1020,10 @@ int gop_step(gop_instance* h, int nsteps, double time_stop, double* time_out) {
 
 }  // extern "C"
 
+// download_fields, and the wait for its copies
 static int download_field(gop_instance* h, int nf, const double* dev, double* host) {
-  const Params& P = h->P;
-  size_t ref = (size_t)P.N[0] * P.N[1] * P.N[2];
-  launch_to_ref(P, nf, dev, h->staging, h->st);
-  CK(cudaMemcpyAsync(host, h->staging, nf * ref * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  return GOP_OK;
+  const int rc = download_fields(h, nf, dev, host);
+  return rc ? rc : wait_fields(h);
 }
 
 template <typename R>
@@ -986,10 +1051,12 @@ int gop_download(gop_instance* h, double* gas, double* face_b, double* gas_h, do
   CK(cudaStreamSynchronize(h->st));
   int cur = s[S_PAR] != 0.0 ? 1 : 0;
   int rc = GOP_OK;
-  if (gas && (rc = download_field(h, 6, P.Wbuf[cur], gas))) return rc;
-  if (face_b && (rc = download_field(h, 3, P.Bbuf[cur], face_b))) return rc;
-  if (gas_p && (rc = download_field(h, 6, P.Wbuf[1 - cur], gas_p))) return rc;
-  if (face_b_p && (rc = download_field(h, 3, P.Bbuf[1 - cur], face_b_p))) return rc;
+  if (gas) rc = download_fields(h, 6, P.Wbuf[cur], gas);
+  if (!rc && face_b) rc = download_fields(h, 3, P.Bbuf[cur], face_b);
+  if (!rc && gas_p) rc = download_fields(h, 6, P.Wbuf[1 - cur], gas_p);
+  if (!rc && face_b_p) rc = download_fields(h, 3, P.Bbuf[1 - cur], face_b_p);
+  const int waited = wait_fields(h);  // also where a call failed: the arrays are the caller's again
+  if (rc || waited) return rc ? rc : waited;
   if (mags) {
     double* tmp = nullptr;
     CK(cudaMallocAsync((void**)&tmp, (size_t)P.fs * 3 * sizeof(double), h->st));

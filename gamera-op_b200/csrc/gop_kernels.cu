@@ -1275,27 +1275,43 @@ __global__ void k_bcface(Params P, int axis, int side, int kind, int gkind, int 
 
 // ------------------------------------------------------ layout transposes
 
-// reference layout [f][i][j][k] (k fastest) <-> device layout
-__global__ void k_from_ref(Params P, int nf, const double* __restrict__ src, double* __restrict__ dst) {
+// reference layout [i][j][k] (k fastest) <-> device layout of one field: the
+// (i, k) plane of each j in 32 x 32 tiles through shared memory (padded by one
+// column against bank conflicts), so both sides move whole lines.  Threads
+// along i that read k-fastest memory directly touch one 32-byte sector per
+// value.  Blocks of 32 x 8 threads over (k tiles, i tiles, rows j).
+constexpr int kXT = 32, kXR = 8;
+template <bool TO_REF>
+__global__ void __launch_bounds__(kXT* kXR) k_transpose(Params P, const double* __restrict__ src,
+                                                        double* __restrict__ dst) {
   pdl_enter();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int kf = blockIdx.z;
-  const int k = kf % P.N[2], f = kf / P.N[2];
-  if (i >= P.N[0] || j >= P.N[1] || f >= nf) return;
-  const size_t r = (((size_t)f * P.N[0] + i) * P.N[1] + j) * P.N[2] + k;
-  dst[(size_t)f * P.fs + lin(P, i, j, k)] = src[r];
-}
-
-__global__ void k_to_ref(Params P, int nf, const double* __restrict__ src, double* __restrict__ dst) {
-  pdl_enter();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int kf = blockIdx.z;
-  const int k = kf % P.N[2], f = kf / P.N[2];
-  if (i >= P.N[0] || j >= P.N[1] || f >= nf) return;
-  const size_t r = (((size_t)f * P.N[0] + i) * P.N[1] + j) * P.N[2] + k;
-  dst[r] = src[(size_t)f * P.fs + lin(P, i, j, k)];
+  __shared__ double tile[kXT][kXT + 1];
+  const int N0 = P.N[0], N1 = P.N[1], N2 = P.N[2];
+  const int k0 = blockIdx.x * kXT, i0 = blockIdx.y * kXT, tx = threadIdx.x, ty = threadIdx.y;
+  for (int j = blockIdx.z; j < N1; j += gridDim.z) {
+    __syncthreads();  // the tile of the row before has been read
+#pragma unroll
+    for (int r = 0; r < kXT; r += kXR) {
+      if (TO_REF) {  // lanes along i
+        const int i = i0 + tx, k = k0 + ty + r;
+        if (i < N0 && k < N2) tile[ty + r][tx] = src[lin(P, i, j, k)];
+      } else {  // lanes along k
+        const int i = i0 + ty + r, k = k0 + tx;
+        if (i < N0 && k < N2) tile[tx][ty + r] = src[((size_t)i * N1 + j) * N2 + k];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kXT; r += kXR) {
+      if (TO_REF) {
+        const int i = i0 + ty + r, k = k0 + tx;
+        if (i < N0 && k < N2) dst[((size_t)i * N1 + j) * N2 + k] = tile[tx][ty + r];
+      } else {
+        const int i = i0 + tx, k = k0 + ty + r;
+        if (i < N0 && k < N2) dst[lin(P, i, j, k)] = tile[ty + r][tx];
+      }
+    }
+  }
 }
 
 template <typename R>
@@ -1580,16 +1596,14 @@ void launch_ghosts(const Params& P, const char bc[6], const char gem_bc[6], int 
   }
 }
 
-void launch_from_ref(const Params& P, int nf, const double* src, double* dst, cudaStream_t st) {
-  const dim3 blk(32, 8, 1);
-  const dim3 g((P.N[0] + 31) / 32, (P.N[1] + 7) / 8, P.N[2] * nf);
-  LAUNCH(k_from_ref, g, blk, st, P, nf, src, dst);
+static dim3 transpose_grid(const Params& P) {
+  return dim3((P.N[2] + kXT - 1) / kXT, (P.N[0] + kXT - 1) / kXT, std::min(P.N[1], 65535));
 }
-
-void launch_to_ref(const Params& P, int nf, const double* src, double* dst, cudaStream_t st) {
-  const dim3 blk(32, 8, 1);
-  const dim3 g((P.N[0] + 31) / 32, (P.N[1] + 7) / 8, P.N[2] * nf);
-  LAUNCH(k_to_ref, g, blk, st, P, nf, src, dst);
+void launch_from_ref(const Params& P, const double* src, double* dst, cudaStream_t st) {
+  LAUNCH(k_transpose<false>, transpose_grid(P), dim3(kXT, kXR), st, P, src, dst);
+}
+void launch_to_ref(const Params& P, const double* src, double* dst, cudaStream_t st) {
+  LAUNCH(k_transpose<true>, transpose_grid(P), dim3(kXT, kXR), st, P, src, dst);
 }
 
 template <typename R>

@@ -109,8 +109,9 @@ void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t
 // which = 0: the buffer being written this step; 1: the current state
 void launch_ghosts(const Params& P, const char bc[6], const char gem_bc[6], int which,
                    cudaStream_t st);
-void launch_from_ref(const Params& P, int nf, const double* src, double* dst, cudaStream_t st);
-void launch_to_ref(const Params& P, int nf, const double* src, double* dst, cudaStream_t st);
+// one field between the reference layout and the device's
+void launch_from_ref(const Params& P, const double* src, double* dst, cudaStream_t st);
+void launch_to_ref(const Params& P, const double* src, double* dst, cudaStream_t st);
 template <typename R>
 void launch_widen(const Params& P, int nf, const R* src, double* dst, cudaStream_t st);
 void launch_mags(const Params& P, const double* B, double* out, cudaStream_t st);

@@ -591,7 +591,10 @@ int gop_create(const gop_desc* desc, gop_instance** out) {
   P.n[0] = d.ni;
   P.n[1] = d.nj;
   P.n[2] = d.nk;
-  for (int a = 0; a < 3; a++) P.N[a] = L.N[a];
+  for (int a = 0; a < 3; a++) {
+    P.N[a] = L.N[a];
+    P.per[a] = d.bc[2 * a] == 'p' && d.bc[2 * a + 1] == 'p';
+  }
   P.pitch = L.pitch;
   P.coord = d.coord;
   P.sj = L.pitch;
@@ -696,11 +699,12 @@ int gop_create(const gop_desc* desc, gop_instance** out) {
   // the tile-staged flux sweeps read the work and state arrays through
   // tensor maps made once here; without them the per-face kernels run
   h->sweep = mixed ? sweep_create<float>(P, h->wf) : sweep_create<double>(P, h->wd);
-  // FP32 edge EMFs: the per-edge kernel measured faster on B200 (blast 256^3:
-  // 1.09 vs 1.26 ms per step), FP64 the sweep (2.06 vs 2.25 ms); the
-  // autotuner decides per launch
-  if (mixed)
-    for (int d = 0; d < 3; d++) h->tune.emf_sweep[d] = false;
+  // FP32 edge EMFs: the sweep, but for a thin grid, whose few k faces leave
+  // most of its 16-row tiles empty, the per-edge kernels (B200, us per step:
+  // blast 256^3 1034 per edge, 854 sweep; 64^3 33, 27; Orszag-Tang 256x256x4
+  // 33, 40).  FP64: the sweep (the thin grid 79 per edge, 49 sweep); the
+  // autotuner decides per launch.
+  if (mixed && d.nk < 8) h->tune.emf_sweep = false;
   cudaError_t le = e != cudaSuccess ? e : cudaStreamSynchronize(h->st);
   if (le == cudaSuccess) le = cudaGetLastError();
   if (le != cudaSuccess) {
@@ -1105,39 +1109,60 @@ int gop_autotune(gop_instance* h, int reps, int* chosen) {
   CK(cudaMemcpyAsync(hist, P.Wbuf[1 - cur], wbytes, cudaMemcpyDeviceToDevice, h->st));
   CK(cudaMemcpyAsync(hist + 6 * P.fs, P.Bbuf[1 - cur], bbytes, cudaMemcpyDeviceToDevice, h->st));
   const bool mixed = h->d.precision == GOP_PREC_MIXED;
+  int pick[NTUNE] = {};
+  // a warm-up run of fn, then reps timed ones
+  auto timed = [&](auto fn, float* ms) -> cudaError_t {
+    for (int r = 0; r <= reps; r++) {
+      if (r == 1) cudaEventRecord(a, h->st);
+      fn();
+    }
+    cudaEventRecord(b, h->st);
+    cudaError_t e = cudaEventSynchronize(b);
+    return e != cudaSuccess ? e : cudaEventElapsedTime(ms, a, b);
+  };
+  auto launch_point = [&](int slot, dim3 blk) {
+    if (mixed) launch_slot<float>(h->P, h->d.coord, h->wf, slot, blk, h->st);
+    else launch_slot<double>(h->P, h->d.coord, h->wd, slot, blk, h->st);
+  };
   for (int slot = 0; slot < NTUNE; slot++) {
     float best = 1e30f;
-    int best_c = 0;
-    // the flux and EMF slots also try the tile-staged sweep kernel
-    // (candidate ncand)
-    const bool flux = slot >= K_FLUX0 && slot <= K_FLUX2;
-    const bool emf = slot >= K_EMF0 && slot <= K_EMF2;
-    const bool try_sweep = h->sweep && (emf || (flux && !P.ps_live));
-    for (int c = 0; c < ncand + (try_sweep ? 1 : 0); c++) {
-      const bool sw = c == ncand;
-      if (!sw && cand[c].x * cand[c].y * cand[c].z > 256) continue;
-      const dim3 blk = sw ? h->tune.blk[slot] : cand[c];
-      // warm-up launch, then reps timed launches
-      for (int r = 0; r <= reps; r++) {
-        if (r == 1) cudaEventRecord(a, h->st);
-        if (mixed) launch_slot<float>(h->P, h->d.coord, h->wf, slot, blk, h->st, sw ? h->sweep : nullptr);
-        else launch_slot<double>(h->P, h->d.coord, h->wd, slot, blk, h->st, sw ? h->sweep : nullptr);
-      }
-      cudaEventRecord(b, h->st);
-      CK(cudaEventSynchronize(b));
+    for (int c = 0; c < ncand; c++) {
+      if (cand[c].x * cand[c].y * cand[c].z > 256) continue;
       float ms = 0.f;
-      cudaEventElapsedTime(&ms, a, b);
+      CK(timed([&] { launch_point(slot, cand[c]); }, &ms));
       if (ms < best) {
         best = ms;
-        best_c = c;
+        pick[slot] = c;
       }
     }
-    if (best_c < ncand) h->tune.blk[slot] = cand[best_c];
-    if (flux) h->tune.flux_sweep[slot - K_FLUX0] = best_c == ncand;
-    if (emf) h->tune.emf_sweep[slot - K_EMF0] = best_c == ncand;
-    if (chosen) chosen[slot] = best_c;
-    drop_step_graph(h);  // the captured step has the old shapes
+    h->tune.blk[slot] = cand[pick[slot]];
   }
+  // the flux and EMF stages: the three per-point launches with those shapes
+  // or the tile-staged sweep (candidate ncand)
+  for (int stage = 0; stage < 2; stage++) {
+    const bool flux = stage == 0;
+    const int first = flux ? K_FLUX0 : K_EMF0;
+    bool* sweep = flux ? &h->tune.flux_sweep : &h->tune.emf_sweep;
+    if (!h->sweep || (flux && P.ps_live)) {
+      *sweep = false;
+      continue;
+    }
+    float t_point = 0.f, t_sweep = 0.f;
+    CK(timed([&] { for (int d = 0; d < 3; d++) launch_point(first + d, h->tune.blk[first + d]); }, &t_point));
+    const int* ord = flux ? h->tune.flux_order : h->tune.emf_order;
+    CK(timed([&] {
+      if (flux && mixed) launch_flux_sweep<float>(h->sweep, P, h->wf, ord, h->st);
+      else if (flux) launch_flux_sweep<double>(h->sweep, P, h->wd, ord, h->st);
+      else if (mixed) launch_emf_sweep<float>(h->sweep, P, h->wf, ord, h->st);
+      else launch_emf_sweep<double>(h->sweep, P, h->wd, ord, h->st);
+    }, &t_sweep));
+    *sweep = t_sweep < t_point;
+    if (*sweep)
+      for (int d = 0; d < 3; d++) pick[first + d] = ncand;
+  }
+  if (chosen)
+    for (int t = 0; t < NTUNE; t++) chosen[t] = pick[t];
+  drop_step_graph(h);  // the captured step has the old shapes
   // The order of the three flux launches and of the three EMF launches
   // (independent launches: the order changes no result, only what L2 holds
   // from one launch to the next): two whole steps timed per rotation of
@@ -1209,7 +1234,7 @@ int gop_set_sweep(gop_instance* h, int on) {
   if (!h) return fail(GOP_EINVAL, "instance is NULL");
   if (on && !h->sweep) return fail(GOP_ENODEV, "the tile-staged sweep kernels are not available");
   CK(cudaStreamSynchronize(h->st));
-  for (int d = 0; d < 3; d++) h->tune.flux_sweep[d] = h->tune.emf_sweep[d] = on != 0;
+  h->tune.flux_sweep = h->tune.emf_sweep = on != 0;
   drop_step_graph(h);
   return GOP_OK;
 }
@@ -1344,7 +1369,7 @@ static int batch_build(gop_batch* b) {
 static int batch_pick_sweeps(gop_batch* b) {
   bool any = false;
   for (gop_instance* h : b->m)
-    for (int d = 0; d < 3; d++) any = any || h->tune.flux_sweep[d] || h->tune.emf_sweep[d];
+    any = any || h->tune.flux_sweep || h->tune.emf_sweep;
   if (!any || !b->graph) return GOP_OK;
   const size_t nm = b->m.size();
   std::vector<double*> saved(nm, nullptr);
@@ -1390,7 +1415,7 @@ static int batch_pick_sweeps(gop_batch* b) {
     std::vector<Tune> pick(nm);
     for (size_t i = 0; i < nm; i++) pick[i] = b->m[i]->tune;
     for (gop_instance* h : b->m) {
-      for (int d = 0; d < 3; d++) h->tune.flux_sweep[d] = h->tune.emf_sweep[d] = false;
+      h->tune.flux_sweep = h->tune.emf_sweep = false;
       drop_step_graph(h);
     }
     if (rc == GOP_OK) rc = batch_build(b);

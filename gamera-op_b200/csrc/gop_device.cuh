@@ -70,6 +70,8 @@ enum Scal : int {
   S_BUDGET,      // steps left in the current gop_step call
   S_PSNZ,        // gop_prepare's check: nonzero if some p_S of the state or
                  // of its AB2 history is nonzero
+  S_TILE,        // two 32-bit counters of the running sweep launch: tiles
+                 // handed out, blocks done; zero between launches
   NSCAL
 };
 
@@ -78,6 +80,7 @@ struct Params {
   int N[3];           // ghost-extended points
   int pitch;          // row pitch (elements)
   int coord;          // 0: Cartesian, 2: spherical (batched kernels select on it)
+  int per[3];         // 1: the axis is periodic
   long long sj, sk;   // strides of j and k (stride of i is 1)
   long long fs;       // stride between fields
   const double* tab;  // [3][NTAB][tmax]
@@ -117,6 +120,12 @@ __device__ __forceinline__ double tb(const Params& P, int axis, int t, int idx) 
 
 __device__ __forceinline__ long long lin(const Params& P, int i, int j, int k) {
   return (long long)k * P.sk + (long long)j * P.sj + i;
+}
+
+// the same in 32 bits: a field has fewer than 2^31 points (an instance holds
+// at least 348 bytes per point, so one of 2^31 would not fit any GPU)
+__device__ __forceinline__ int lin32(const Params& P, int i, int j, int k) {
+  return (k * P.N[1] + j) * P.pitch + i;
 }
 
 __device__ __forceinline__ long long stride(const Params& P, int axis) {

@@ -394,7 +394,8 @@ __device__ __forceinline__ void flux_body(const Params& P, const Work<R>& wk, Po
     for (int u = 0; u < 4; u++) lim[u] = ms[(u - 2) * s];
     recon_lr(v, lim, Wt, mL[a], mR[a]);
   }
-  flux_out<R, D, BG, PSL>(P, wk, x, L, Rt, mL, mR, lim_b<R>(P, wk)[x + D * fs]);
+  flux_out<R, D, BG, PSL>(P, wk, (int)x, D == 0 ? j : (D == 1 ? k : i), L, Rt, mL, mR,
+                          lim_b<R>(P, wk)[x + D * fs]);
 }
 
 // --------------------------------------------------------------- update
@@ -1232,17 +1233,6 @@ __global__ void __launch_bounds__(256, GOP_MINB(FLUX, R)) k_flux(Params P, Work<
   if (stopped(P)) return;
   flux_body<R, D, BG, PSL>(P, w, grid_pos());
 }
-// The faces i = NGH + n0 (the upper boundary face of every i row) of the
-// flux along i, one thread per (j, k) row: the i sweep leaves them out when
-// 32 divides n0 (a ninth tile of 32 lanes per row would run with one live
-// lane per warp)
-template <typename R, bool BG>
-__global__ void __launch_bounds__(256) k_flux_col(Params P, Work<R> w) {
-  pdl_enter();
-  if (stopped(P)) return;
-  const int tj = blockIdx.x * blockDim.x + threadIdx.x, tk = blockIdx.y * blockDim.y + threadIdx.y;
-  flux_body<R, 0, BG, false>(P, w, Pos{P.n[0], tj, tk});
-}
 template <int COORD, typename R>
 __global__ void __launch_bounds__(256, GOP_MINB_CT) k_ct(Params P, Work<R> w) {
   pdl_enter();
@@ -1382,9 +1372,9 @@ Tune::Tune() {
   // the first edge sweep of edges along j covers only the 8 ghost layers of i
   blk[K_C2C1] = dim3(8, 32, 1);
   for (int d = 0; d < 3; d++) {
-    flux_sweep[d] = emf_sweep[d] = true;
     flux_order[d] = emf_order[d] = d;
   }
+  flux_sweep = emf_sweep = true;
 }
 
 dim3 launch_space(const Params& P, int slot) {
@@ -1400,7 +1390,7 @@ dim3 launch_space(const Params& P, int slot) {
   const int stage = (slot - K_C2C0) / 3, D = (slot - K_C2C0) % 3;
   const int p = (D + 1) % 3, q = (D + 2) % 3;
   int cnt[3];
-  if (stage == 0) {  // ghost layers of q only (the flux stage covers the rest)
+  if (stage == 0) {  // ghost layers of q only (see c2c_body)
     cnt[D] = P.n[D];
     cnt[p] = P.n[p] + 1;
     cnt[q] = 2 * NGH;
@@ -1450,9 +1440,7 @@ void launch_dt(const Params& P, int coord, bool mixed, cudaStream_t st) {
 
 template <typename R, bool BG>
 static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slot, dim3 blk,
-                           cudaStream_t st, const SweepSet* sw, bool pdl) {
-  if (slot >= K_FLUX0 && slot <= K_FLUX2 && launch_flux_sweep<R>(sw, P, w, slot - K_FLUX0, st)) return;
-  if (slot >= K_EMF0 && slot <= K_EMF2 && launch_emf_sweep<R>(sw, P, w, slot - K_EMF0, st)) return;
+                           cudaStream_t st, bool pdl) {
   const dim3 sp = launch_space(P, slot);
   const dim3 g = grid3(sp.x, sp.y, sp.z, blk);
   switch (slot) {
@@ -1461,11 +1449,11 @@ static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slo
       else LAUNCH((k_ab2<R, false>), g, blk, st, P, w);
       break;
     case K_C2C0: LAUNCH_PDL(pdl, (k_c2c<R, 0>), g, blk, st, P, w); break;
-    case K_C2C1: LAUNCH((k_c2c<R, 1>), g, blk, st, P, w); break;
-    case K_C2C2: LAUNCH((k_c2c<R, 2>), g, blk, st, P, w); break;
-    case K_EMF0: LAUNCH((k_emf<R, 0, BG>), g, blk, st, P, w); break;
-    case K_EMF1: LAUNCH((k_emf<R, 1, BG>), g, blk, st, P, w); break;
-    case K_EMF2: LAUNCH((k_emf<R, 2, BG>), g, blk, st, P, w); break;
+    case K_C2C1: LAUNCH_PDL(pdl, (k_c2c<R, 1>), g, blk, st, P, w); break;
+    case K_C2C2: LAUNCH_PDL(pdl, (k_c2c<R, 2>), g, blk, st, P, w); break;
+    case K_EMF0: LAUNCH_PDL(pdl, (k_emf<R, 0, BG>), g, blk, st, P, w); break;
+    case K_EMF1: LAUNCH_PDL(pdl, (k_emf<R, 1, BG>), g, blk, st, P, w); break;
+    case K_EMF2: LAUNCH_PDL(pdl, (k_emf<R, 2, BG>), g, blk, st, P, w); break;
     case K_FLUX0:
       if (P.ps_live) LAUNCH((k_flux<R, 0, BG, true>), g, blk, st, P, w);
       else LAUNCH((k_flux<R, 0, BG, false>), g, blk, st, P, w);
@@ -1492,27 +1480,14 @@ static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slo
 }
 
 template <typename R>
-void launch_flux_col(const Params& P, const Work<R>& w, cudaStream_t st) {
-  const dim3 blk(32, 8, 1);
-  const dim3 g((P.n[1] + 31) / 32, (P.n[2] + 7) / 8, 1);
-  // right after a sweep: no early launch (see launch_step_body)
-  if (P.bg) LAUNCH_PDL(false, (k_flux_col<R, true>), g, blk, st, P, w);
-  else LAUNCH_PDL(false, (k_flux_col<R, false>), g, blk, st, P, w);
-}
-template void launch_flux_col<double>(const Params&, const Work<double>&, cudaStream_t);
-template void launch_flux_col<float>(const Params&, const Work<float>&, cudaStream_t);
-
-template <typename R>
 void launch_slot(const Params& P, int coord, const Work<R>& w, int slot, dim3 blk,
-                 cudaStream_t st, const SweepSet* sw, bool pdl) {
-  if (P.bg) launch_slot_bg<R, true>(P, coord, w, slot, blk, st, sw, pdl);
-  else launch_slot_bg<R, false>(P, coord, w, slot, blk, st, sw, pdl);
+                 cudaStream_t st, bool pdl) {
+  if (P.bg) launch_slot_bg<R, true>(P, coord, w, slot, blk, st, pdl);
+  else launch_slot_bg<R, false>(P, coord, w, slot, blk, st, pdl);
 }
 
-template void launch_slot<double>(const Params&, int, const Work<double>&, int, dim3, cudaStream_t,
-                                  const SweepSet*, bool);
-template void launch_slot<float>(const Params&, int, const Work<float>&, int, dim3, cudaStream_t,
-                                 const SweepSet*, bool);
+template void launch_slot<double>(const Params&, int, const Work<double>&, int, dim3, cudaStream_t, bool);
+template void launch_slot<float>(const Params&, int, const Work<float>&, int, dim3, cudaStream_t, bool);
 
 template <typename R>
 void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t st,
@@ -1520,34 +1495,46 @@ void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t
   hook(G_AB2, 1);
   launch_slot<R>(P, coord, w, K_AB2, tune.blk[K_AB2], st);
   hook(G_AB2, 0);
-  // flux first: it also writes the edge velocities of the active range
-  // the three launches of a stage are independent (each axis writes its own
-  // fluxes, edge velocities or EMFs), so their order (Tune) changes no result
-  const int last_flux = tune.flux_order[2], last_emf = tune.emf_order[2];
-  for (int stage : {2, 0, 1}) {
-    const int g = stage == 0 ? G_C2C : (stage == 1 ? G_EMF : G_FLUX);
-    hook(g, 1);
+  // flux first: it also writes the edge velocities of the active range and
+  // of the ghost layers of periodic axes.  The axes of a stage are
+  // independent (each writes its own fluxes, edge velocities or EMFs), so
+  // their order (Tune) changes no result.  The launch after a persistent
+  // sweep grid waits for it to finish instead of being placed early on SMs
+  // still configured for the sweep's shared memory (and its short L1).
+  hook(G_FLUX, 1);
+  bool after_sweep = tune.flux_sweep && launch_flux_sweep<R>(sw, P, w, tune.flux_order, st);
+  if (!after_sweep)
     for (int n = 0; n < 3; n++) {
-      const int d = stage == 2 ? tune.flux_order[n] : (stage == 1 ? tune.emf_order[n] : n);
-      const int slot = K_C2C0 + 3 * stage + d;
-      const bool sweep = sw && ((stage == 2 && tune.flux_sweep[d]) || (stage == 1 && tune.emf_sweep[d]));
-      // the launch after a persistent sweep grid waits for it to finish
-      // instead of being placed early on SMs still configured for the
-      // sweep's shared memory (and its short L1)
-      const bool pdl = !(stage == 0 && n == 0 && sw && tune.flux_sweep[last_flux]) || GOP_PDL_AFTER_SWEEP;
-      launch_slot<R>(P, coord, w, slot, tune.blk[slot], st, sweep ? sw : nullptr, pdl);
+      const int slot = K_FLUX0 + tune.flux_order[n];
+      launch_slot<R>(P, coord, w, slot, tune.blk[slot], st);
     }
-    hook(g, 0);
+  hook(G_FLUX, 0);
+  hook(G_C2C, 1);
+  for (int d = 0; d < 3; d++) {
+    if (P.per[(d + 2) % 3]) continue;  // the flux stage has written those ghost layers
+    launch_slot<R>(P, coord, w, K_C2C0 + d, tune.blk[K_C2C0 + d], st, !after_sweep || GOP_PDL_AFTER_SWEEP);
+    after_sweep = false;
   }
+  hook(G_C2C, 0);
+  hook(G_EMF, 1);
+  if (tune.emf_sweep && launch_emf_sweep<R>(sw, P, w, tune.emf_order, st)) {
+    after_sweep = true;
+  } else {
+    for (int n = 0; n < 3; n++) {
+      const int slot = K_EMF0 + tune.emf_order[n];
+      launch_slot<R>(P, coord, w, slot, tune.blk[slot], st, !after_sweep || GOP_PDL_AFTER_SWEEP);
+      after_sweep = false;
+    }
+  }
+  hook(G_EMF, 0);
   hook(G_UPDATE, 1);
-  const bool after_emf_sweep = sw && tune.emf_sweep[last_emf] && !GOP_PDL_AFTER_SWEEP;
+  const bool after_emf_sweep = after_sweep && !GOP_PDL_AFTER_SWEEP;
   launch_pole_emf<R>(P, w, st);  // pole ring average only
   if (coord != 0) {  // curvilinear: the face fields in their own launch
     const dim3 blk = tune.blk[K_UPDATE];
     LAUNCH_PDL(!after_emf_sweep, (k_ct<2, R>), grid3(P.n[0], P.n[1], P.n[2], blk), blk, st, P, w);
   }
-  launch_slot<R>(P, coord, w, K_UPDATE, tune.blk[K_UPDATE], st, nullptr,
-                 coord != 0 || !after_emf_sweep);
+  launch_slot<R>(P, coord, w, K_UPDATE, tune.blk[K_UPDATE], st, coord != 0 || !after_emf_sweep);
   // the work arrays are free after the update: 2 fields of doubles of scratch
   if (P.ring) {
     launch_ring_average(P, reinterpret_cast<double*>(w.Wh), st);

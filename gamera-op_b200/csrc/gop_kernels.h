@@ -43,12 +43,11 @@ enum TuneSlot : int { K_AB2 = 0, K_C2C0, K_C2C1, K_C2C2, K_EMF0, K_EMF1, K_EMF2,
                       K_BC5, NSLOT };
 struct Tune {
   dim3 blk[NTUNE];
-  // flux of axis d / EMF of the edges along d from the tile-staged sweep
-  // kernels (gop_sweep.cu) instead of the per-point kernels, where the
-  // sweeps apply
-  bool flux_sweep[3];
-  bool emf_sweep[3];
-  // order of the three (independent) launches of the flux and EMF stages
+  // the stage's fluxes / edge EMFs from the tile-staged sweep kernels
+  // (gop_sweep.cu) instead of the per-point kernels, where the sweeps apply
+  bool flux_sweep;
+  bool emf_sweep;
+  // order of the axes (independent) in the flux and EMF stages
   int flux_order[3];
   int emf_order[3];
   Tune();
@@ -60,18 +59,14 @@ struct SweepSet;
 template <typename R>
 SweepSet* sweep_create(const Params& P, const Work<R>& w);
 void sweep_destroy(SweepSet* s);
-// the flux of axis D by the sweep kernel; false (nothing launched) where the
-// sweep does not apply (no maps, or the entropy channel is live)
+// The fluxes (edge EMFs) of the three axes by the sweep kernels, their tiles
+// in the given order; false (nothing launched) where the sweep does not apply
+// (no maps; for the flux, the entropy channel is live)
 template <typename R>
-bool launch_flux_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, int D,
+bool launch_flux_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, const int order[3],
                        cudaStream_t st);
-// the row-end faces of the flux along i that its sweep leaves out (32
-// dividing n0), by the per-face arithmetic
 template <typename R>
-void launch_flux_col(const Params& P, const Work<R>& w, cudaStream_t st);
-// the EMF of the edges along D by the sweep kernel; false without maps
-template <typename R>
-bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, int D,
+bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, const int order[3],
                       cudaStream_t st);
 
 // points covered by the launch of one slot (x, y, z extents)
@@ -79,12 +74,11 @@ dim3 launch_space(const Params& P, int slot);
 // thread-block shape of a ghost-fill slot (K_WRAP*, K_BC*)
 dim3 ghost_block(int slot);
 
-// launches one tunable kernel alone (for the autotuner); a flux or EMF slot
-// with sw set runs the sweep kernel instead (blk unused); pdl false:
-// without programmatic dependent launch
+// launches one tunable kernel; pdl false: without programmatic dependent
+// launch
 template <typename R>
 void launch_slot(const Params& P, int coord, const Work<R>& w, int slot, dim3 blk,
-                 cudaStream_t st, const SweepSet* sw = nullptr, bool pdl = true);
+                 cudaStream_t st, bool pdl = true);
 
 // optional timing hook: mark(ctx, group, start) records an event on the stream
 struct Hook {

@@ -17,11 +17,11 @@
 //            residency) with cp.async.bulk.tensor (one TMA box per
 //            input array and tile: stencil windows, limiter windows, PDM
 //            weights), completing on the slot's "full" mbarrier;
-//   compute  8 warps compute one face or edge per thread from shared memory
-//            (every stencil tap is a load at a compile-time offset from one
-//            per-thread base) and release the slot on its "empty" mbarrier;
-//            the feeding thread refills a released slot with the next tile
-//            not yet issued, a ring's length ahead.
+//   compute  8 warps compute one face, or one or two edges, per thread from
+//            shared memory (every stencil tap is a load at a compile-time
+//            offset from one per-thread base) and release the slot on its
+//            "empty" mbarrier; the feeding thread refills a released slot
+//            with the next tile not yet taken, a ring's length ahead.
 //
 // So the global-memory latency of tile n+1 overlaps the arithmetic of tile
 // n, and the stencil re-reads come from shared memory instead of L1.  The
@@ -29,7 +29,7 @@
 // emf_finish), in the same order, so both forms give the same bits.
 //
 // Lanes always run along i (x, the TMA box's contiguous axis); a tile is 32
-// lanes x 8 warps, one warp per row along the stage's sweep axis or its
+// lanes x 8 or 16 rows, a warp's row along the stage's sweep axis or its
 // third axis.  Every box starts at an x of 32 t or 4 + 32 t, so x times the
 // element size is a multiple of 16 bytes (the TMA's alignment rule); no
 // coordinate is negative.  Boxes reaching past the grid are filled with
@@ -42,6 +42,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "gop_stage.cuh"
 #include "gop_tma.cuh"
@@ -101,39 +102,22 @@ struct Box {
   __host__ __device__ constexpr int elems() const { return x * y * z * f; }
   __host__ __device__ constexpr int padded() const { return (elems() + 31) / 32 * 32; }
 };
-constexpr Box kRec8{FW, 8, 1, 1};    // 8 packed face records
-constexpr Box kRec1{FW, 1, 1, 1};    // 1 packed face record
-// tap-major weights (T_WL0..T_CR2) of the 32 faces of a warp row, and of
-// the face after them (the edge-EMF sweeps on i faces, below)
-constexpr Box kTap32{32, 18, 1, 1};
+// n packed face records
+constexpr Box rec(int n) { return Box{FW, n, 1, 1}; }
+// tap-major weights (T_WL0..T_CR2) of the 32 faces of a warp row and of the
+// face after them (the sweeps on i faces, below)
 constexpr Box kTap40{40, 18, 1, 1};
 
-// The edge-EMF sweeps whose lanes run along i over the n+1 faces of an i
-// row (the EMFs along j and k) tile the row in ceil(n/32) tiles of 32
+// The sweeps whose lanes run along i over the n+1 faces of an i row (the flux
+// along i, the EMFs along j and k) tile the row in ceil(n/32) tiles of 32
 // faces; when 32 divides n the last face of the row, the upper boundary
 // face, is left over.  The last tile of the row then computes it too, in
 // one extra pass of one warp whose lanes take the tile's 8 rows (its boxes
 // are 40 wide along i, so that face's stencil is in the slot), where a
-// ninth tile would cost eight warp passes with one live lane each: 1.6 %
-// off the FP64 EMF stage at 256^3 on B200.  The flux sweep along i keeps
-// its ninth tile: the same pass made it 1 % slower there (FP32 3.5 %).
+// ninth tile would cost eight warp passes with one live lane each.  The pass
+// is a second trip through the same code (a second copy of a face's
+// arithmetic, or a call, cost the flux more than it saved).
 __device__ __forceinline__ bool row_end_face(const Params& P, int x0) { return x0 + 32 == NGH + P.n[0]; }
-// 1: the FP64 flux sweep along i leaves the row-end faces (32 dividing n)
-// to a one-column launch of the per-face arithmetic (k_flux_col) instead
-// of a ninth tile per row: FP64 step 7.26 -> 7.20 ms at 256^3 on B200; the
-// FP32 step measured 1.5 % slower that way and keeps the ninth tile
-#ifndef GOP_FLUX_COL
-#define GOP_FLUX_COL 1
-#endif
-template <typename R>
-constexpr bool flux_col() {
-  return GOP_FLUX_COL && sizeof(R) == 8;
-}
-// the warp that takes it: rotates over the row sets (kWarps a power of 2)
-template <class T>
-__device__ __forceinline__ int row_end_warp(const int nt[3], const T& t) {
-  return (t.b + nt[1] * t.c) & (kWarps - 1);
-}
 
 // the weights of one face of the tile (tap-major rows of X faces in shared
 // memory)
@@ -155,8 +139,9 @@ struct FluxTile {
   // stencil and limiter windows of the tile's faces
   static constexpr Box S = D == 0 ? Box{40, 8, 1, 1} : (D == 1 ? Box{32, 15, 1, 1} : Box{32, 1, 15, 1});
   static constexpr Box L = D == 0 ? Box{40, 8, 1, 1} : (D == 1 ? Box{32, 11, 1, 1} : Box{32, 1, 11, 1});
-  static constexpr Box WT = D == 0 ? kTap32 : kRec8;
-  static constexpr Box BN = D == 2 ? Box{32, 1, 8, 1} : Box{32, 8, 1, 1};
+  static constexpr int ROWS = kWarps;
+  static constexpr Box WT = D == 0 ? kTap40 : rec(8);
+  static constexpr Box BN = D == 0 ? Box{40, 8, 1, 1} : (D == 2 ? Box{32, 1, 8, 1} : Box{32, 8, 1, 1});
   static constexpr int SB = S.elems(), LB = L.elems();
   // slot layout in elements: W_h, limiter W, mags_h, mags, weights, B_n
   static constexpr int OFF_WH = 0;
@@ -181,59 +166,57 @@ struct alignas(64) FluxMaps {
   CUtensorMap wt;     // PDM weights of the tile's faces
   CUtensorMap bn[2];  // step-start face field (as wl: per parity in FP64)
   int nt[3];          // tiles: x, along the warps, third axis
+  uint64_t inv[2];    // inverse_of(nt[0]), inverse_of(nt[1])
 };
 
-// tile t of the flux sweep along D: its first cell / face on each axis
-struct TileAt {
+// a tile: its axis, its first cell or face on each axis, and the warp that
+// takes the row's upper boundary face (-1: not this tile's)
+struct alignas(16) Tile {
+  short D, end_warp;
   int x0, y0, z0;
 };
-// A tile index t = a + nt[0] * (b + nt[1] * c) as its three digits.  The
-// blocks walk the tiles in steps of the grid size, and adding the step's
-// digits with carries replaces the divisions by nt of every tile (about a
-// hundred integer instructions per thread and tile).
-struct Tile {
-  int a, b, c;
-};
-__device__ __forceinline__ Tile tile_of(const int nt[3], int t) {
-  const int r = t / nt[0];
-  return {t % nt[0], r % nt[1], r / nt[1]};
+// n / d for d > 1 from inv = floor(2^64 / d) + 1: exact while n d < 2^64
+__host__ __device__ constexpr uint64_t inverse_of(int d) { return d > 1 ? ~0ull / (uint64_t)d + 1 : 0; }
+__device__ __forceinline__ int div_by(int n, int d, uint64_t inv) {
+  return d > 1 ? (int)__umul64hi((uint64_t)n, inv) : n;
 }
-// p += s (s's digits below nt: one carry per digit at most)
-__device__ __forceinline__ void tile_add(Tile& p, const Tile& s, const int nt[3]) {
-  p.a += s.a;
-  int carry = p.a >= nt[0];
-  if (carry) p.a -= nt[0];
-  p.b += s.b + carry;
-  carry = p.b >= nt[1];
-  if (carry) p.b -= nt[1];
-  p.c += s.c + carry;
-}
-template <int D>
-__device__ __forceinline__ TileAt flux_at(const Tile& p) {
-  const int a = p.a, b = p.b, c = p.c;
-  TileAt T;
+// Tile r of the nt[0] x nt[1] x nt[2] tiles of a sweep along D, x fastest.
+// The feeding thread works this out and the others read it from shared
+// memory; its warp is the last of the block at every tile, so the two
+// divisions are products with the counts' inverses (FP64 EMF stage 1.81 ->
+// 1.76 ms per blast 256^3 step on B200).
+template <int D, bool EMF, int ROWS, class Maps>
+__device__ __forceinline__ Tile tile_of(const Params& P, const Maps& m, int r) {
+  const int* nt = m.nt;
+  const int q = div_by(r, nt[0], m.inv[0]), c = div_by(q, nt[1], m.inv[1]);
+  const int a = r - q * nt[0], b = q - c * nt[1];
+  Tile T;
+  T.D = D;
   T.x0 = NGH + 32 * a;
-  if constexpr (D == 2) {  // warps: faces along k, one row j
+  // the rows of a tile run along k where its windows do (flux along k, EMFs
+  // along i and j), along j otherwise
+  if constexpr (EMF ? D != 2 : D == 2) {
     T.y0 = NGH + c;
-    T.z0 = NGH + 8 * b;
-  } else {  // warps: rows along j (D = 0) or faces along j (D = 1), one plane k
-    T.y0 = NGH + 8 * b;
+    T.z0 = NGH + ROWS * b;
+  } else {
+    T.y0 = NGH + ROWS * b;
     T.z0 = NGH + c;
   }
+  // the warp of the row-end pass rotates over the row sets
+  constexpr bool ends = EMF ? D != 0 : D == 0;
+  T.end_warp = ends && row_end_face(P, T.x0) ? (short)((b + nt[1] * c) & (kWarps - 1)) : (short)-1;
   return T;
 }
 
 template <typename R, int D, bool BG>
 struct FluxStage {
-  static constexpr bool EMF = false;
   using F = FluxTile<D>;
   using Maps = FluxMaps;
-  static constexpr int ELEMS = F::ELEMS;
+  static constexpr int ELEMS = F::ELEMS, ROWS = F::ROWS;
   static constexpr int TX = F::TX;
 
-  __device__ static void issue(const Params& P, const Maps& m, int par, const Tile& t, R* s,
+  __device__ static void issue(const Params& P, const Maps& m, int par, const Tile& T, R* s,
                                uint64_t* bar) {
-    const TileAt T = flux_at<D>(t);
     const int f0 = D == 0 ? T.x0 : (D == 1 ? T.y0 : T.z0);  // first face along D
     // stencil windows start 4 cells before the first face, limiter windows
     // 2 (along i both start 4 before, keeping x aligned)
@@ -248,11 +231,9 @@ struct FluxStage {
     tma_load_4d(s + F::OFF_BN, &m.bn[par], bar, T.x0, T.y0, T.z0, D);
   }
 
-  // one face per thread
-  __device__ static void compute(const Params& P, const Work<R>& wk, const Maps& m, const R* s,
-                                 const Tile& t, int warp, int lane) {
-    const TileAt T = flux_at<D>(t);
-    const int row = warp, col = lane;
+  // the face in tile row `row` (a warp's row), column `col` (a lane's face)
+  __device__ __forceinline__ static void point(const Params& P, const Work<R>& wk, const R* s,
+                                               const Tile& T, int row, int col) {
     const int i = T.x0 + col, j = T.y0 + (D == 2 ? 0 : row), k = T.z0 + (D == 2 ? row : 0);
     if (!(i < NGH + P.n[0] + (D == 0) && j < NGH + P.n[1] + (D == 1) && k < NGH + P.n[2] + (D == 2)))
       return;
@@ -273,7 +254,7 @@ struct FluxStage {
     }
     constexpr int TS = D == 0 ? 1 : 32;  // stride of one stencil tap in the slot
     FaceWeights<R> Wt;
-    if constexpr (D == 0) load_tap<32>(s + F::OFF_W + col, Wt);
+    if constexpr (D == 0) load_tap<40>(s + F::OFF_W + col, Wt);
     else load_fw_smem(s + F::OFF_W + row * FW, Wt);
     const R bn = s[F::OFF_BN + row * F::BN.x + col];
     R L[6], Rt[6], mL[3], mR[3];
@@ -296,7 +277,8 @@ struct FluxStage {
       for (int u = 0; u < 4; u++) lim[u] = ms[a * F::LB + u * TS];
       recon_lr(v, lim, Wt, mL[a], mR[a]);
     }
-    flux_out<R, D, BG, false>(P, wk, lin(P, i, j, k), L, Rt, mL, mR, bn);
+    flux_out<R, D, BG, false>(P, wk, lin32(P, i, j, k), D == 0 ? j : (D == 1 ? k : i), L, Rt, mL, mR,
+                              bn);
   }
 };
 
@@ -311,14 +293,22 @@ struct FluxStage {
 //   D = 2 (p = i, q = j): lanes i faces, warps j faces, one k cell
 template <int D>
 struct EmfTile {
-  static constexpr Box V = D == 0 ? Box{32, 1, 15, 2} : (D == 1 ? Box{40, 1, 8, 2} : Box{40, 15, 1, 2});
-  static constexpr Box BHP = D == 0 ? Box{32, 1, 15, 1} : (D == 1 ? Box{40, 1, 8, 1} : Box{40, 15, 1, 1});
-  static constexpr Box BLP = D == 0 ? Box{32, 1, 11, 1} : (D == 1 ? Box{40, 1, 8, 1} : Box{40, 11, 1, 1});
-  static constexpr Box BHQ = D == 0 ? Box{32, 8, 8, 1} : (D == 1 ? Box{40, 1, 15, 1} : Box{40, 8, 1, 1});
-  static constexpr Box BLQ = D == 0 ? Box{32, 4, 8, 1} : (D == 1 ? Box{40, 1, 11, 1} : Box{40, 8, 1, 1});
-  static constexpr Box RHO = D == 0 ? Box{32, 2, 9, 1} : (D == 1 ? Box{40, 1, 9, 1} : Box{40, 9, 1, 1});
-  static constexpr Box WQ = D == 1 ? kTap40 : kRec8;
-  static constexpr Box WP = D == 0 ? kRec1 : (D == 1 ? kRec8 : kTap40);
+  // Rows of edges per tile.  A tile's fixed costs (its number, its eight
+  // copies, the barrier waits, the row halo of the windows) weigh on an edge's
+  // 530 instructions: two rows per warp share them, 16 instead of 8 taking
+  // the EMF stage of a blast 256^3 step on B200 from 1.76 to 1.55 ms (FP64)
+  // and 0.93 to 0.85 (FP32).  Along i 16 rows would leave no room for a
+  // second slot.
+  static constexpr int ROWS = D == 0 ? 8 : 16;
+  static constexpr int H7 = ROWS + 7, H3 = ROWS + 3, H1 = ROWS + 1;  // rows with the windows' halos
+  static constexpr Box V = D == 0 ? Box{32, 1, H7, 2} : (D == 1 ? Box{40, 1, ROWS, 2} : Box{40, H7, 1, 2});
+  static constexpr Box BHP = D == 0 ? Box{32, 1, H7, 1} : (D == 1 ? Box{40, 1, ROWS, 1} : Box{40, H7, 1, 1});
+  static constexpr Box BLP = D == 0 ? Box{32, 1, H3, 1} : (D == 1 ? Box{40, 1, ROWS, 1} : Box{40, H3, 1, 1});
+  static constexpr Box BHQ = D == 0 ? Box{32, 8, ROWS, 1} : (D == 1 ? Box{40, 1, H7, 1} : Box{40, ROWS, 1, 1});
+  static constexpr Box BLQ = D == 0 ? Box{32, 4, ROWS, 1} : (D == 1 ? Box{40, 1, H3, 1} : Box{40, ROWS, 1, 1});
+  static constexpr Box RHO = D == 0 ? Box{32, 2, H1, 1} : (D == 1 ? Box{40, 1, H1, 1} : Box{40, H1, 1, 1});
+  static constexpr Box WQ = D == 1 ? kTap40 : rec(ROWS);
+  static constexpr Box WP = D == 0 ? rec(1) : (D == 1 ? rec(ROWS) : kTap40);
   static constexpr int VF = V.x * V.y * V.z;  // elements of one V field
   static constexpr int OFF_V = 0;
   static constexpr int OFF_BHP = OFF_V + V.padded();
@@ -344,35 +334,19 @@ struct alignas(64) EmfMaps {
   CUtensorMap wq;      // weights of the q faces
   CUtensorMap wp;      // weights of the p faces
   int nt[3];
+  uint64_t inv[2];
 };
-
-template <int D>
-__device__ __forceinline__ TileAt emf_at(const Tile& p) {
-  const int a = p.a, b = p.b, c = p.c;
-  TileAt T;
-  T.x0 = NGH + 32 * a;
-  if constexpr (D == 2) {  // warps: faces along j, one plane k
-    T.y0 = NGH + 8 * b;
-    T.z0 = NGH + c;
-  } else {  // warps: faces along k, one row j
-    T.y0 = NGH + c;
-    T.z0 = NGH + 8 * b;
-  }
-  return T;
-}
 
 template <typename R, int D, bool BG>
 struct EmfStage {
-  static constexpr bool EMF = true;
   using E = EmfTile<D>;
   using Maps = EmfMaps;
-  static constexpr int ELEMS = E::ELEMS;
+  static constexpr int ELEMS = E::ELEMS, ROWS = E::ROWS;
   static constexpr int TX = E::TX;
   static constexpr int p = (D + 1) % 3, q = (D + 2) % 3;
 
-  __device__ static void issue(const Params& P, const Maps& m, int par, const Tile& t, R* s,
+  __device__ static void issue(const Params& P, const Maps& m, int par, const Tile& T, R* s,
                                uint64_t* bar) {
-    const TileAt T = emf_at<D>(t);
     const int x0 = T.x0, y0 = T.y0, z0 = T.z0;
     if constexpr (D == 0) {  // i cells, j face y0, k faces z0..
       tma_load_4d(s + E::OFF_V, &m.v, bar, x0, y0, z0 - 4, 0);
@@ -404,26 +378,9 @@ struct EmfStage {
     }
   }
 
-  // one edge per thread; the edges along j and k (lanes on i faces) take
-  // the row's upper boundary face in the last tile of a row when 32
-  // divides n (row_end_face)
-  __device__ static void compute(const Params& P, const Work<R>& wk, const Maps& m, const R* s,
-                                 const Tile& t, int warp, int lane) {
-    const TileAt T = emf_at<D>(t);
-    edge(P, wk, s, T, warp, lane);
-    if constexpr (D != 0)
-      if (row_end_face(P, T.x0) && warp == row_end_warp(m.nt, t) && lane < kWarps)
-        row_end(P, wk, s, T, lane);
-  }
-  __device__ __forceinline__ static void row_end(const Params& P, const Work<R>& wk, const R* s,
-                                                const TileAt T, int row) {
-    edge(P, wk, s, T, row, 32);
-  }
-
-  // the edge in tile row `row` (a warp's row), column `col` (a lane's edge)
-  __device__ static void edge(const Params& P, const Work<R>& wk, const R* s, const TileAt& T,
-                              int row, int col) {
-    const int warp = row, lane = col;
+  // the edge in tile row `warp` (a warp's row), column `lane` (a lane's edge)
+  __device__ __forceinline__ static void point(const Params& P, const Work<R>& wk, const R* s,
+                                               const Tile& T, int warp, int lane) {
     const int i = T.x0 + lane, j = T.y0 + (D == 2 ? warp : 0), k = T.z0 + (D == 2 ? 0 : warp);
     if (!(i < NGH + P.n[0] + (D != 0) && j < NGH + P.n[1] + (D != 1) && k < NGH + P.n[2] + (D != 2)))
       return;
@@ -497,7 +454,7 @@ struct EmfStage {
       for (int u = 0; u < 4; u++) lim[u] = bql[u * tp];
       recon_lr(v, lim, Wp, bqL, bqR);
     }
-    const long long x = lin(P, i, j, k);
+    const int x = lin32(P, i, j, k);
     const size_t fs = P.fs;
     R b0p = R(0), b0q = R(0);
     if constexpr (BG) {  // B0 averaged along the edge (B0Aedge*)
@@ -511,124 +468,217 @@ struct EmfStage {
 
 // ------------------------------------------------------------- pipeline
 
-template <class Stage, typename R>
-__host__ __device__ constexpr int slot_bytes() {
-  return Stage::ELEMS * (int)sizeof(R);
-}
-// Slots in a block's ring: as many as fit the SM's 228 KB of shared memory
-// at SweepCfg::CTAS blocks per SM (each block also reserves 1 KB), at least
-// SweepCfg::STAGES, at most GOP_SWEEP_MAX_STAGES.  The small slots of the
-// edge-EMF sweeps get 3-4: their tiles compute for less time than the
-// copies of the next take to land.
-template <class Stage, typename R>
-__host__ __device__ constexpr int ring_slots() {
-  using Cfg = SweepCfg<R, Stage::EMF>;
-  constexpr int per_block = 228 * 1024 / Cfg::CTAS - 1024 - 128 - 64;
-  constexpr int fit = per_block / slot_bytes<Stage, R>();
-  return fit < Cfg::STAGES ? Cfg::STAGES
-                                   : (fit > GOP_SWEEP_MAX_STAGES ? GOP_SWEEP_MAX_STAGES : fit);
-}
-template <class Stage, typename R>
-__host__ __device__ constexpr int sweep_smem() {
-  return ring_slots<Stage, R>() * slot_bytes<Stage, R>() + 2 * ring_slots<Stage, R>() * 8 + 128;
-}
+// A stage's three sweeps as one launch: the stage of each axis, their tensor
+// maps, and the order in which the axes' tiles are taken.
+// MASK: the axes it is compiled for (bit d).
+template <typename R, bool EMF_, bool BG, unsigned MASK_>
+struct Sweep {
+  static constexpr bool EMF = EMF_;
+  static constexpr unsigned MASK = MASK_;
+  static constexpr bool H0 = MASK & 1, H1 = MASK >> 1 & 1, H2 = MASK >> 2 & 1;
+  template <int D>
+  using Stage = typename std::conditional<EMF, EmfStage<R, D, BG>, FluxStage<R, D, BG>>::type;
+  using Maps = typename Stage<0>::Maps;
+  static constexpr int max3(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
+  // a slot holds the tile of any axis
+  static constexpr int ELEMS = max3(H0 ? Stage<0>::ELEMS : 0, H1 ? Stage<1>::ELEMS : 0,
+                                    H2 ? Stage<2>::ELEMS : 0);
+  static constexpr int SLOT = ELEMS * (int)sizeof(R);
+  static constexpr int CTAS = SweepCfg<R, EMF>::CTAS;
+  // Slots in a block's ring: as many as fit the SM's 228 KB of shared memory
+  // at CTAS blocks per SM (each block also reserves 1 KB), at least
+  // SweepCfg::STAGES, at most GOP_SWEEP_MAX_STAGES
+  static constexpr int fit = (228 * 1024 / CTAS - 1024 - 128 - 256) / SLOT;
+  static constexpr int S = fit < SweepCfg<R, EMF>::STAGES
+                               ? SweepCfg<R, EMF>::STAGES
+                               : (fit > GOP_SWEEP_MAX_STAGES ? GOP_SWEEP_MAX_STAGES : fit);
+  static constexpr int SMEM = S * SLOT + S * (2 * 8 + (int)sizeof(Tile)) + 128;
+};
+template <class Maps>
+struct alignas(64) SweepMaps {
+  Maps m[3];
+  int first[4];  // the tiles of axis order[g] are first[g] .. first[g + 1] - 1
+  int order[3];
+};
 
 // Persistent sweep: lane 0 of warp 0 also feeds the ring.  It fills the
 // first S slots, and after each tile waits until all 8 warps have released
-// that tile's slot, then issues the tile S ahead into it; the
-// other warps meanwhile compute the next tile, whose copies were issued a
-// tile earlier.  Every wait is bounded; a block that gives up records the
-// failure in S_FLAGS (2) and drains its copies in flight before it exits.
-template <class Stage, typename R>
+// that tile's slot, then issues the next tile into it; the
+// other warps meanwhile compute the tile whose copies were issued S - 1 tiles
+// earlier.  Always the same warp: it runs a little behind the others and so
+// finds the slot released (with the warps taking turns every tile waited for
+// its slowest warp: FP64 flux 2.34 -> 2.90 ms per blast 256^3 step on B200).
+// Every wait is bounded; a block that gives up records the failure in S_FLAGS
+// (2) and waits for its copies in flight before it exits.
+//
+// The tiles of several axes run through one launch.  Their number is rarely
+// a multiple of the blocks the GPU holds, so three launches leave three
+// partly filled last waves, and each starts with an empty ring (a barrier
+// set-up and a copy's latency, about 5 us): flux and EMF stage of an FP64 step
+// on B200, Orszag-Tang 64x64x4 32 + 21 -> 13 + 13 us, blast 64^3 84 + 54 -> 54
+// + 41 us.
+//
+// A block takes its first tile by its number and each further one from a
+// counter (S_TILE), so the tiles in flight at any time are neighbours.  With
+// tiles dealt out in turn (t + grid, t + 2 grid, ...) the blocks whose tiles
+// take longer -- always the same ones where the row's tiles divide the grid:
+// the row-end tiles -- fell behind, and neighbours along i, which share
+// memory lines at their common edge, met them at different times (FP64 flux
+// stage of a blast 256^3 step 3.16 ms, with the counter 2.40).  In a batch a block that starts late finds less work left.
+template <class SW, typename R>
 __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
-                                          const typename Stage::Maps& maps) {
+                                          const SweepMaps<typename SW::Maps>& maps) {
   // stop flag, or an earlier pipeline wait that timed out: do nothing
   if (stopped(P) || P.scal[S_FLAGS] == 2.0) return;
-  constexpr int S = ring_slots<Stage, R>();
-  constexpr int SLOT = slot_bytes<Stage, R>();
-  constexpr int TXB = Stage::TX * (int)sizeof(R);  // bytes the copies of one tile deliver
-  static_assert(TXB <= SLOT, "slot holds its boxes");
+  constexpr int S = SW::S;
+  using S0 = typename SW::template Stage<0>;
+  using S1 = typename SW::template Stage<1>;
+  using S2 = typename SW::template Stage<2>;
+  static_assert((!SW::H0 || S0::TX <= SW::ELEMS) && (!SW::H1 || S1::TX <= SW::ELEMS) &&
+                    (!SW::H2 || S2::TX <= SW::ELEMS),
+                "slot holds its boxes");
   extern __shared__ unsigned char smem_dyn[];
   // TMA destinations on 128-byte boundaries (the launch adds 128 bytes)
   unsigned char* base = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_dyn) + 127) & ~static_cast<uintptr_t>(127));
   R* slots = reinterpret_cast<R*>(base);
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + S * SLOT);
+  Tile* tiles = reinterpret_cast<Tile*>(base + S * SW::SLOT);
+  uint64_t* full = reinterpret_cast<uint64_t*>(tiles + S);
   uint64_t* empty = full + S;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool feeder = threadIdx.x == 0;
-  const int nt2 = maps.nt[2];  // tiles run out when the third digit reaches it
+  const int ntiles = maps.first[3];
   const int par = sizeof(R) == 8 ? cur_buf(P) : 0;
-  auto issue = [&](int n, const Tile& t) {
-    const int q = n % S;
-    mbar_arrive_expect_tx(&full[q], TXB);
-    Stage::issue(P, maps, par, t, slots + (size_t)q * Stage::ELEMS, &full[q]);
+  // the feeder: tile t into slot q
+  auto issue = [&](int q, int t) {
+    const int g = (t >= maps.first[1]) + (t >= maps.first[2]), r = t - maps.first[g];
+    R* slot = slots + (size_t)q * SW::ELEMS;
+    uint64_t* bar = &full[q];
+    auto go = [&](auto stage, auto d) {
+      using St = decltype(stage);
+      constexpr int D = decltype(d)::value;
+      if constexpr (!(SW::MASK >> D & 1)) return;
+      const Tile T = tile_of<D, SW::EMF, St::ROWS>(P, maps.m[D], r);
+      tiles[q] = T;
+      mbar_arrive_expect_tx(bar, St::TX * (int)sizeof(R));
+      St::issue(P, maps.m[D], par, T, slot, bar);
+    };
+    const int D = maps.order[g];
+    if (SW::H0 && (SW::MASK == 1 || D == 0)) go(S0{}, std::integral_constant<int, 0>{});
+    else if (SW::H1 && (SW::MASK == 2 || D == 1)) go(S1{}, std::integral_constant<int, 1>{});
+    else go(S2{}, std::integral_constant<int, 2>{});
   };
-  const Tile step = tile_of(maps.nt, gridDim.x);
-  Tile next = tile_of(maps.nt, blockIdx.x);  // feeder only: the first tile not yet issued
-  int issued = 0;                            // feeder only: tiles whose copies were issued
+  // the two counters of S_TILE: tiles handed out beyond the first of each
+  // block, blocks done
+  unsigned* counters = reinterpret_cast<unsigned*>(P.scal + S_TILE);
+  const bool feeder = threadIdx.x == 0;
+  int next = blockIdx.x;  // feeder only: the next tile to issue
+  int issued = 0;         // feeder only: tiles whose copies were issued
+  bool more = true;       // feeder only: the end has not been passed on
+  // the feeder: the next tile into slot q, or the end of the work
+  auto feed = [&](int q) {
+    if (next < ntiles) {
+      const int t = next;
+      next = gridDim.x + (int)atomicAdd(counters, 1u);  // used a tile later
+      issue(q, t);
+      issued++;
+    } else {
+      tiles[q].D = -1;
+      mbar_arrive(&full[q]);
+      more = false;
+    }
+  };
   if (feeder) {
     for (int q = 0; q < S; q++) {
       mbar_init(&full[q], 1);
       mbar_init(&empty[q], kWarps);
     }
     fence_mbar_init();
-    for (; next.c < nt2 && issued < S; tile_add(next, step, maps.nt)) issue(issued++, next);
+    for (int q = 0; q < S && more; q++) feed(q);
   }
   __syncthreads();
   bool ok = true;
-  int n = 0;
-  for (Tile t = tile_of(maps.nt, blockIdx.x); t.c < nt2; tile_add(t, step, maps.nt), n++) {
-    const int q = n % S;
-    const uint32_t ph = (n / S) & 1;
+  int q = 0;
+  uint32_t ph = 0;
+  for (;;) {
     if (!mbar_wait(&full[q], ph)) {
       ok = false;
       break;
     }
-    Stage::compute(P, wk, maps, slots + (size_t)q * Stage::ELEMS, t, warp, lane);
+    const Tile T = tiles[q];
+    if (T.D < 0) break;
+    const R* slot = slots + (size_t)q * SW::ELEMS;
+    auto rows = [&](auto stage) {
+      using St = decltype(stage);
+      int row = warp, col = lane;
+#pragma unroll 1
+      for (;;) {
+        St::point(P, wk, slot, T, row, col);
+        if (St::ROWS > kWarps && col < 32 && row + kWarps < St::ROWS) {
+          row += kWarps;
+          continue;
+        }
+        // the row-end pass: column 32 of the tile's rows
+        if (warp != T.end_warp || col == 32 || lane >= St::ROWS) break;
+        row = lane;
+        col = 32;
+      }
+    };
+    if constexpr (SW::MASK == 1) rows(S0{});
+    else if constexpr (SW::MASK == 2) rows(S1{});
+    else if constexpr (SW::MASK == 4) rows(S2{});
+    else {
+      if (SW::H0 && T.D == 0) rows(S0{});
+      else if (T.D == 1) rows(S1{});
+      else rows(S2{});
+    }
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[q]);
-    if (feeder && next.c < nt2) {
-      // every warp has released this slot: refill it with the tile S ahead
+    if (feeder && more) {
+      // every warp has released this slot: refill it
       if (!mbar_wait(&empty[q], ph)) {
         ok = false;
         break;
       }
-      issue(issued++, next);
-      tile_add(next, step, maps.nt);
+      feed(q);
+    }
+    if (++q == S) {
+      q = 0;
+      ph ^= 1;
     }
   }
   if (feeder) {
-    // the copies of the tiles issued last must land before the block exits
-    for (int k = issued > S ? issued - S : 0; k < issued; k++)
-      if (!mbar_wait(&full[k % S], (k / S) & 1)) ok = false;
+    // A block that gave up lets the copies of the tiles issued last land
+    // before it exits (at the end of the work all have been waited for; the
+    // slot that carries the end had been released)
+    if (!ok) {
+      const int k0 = issued - S + (more ? 0 : 1);
+      for (int k = k0 > 0 ? k0 : 0; k < issued; k++) mbar_wait(&full[k % S], (k / S) & 1);
+    }
+    // the last block leaves the counters at zero for the next launch
+    if (atomicAdd(counters + 1, 1u) == gridDim.x - 1) {
+      counters[0] = 0;
+      counters[1] = 0;
+    }
   }
   if (!ok) P.scal[S_FLAGS] = 2.0;
 }
 
-template <typename R, int D, bool BG>
-__global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, false>::CTAS))
-    k_flux_sweep(Params P, Work<R> wk, const __grid_constant__ FluxMaps maps) {
+template <typename R, bool EMF, bool BG, unsigned MASK>
+__global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, EMF>::CTAS))
+    k_sweep(Params P, Work<R> wk,
+            const __grid_constant__ SweepMaps<typename Sweep<R, EMF, BG, MASK>::Maps> maps) {
   pdl_enter();
-  sweep_run<FluxStage<R, D, BG>, R>(P, wk, maps);
+  sweep_run<Sweep<R, EMF, BG, MASK>, R>(P, wk, maps);
 }
 
-template <typename R, int D, bool BG>
-__global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, true>::CTAS))
-    k_emf_sweep(Params P, Work<R> wk, const __grid_constant__ EmfMaps maps) {
-  pdl_enter();
-  sweep_run<EmfStage<R, D, BG>, R>(P, wk, maps);
-}
-
-template <typename R, int D>
+template <typename R, unsigned MASK>
 constexpr bool smem_fits() {
-  return (size_t)sweep_smem<FluxStage<R, D, false>, R>() * SweepCfg<R, false>::CTAS <= 228 * 1024 &&
-         (size_t)sweep_smem<EmfStage<R, D, false>, R>() * SweepCfg<R, true>::CTAS <= 228 * 1024;
+  using F = Sweep<R, false, false, MASK>;
+  using E = Sweep<R, true, false, MASK>;
+  return (F::SMEM + 1024) * F::CTAS <= 228 * 1024 && (E::SMEM + 1024) * E::CTAS <= 228 * 1024;
 }
-static_assert(smem_fits<double, 0>() && smem_fits<double, 1>() && smem_fits<double, 2>(),
-              "FP64 sweep blocks per SM");
-static_assert(smem_fits<float, 0>() && smem_fits<float, 1>() && smem_fits<float, 2>(),
-              "FP32 sweep blocks per SM");
+static_assert(smem_fits<double, 7>() && smem_fits<double, 1>(), "FP64 sweep blocks per SM");
+static_assert(smem_fits<float, 7>() && smem_fits<float, 1>(), "FP32 sweep blocks per SM");
 
 // ------------------------------------------------------------------ host
 
@@ -680,7 +730,7 @@ static bool field_map(CUtensorMap* m, const R* base, int nf, const Params& P, co
 template <typename R>
 static bool weight_map(CUtensorMap* m, const Work<R>& w, const Params& P, const Box& b) {
   const cuuint64_t es = sizeof(R), tm = (cuuint64_t)P.tmax;
-  if (b.y == kTap32.y && (b.x == kTap32.x || b.x == kTap40.x)) {
+  if (b.y == kTap40.y && b.x == kTap40.x) {
     const cuuint64_t d[4] = {tm, (cuuint64_t)NTAB, 3, 1};
     const cuuint64_t st[3] = {tm * es, tm * NTAB * es, tm * NTAB * 3 * es};
     return encode<R>(m, w.tab, d, st, b);
@@ -712,8 +762,8 @@ static bool make_flux_maps(FluxMaps& m, const Params& P, const Work<R>& w) {
     ok = field_map<R>(&m.wl[b], lim_state<R>(P, w, b), 6, P, L5) &&
          field_map<R>(&m.bn[b], lim_face<R>(P, w, b), 3, P, F::BN);
   const int n0 = P.n[0], n1 = P.n[1], n2 = P.n[2];
-  if (D == 0) {  // i-face tiles (the row-end faces by k_flux_col), j-row tiles, k planes
-    m.nt[0] = flux_col<R>() ? (n0 + 31) / 32 : (n0 + 1 + 31) / 32;
+  if (D == 0) {  // i-face tiles (the row-end face in the last), j-row tiles, k planes
+    m.nt[0] = (n0 + 31) / 32;
     m.nt[1] = (n1 + 7) / 8;
     m.nt[2] = n2;
   } else if (D == 1) {  // i tiles, j-face tiles, k planes
@@ -725,6 +775,7 @@ static bool make_flux_maps(FluxMaps& m, const Params& P, const Work<R>& w) {
     m.nt[1] = (n2 + 1 + 7) / 8;
     m.nt[2] = n1;
   }
+  for (int a = 0; a < 2; a++) m.inv[a] = inverse_of(m.nt[a]);
   return ok;
 }
 
@@ -740,34 +791,36 @@ static bool make_emf_maps(EmfMaps& m, const Params& P, const Work<R>& w) {
   const int n0 = P.n[0], n1 = P.n[1], n2 = P.n[2];
   if (D == 0) {  // i-cell tiles, k-face tiles, j faces
     m.nt[0] = (n0 + 31) / 32;
-    m.nt[1] = (n2 + 1 + 7) / 8;
+    m.nt[1] = (n2 + E::ROWS) / E::ROWS;
     m.nt[2] = n1 + 1;
   } else if (D == 1) {  // i-face tiles (the row-end face in the last), k-face tiles, j cells
     m.nt[0] = (n0 + 31) / 32;
-    m.nt[1] = (n2 + 1 + 7) / 8;
+    m.nt[1] = (n2 + E::ROWS) / E::ROWS;
     m.nt[2] = n1;
   } else {  // i-face tiles (the row-end face in the last), j-face tiles, k cells
     m.nt[0] = (n0 + 31) / 32;
-    m.nt[1] = (n1 + 1 + 7) / 8;
+    m.nt[1] = (n1 + E::ROWS) / E::ROWS;
     m.nt[2] = n2;
   }
+  for (int a = 0; a < 2; a++) m.inv[a] = inverse_of(m.nt[a]);
   return ok;
 }
 
 struct SweepSet {
-  FluxMaps flux[3];
-  EmfMaps emf[3];
+  SweepMaps<FluxMaps> flux;
+  SweepMaps<EmfMaps> emf;
   int sms = 0;
 };
 
-template <typename R, int D, bool BG>
-static cudaError_t allow_smem() {
-  cudaError_t e = cudaFuncSetAttribute(k_flux_sweep<R, D, BG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       sweep_smem<FluxStage<R, D, BG>, R>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_emf_sweep<R, D, BG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             sweep_smem<EmfStage<R, D, BG>, R>());
-  return e;
+template <typename R, bool EMF, bool BG, unsigned MASK>
+static bool allow_smem() {
+  return cudaFuncSetAttribute(k_sweep<R, EMF, BG, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              Sweep<R, EMF, BG, MASK>::SMEM) == cudaSuccess;
+}
+template <typename R, bool BG>
+static bool allow_smem() {
+  return allow_smem<R, false, BG, 1>() && allow_smem<R, false, BG, 2>() && allow_smem<R, false, BG, 4>() &&
+         allow_smem<R, false, BG, 7>() && allow_smem<R, true, BG, 7>();
 }
 
 template <typename R>
@@ -777,12 +830,10 @@ SweepSet* sweep_create(const Params& P, const Work<R>& w) {
   int dev = 0;
   bool ok = cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
-  ok = ok && make_flux_maps<R, 0>(s->flux[0], P, w) && make_flux_maps<R, 1>(s->flux[1], P, w) &&
-       make_flux_maps<R, 2>(s->flux[2], P, w) && make_emf_maps<R, 0>(s->emf[0], P, w) &&
-       make_emf_maps<R, 1>(s->emf[1], P, w) && make_emf_maps<R, 2>(s->emf[2], P, w);
-  ok = ok && allow_smem<R, 0, false>() == cudaSuccess && allow_smem<R, 1, false>() == cudaSuccess &&
-       allow_smem<R, 2, false>() == cudaSuccess && allow_smem<R, 0, true>() == cudaSuccess &&
-       allow_smem<R, 1, true>() == cudaSuccess && allow_smem<R, 2, true>() == cudaSuccess;
+  ok = ok && make_flux_maps<R, 0>(s->flux.m[0], P, w) && make_flux_maps<R, 1>(s->flux.m[1], P, w) &&
+       make_flux_maps<R, 2>(s->flux.m[2], P, w) && make_emf_maps<R, 0>(s->emf.m[0], P, w) &&
+       make_emf_maps<R, 1>(s->emf.m[1], P, w) && make_emf_maps<R, 2>(s->emf.m[2], P, w);
+  ok = ok && allow_smem<R, false>() && allow_smem<R, true>();
   if (!ok) {
     cudaGetLastError();
     delete s;
@@ -795,18 +846,23 @@ template SweepSet* sweep_create<float>(const Params&, const Work<float>&);
 
 void sweep_destroy(SweepSet* s) { delete s; }
 
-template <class Stage, typename R, class Maps, class K>
+// the tiles of the axes SW is compiled for, in the given order
+template <class SW, typename R, class K>
 static void launch_persistent(K kern, const SweepSet* sw, const Params& P, const Work<R>& w,
-                              const Maps& m, cudaStream_t st) {
-  const int ntiles = m.nt[0] * m.nt[1] * m.nt[2];
-  const int grid = std::max(1, std::min(ntiles, sw->sms * SweepCfg<R, Stage::EMF>::CTAS));
+                              SweepMaps<typename SW::Maps> m, const int order[3], cudaStream_t st) {
+  m.first[0] = 0;
+  for (int g = 0; g < 3; g++) {
+    const int D = m.order[g] = order[g], *nt = m.m[D].nt;
+    m.first[g + 1] = m.first[g] + (SW::MASK >> D & 1 ? nt[0] * nt[1] * nt[2] : 0);
+  }
+  const int grid = std::min(m.first[3], sw->sms * SW::CTAS);
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kSweepThreads);
-  cfg.dynamicSmemBytes = sweep_smem<Stage, R>();
+  cfg.dynamicSmemBytes = SW::SMEM;
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = GOP_SWEEP_PDL ? 1 : 0;
@@ -814,49 +870,61 @@ static void launch_persistent(K kern, const SweepSet* sw, const Params& P, const
   count_launches(1);
 }
 
-template <typename R, int D, bool BG>
-static void launch_flux_d(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
-  launch_persistent<FluxStage<R, D, BG>, R>(k_flux_sweep<R, D, BG>, sw, P, w, sw->flux[D], st);
+template <typename R, bool EMF, bool BG, unsigned MASK, class Maps>
+static void launch_mask(const SweepSet* sw, const Params& P, const Work<R>& w, const Maps& m,
+                        const int order[3], cudaStream_t st) {
+  launch_persistent<Sweep<R, EMF, BG, MASK>, R>(k_sweep<R, EMF, BG, MASK>, sw, P, w, m, order, st);
 }
-template <typename R, int D, bool BG>
-static void launch_emf_d(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
-  launch_persistent<EmfStage<R, D, BG>, R>(k_emf_sweep<R, D, BG>, sw, P, w, sw->emf[D], st);
+// The axes of a stage in one launch, or (flux) one launch each where each
+// axis alone keeps the GPU busy for long: the kernels of one axis are about 3 %
+// faster per tile (a third of the code, registers left over), which beats the
+// two waves and fills saved from about 128 tiles per resident block on.  Blast
+// on B200, flux stage per step, one launch / three: FP64 128^3 321 / 334 us,
+// 192^3 1034 / 1022, 256^3 2405 / 2342; FP32 217 / 228, 695 / 684, 1620 / 1566.
+// EMF tiles are shorter and gain by the common launch at every size (FP32
+// 128^3 120 / 137, 256^3 854 / 851).
+constexpr int kTilesApart = 128;
+template <typename R, bool EMF, bool BG, class Maps>
+static void launch_axes(const SweepSet* sw, const Params& P, const Work<R>& w, const Maps& m,
+                        const int order[3], cudaStream_t st) {
+  if constexpr (!EMF) {
+    long long tiles = 0;
+    for (int d = 0; d < 3; d++) tiles += (long long)m.m[d].nt[0] * m.m[d].nt[1] * m.m[d].nt[2];
+    if (tiles >= (long long)kTilesApart * sw->sms * SweepCfg<R, false>::CTAS) {
+      for (int g = 0; g < 3; g++) {
+        if (order[g] == 0) launch_mask<R, EMF, BG, 1>(sw, P, w, m, order, st);
+        else if (order[g] == 1) launch_mask<R, EMF, BG, 2>(sw, P, w, m, order, st);
+        else launch_mask<R, EMF, BG, 4>(sw, P, w, m, order, st);
+      }
+      return;
+    }
+  }
+  launch_mask<R, EMF, BG, 7>(sw, P, w, m, order, st);
 }
 
 template <typename R>
-bool launch_flux_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, int D,
+bool launch_flux_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, const int order[3],
                        cudaStream_t st) {
   if (!sw || P.ps_live) return false;  // the entropy channel runs the per-face kernels
-  const bool bg = P.bg != nullptr;
-  switch (D) {
-    case 0:
-      bg ? launch_flux_d<R, 0, true>(sw, P, w, st) : launch_flux_d<R, 0, false>(sw, P, w, st);
-      if (flux_col<R>() && P.n[0] % 32 == 0) launch_flux_col<R>(P, w, st);
-      break;
-    case 1: bg ? launch_flux_d<R, 1, true>(sw, P, w, st) : launch_flux_d<R, 1, false>(sw, P, w, st); break;
-    default: bg ? launch_flux_d<R, 2, true>(sw, P, w, st) : launch_flux_d<R, 2, false>(sw, P, w, st); break;
-  }
+  if (P.bg) launch_axes<R, false, true>(sw, P, w, sw->flux, order, st);
+  else launch_axes<R, false, false>(sw, P, w, sw->flux, order, st);
   return true;
 }
-template bool launch_flux_sweep<double>(const SweepSet*, const Params&, const Work<double>&, int,
-                                        cudaStream_t);
-template bool launch_flux_sweep<float>(const SweepSet*, const Params&, const Work<float>&, int,
-                                       cudaStream_t);
-
 template <typename R>
-bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, int D, cudaStream_t st) {
+bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, const int order[3],
+                      cudaStream_t st) {
   if (!sw) return false;
-  const bool bg = P.bg != nullptr;
-  switch (D) {
-    case 0: bg ? launch_emf_d<R, 0, true>(sw, P, w, st) : launch_emf_d<R, 0, false>(sw, P, w, st); break;
-    case 1: bg ? launch_emf_d<R, 1, true>(sw, P, w, st) : launch_emf_d<R, 1, false>(sw, P, w, st); break;
-    default: bg ? launch_emf_d<R, 2, true>(sw, P, w, st) : launch_emf_d<R, 2, false>(sw, P, w, st); break;
-  }
+  if (P.bg) launch_axes<R, true, true>(sw, P, w, sw->emf, order, st);
+  else launch_axes<R, true, false>(sw, P, w, sw->emf, order, st);
   return true;
 }
-template bool launch_emf_sweep<double>(const SweepSet*, const Params&, const Work<double>&, int,
-                                       cudaStream_t);
-template bool launch_emf_sweep<float>(const SweepSet*, const Params&, const Work<float>&, int,
-                                      cudaStream_t);
+#define GOP_INST(R)                                                                            \
+  template bool launch_flux_sweep<R>(const SweepSet*, const Params&, const Work<R>&,            \
+                                     const int[3], cudaStream_t);                     \
+  template bool launch_emf_sweep<R>(const SweepSet*, const Params&, const Work<R>&,             \
+                                    const int[3], cudaStream_t);
+GOP_INST(double)
+GOP_INST(float)
+#undef GOP_INST
 
 }  // namespace gop

@@ -150,9 +150,10 @@ int gop_get_stats(gop_instance *h, gop_stats *out);
 /* Autotuner: times candidate thread-block shapes for each of the 11
  * tunable launches of a step on the instance's current state (after
  * gop_prepare; the state is not advanced) and keeps the fastest for the
- * following steps; then the order of the three flux launches and of the
- * three edge-EMF launches (each order a rotation of the axes; the launches
- * are independent, so no result changes), timing two whole steps per
+ * following steps, and for the flux and the edge-EMF stage the tile-staged
+ * sweep where that beats their three launches; then the order of the axes in
+ * the flux stage and in the edge-EMF stage (each order a rotation of the axes;
+ * they are independent, so no result changes), timing two whole steps per
  * rotation with the state restored after each.  reps: timed launches per
  * candidate (0 = 3); chosen (optional, 11 ints) receives the picked
  * candidate index per launch. */

@@ -925,11 +925,11 @@ static const dim3 kBlockCandidates[] = {dim3(32, 4, 2), dim3(32, 8, 1), dim3(32,
                                         dim3(8, 32, 1),  dim3(8, 4, 8)};
 static const int kNumBlockCandidates = sizeof(kBlockCandidates) / sizeof(kBlockCandidates[0]);
 
-// one step's launches: begin, the stages, the ghost fill, end
+// one step's launches: the stages, the ghost fill with the turn to the next
+// step (the begin and end groups hold no launch of their own)
 static void enqueue_one_step(gop_instance* h, cudaStream_t st, const Hook& hook) {
   const Params& P = h->P;
   hook(G_BEGIN, 1);
-  launch_begin(P, st);
   hook(G_BEGIN, 0);
   if (h->d.precision == GOP_PREC_MIXED)
     launch_step_body<float>(P, h->d.coord, h->wf, st, h->tune, h->sweep, hook);
@@ -939,7 +939,6 @@ static void enqueue_one_step(gop_instance* h, cudaStream_t st, const Hook& hook)
   launch_ghosts(P, h->d.bc, h->d.gem_bc, 0, st);
   hook(G_GHOST, 0);
   hook(G_END, 1);
-  launch_end(P, st);
   hook(G_END, 0);
 }
 
@@ -1102,6 +1101,10 @@ int gop_autotune(gop_instance* h, int reps, int* chosen) {
   CK(cudaMemcpyAsync(h->hscal, h->scal, NSCAL * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
   std::vector<double> saved_scal(h->hscal, h->hscal + NSCAL);
+  // (the last step of a call sets the stop flag, which makes launches return
+  // at once)
+  h->hscal[S_STOP] = 0.0;
+  CK(cudaMemcpyAsync(h->scal, h->hscal, NSCAL * sizeof(double), cudaMemcpyHostToDevice, h->st));
   cur = saved_scal[S_PAR] != 0.0 ? 1 : 0;
   double* hist = nullptr;
   const size_t wbytes = (size_t)P.fs * 6 * sizeof(double), bbytes = (size_t)P.fs * 3 * sizeof(double);

@@ -70,8 +70,8 @@ enum Scal : int {
   S_BUDGET,      // steps left in the current gop_step call
   S_PSNZ,        // gop_prepare's check: nonzero if some p_S of the state or
                  // of its AB2 history is nonzero
-  S_TILE,        // two 32-bit counters of the running sweep launch: tiles
-                 // handed out, blocks done; zero between launches
+  S_TILE,        // two 32-bit counters of the running launch: tiles handed
+                 // out (sweeps), blocks done; zero between launches
   NSCAL
 };
 

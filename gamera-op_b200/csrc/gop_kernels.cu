@@ -5,15 +5,18 @@
 // the sequence can be captured in a CUDA graph and replayed without host
 // synchronisation:
 //
-//   begin     dt <- running CFL minimum, time += dt, c = dt/(2 dt0)
 //   ab2       W_h, mags, mags_h, B_h over the ghost-extended grid
 //   c2c       centre-to-edge velocity, first sweep (3 edge directions)
 //   emf       centre-to-edge second sweep, face-B reconstruction, edge EMF
 //   flux      PDM reconstruction + Rusanov flux + Maxwell stress per face
 //   update    divergence, sources, constrained transport, cons->prim,
 //             floors, Alfven/Boris correction, next CFL dt, max|div B|
-//   ghost     periodic wrap and boundary fills of the new state
-//   end       the written buffer becomes the current state
+//   ghost     periodic wrap and boundary fills of the new state; its last
+//             block ends the step (the written buffer becomes the current
+//             state) and opens the next one: dt <- running CFL minimum, time
+//             += dt, c = dt/(2 dt0)
+//
+// (the first step of a call is opened by k_arm, which sets its budget)
 //
 // Every stage is a per-point body function of a kernel whose launch grid
 // covers one grid; a batch of grids captures each member's launches on
@@ -900,83 +903,94 @@ __device__ __forceinline__ void dt_body(const Params& P, Pos t, double& dtc, dou
 
 // ---------------------------------------------------------------- ghosts
 
-// Periodic wrap of one axis for all 9 state fields (src/boundary_exchange.c,
-// index sets of src/setup_mpi.c:62-253), over the full transverse extent.
-// Space: (N[oa], N[ob], 2*NGH); sources (active layers) and destinations
-// (ghost layers) are disjoint for n >= NGH, so both sides go in one launch.
-__device__ __forceinline__ void wrap_body(const Params& P, int axis, int which, Pos t) {
-  // t = (i, j, k) with the component along `axis` replaced by the ghost
-  // layer 0..2*NGH-1, so lanes run along i (along the layers for axis 0)
-  int ijk[3] = {t.x, t.y, t.z};
-  const int lay = ijk[axis];
-  for (int a = 0; a < 3; a++)
-    if (ijk[a] >= (a == axis ? 2 * NGH : P.N[a])) return;
-  const int bsel = which ? cur_buf(P) : 1 - cur_buf(P);
-  double* __restrict__ W = P.Wbuf[bsel];
-  double* __restrict__ B = P.Bbuf[bsel];
-  const int N = P.N[axis];
-  const int side = lay / NGH, l = lay % NGH;
-  // the sources are active cells and the destinations ghost cells, so no
-  // thread writes what another reads: all 9 loads go out before the stores
-  long long src[2], dst[2];  // [0]: cell-centred fields, [1]: the face field along axis
-  for (int onface = 0; onface < 2; onface++) {
-    if (side == 0) {  // high ghosts <- low active
-      ijk[axis] = NGH + onface + l;
-      src[onface] = lin(P, ijk[0], ijk[1], ijk[2]);
-      ijk[axis] = N - NGH - 1 + onface + l;
-    } else {          // low ghosts <- high active
-      ijk[axis] = N - 2 * NGH - 1 + l;
-      src[onface] = lin(P, ijk[0], ijk[1], ijk[2]);
-      ijk[axis] = l;
+// The reference fills its ghost layers axis by axis: the periodic halos along
+// i, j and k (src/boundary_exchange.c, index sets of src/setup_mpi.c:62-253),
+// then the problem's fills face by face (src/boundary_conditions.c: gas_bc_*
+// and gem_bc_*), each over the full transverse extent, so that later fills
+// copy what earlier ones wrote at edges and corners.  Here every ghost point
+// finds the value it ends with: going back through the fills from the last,
+// each fill whose target holds the point moves it to that fill's source (with
+// its sign), until no fill applies.  That source is written by no fill, so
+// all points go at once, in one launch, where the fills took one each (6 for
+// a shell open on all sides: 52 -> GOP_GH_SH us of a 192x128x128 step on B200).
+
+// Where the value of a cell field (fa < 0) or of the face field along axis fa
+// at point x comes from: x moves to the source.  False: no fill writes the
+// point.  neg: the axes whose 'r' fills reflect the point (bit a) and, bit 3,
+// pole fills; fixed: the face of a fixed-state fill (-1: none); entropy: for
+// p_S, which the fixed-state fills leave alone.
+template <bool PERIODIC>
+__device__ __forceinline__ bool ghost_source(const Params& P, const GhostFill& G, const char* kind, int fa,
+                                             int x[3], int& neg, int& fixed, bool entropy = false) {
+  bool any = false;
+  neg = 0;
+  fixed = -1;
+  if constexpr (!PERIODIC) {
+#pragma unroll
+    for (int face = 5; face >= 0; face--) {
+      const int a = face / 2, side = face % 2, n = P.n[a], o = fa == a;
+      const int kd = kind[face];
+      const int l = side ? x[a] - (n + NGH + o) : x[a];
+      if (fixed >= 0 || G.per[a] || l < 0 || l >= NGH || kd == 'n') continue;
+      if ((fa >= 0 && kd == 'r') || (entropy && kd == 'f')) continue;  // gem_bc_reflective_* are empty
+      any = true;
+      if (kd == 'f') {
+        fixed = face;
+      } else if (kd == 'e') {
+        x[a] = side ? n + NGH - 1 + o : NGH;
+      } else {
+        x[a] = side ? n + NGH - 1 - l : 2 * NGH - 1 - l + o;
+        if (kd == 'r') neg ^= 1 << a;
+        // pole (j faces): mirrored across the axis half a turn away in phi
+        // (src/spherical/spherical_boundary.c:23-138)
+        if (kd == 'o') {
+          x[2] = NGH + (x[2] - NGH + P.n[2] / 2) % P.n[2];
+          neg ^= 8;
+        }
+      }
     }
-    dst[onface] = lin(P, ijk[0], ijk[1], ijk[2]);
-  }
-  const bool ps = P.ps_live != 0;  // p_S zero everywhere stays so: skipped
-  double v[9];
-#pragma unroll
-  for (int f = 0; f < 9; f++) {
-    const int o = (f >= 6 && f - 6 == axis) ? 1 : 0;
-    const double* a = f < 6 ? W + (size_t)f * P.fs : B + (size_t)(f - 6) * P.fs;
-    if (f != PS || ps) v[f] = a[src[o]];
   }
 #pragma unroll
-  for (int f = 0; f < 9; f++) {
-    const int o = (f >= 6 && f - 6 == axis) ? 1 : 0;
-    double* a = f < 6 ? W + (size_t)f * P.fs : B + (size_t)(f - 6) * P.fs;
-    if (f != PS || ps) a[dst[o]] = v[f];
+  for (int a = 2; a >= 0; a--) {
+    const int n = P.n[a], o = fa == a;
+    if (fixed >= 0 || !(PERIODIC || G.per[a])) continue;
+    if (x[a] < NGH) {
+      x[a] += n;
+      any = true;
+    } else if (x[a] >= n + NGH + o && x[a] < n + 2 * NGH + o) {
+      x[a] -= n;
+      any = true;
+    }
   }
+  return any;
 }
 
-// All three axes periodic: the three wraps above in one launch.  The three
-// in turn leave at every ghost point the value of the active point reached
-// by wrapping each of its ghost coordinates (x + n below the active range,
-// x - n above it): each later wrap copies what the earlier ones wrote, edges
-// and corners included.  Thread g runs over three slabs, axis a's 9 layers
-// (4 ghost layers below, 5 points above: the cell fields' 4 ghost layers
-// and the padding point, or the upper boundary face and the face field's 4
-// ghost layers) times all points of the other two axes; a (point, field)
-// pair is written by the slab of its lowest ghost axis only, so once, and
-// no thread writes a point that another reads (sources have no ghost
-// coordinate).
-__device__ __forceinline__ void wrap3_body(const Params& P, int which, long long g) {
-  const long long N0 = P.N[0], N1 = P.N[1], N2 = P.N[2];
-  const long long s0 = 9 * N1 * N2, s1 = N0 * 9 * N2, s2 = N0 * N1 * 9;
+// Thread g runs over three slabs, axis a's 9 layers (4 ghost layers below, 5
+// points above: the cell fields' 4 ghost layers and the padding point, or the
+// upper boundary face and the face field's 4 ghost layers) times all points
+// of the other two axes; a point belongs to the slab of the lowest axis whose
+// layers hold it.
+template <bool PERIODIC>
+__device__ __forceinline__ void ghost_body(const Params& P, const GhostFill& G, int which, unsigned g) {
+  // (32 bits: the slabs of a grid of fewer than 2^29 points, see lin32)
+  const unsigned N0 = P.N[0], N1 = P.N[1], N2 = P.N[2];
+  const unsigned s0 = 9 * N1 * N2, s1 = N0 * 9 * N2, s2 = N0 * N1 * 9;
   int a, x[3];
   if (g < s0) {
     a = 0;
     x[0] = (int)(g % 9);
-    const long long r = g / 9;
+    const unsigned r = g / 9;
     x[1] = (int)(r % N1);
     x[2] = (int)(r / N1);
   } else if (g < s0 + s1) {
     a = 1;
-    const long long r = g - s0;
+    const unsigned r = g - s0;
     x[0] = (int)(r % N0);
     x[1] = (int)((r / N0) % 9);
     x[2] = (int)(r / N0 / 9);
   } else if (g < s0 + s1 + s2) {
     a = 2;
-    const long long r = g - s0 - s1;
+    const unsigned r = g - s0 - s1;
     x[0] = (int)(r % N0);
     x[1] = (int)((r / N0) % N1);
     x[2] = (int)(r / N0 / N1);
@@ -984,104 +998,55 @@ __device__ __forceinline__ void wrap3_body(const Params& P, int which, long long
     return;
   }
   if (x[a] >= NGH) x[a] += P.n[a];  // the 5 points above the active range
+  for (int b = 0; b < a; b++)
+    if (x[b] < NGH || x[b] >= NGH + P.n[b]) return;
   const int bsel = which ? cur_buf(P) : 1 - cur_buf(P);
   double* __restrict__ W = P.Wbuf[bsel];
   double* __restrict__ B = P.Bbuf[bsel];
   const bool ps = P.ps_live != 0;  // p_S zero everywhere stays so: skipped
-  long long src[9], dst[9];
-  bool on[9];
-#pragma unroll
-  for (int f = 0; f < 9; f++) {
-    int y[3] = {x[0], x[1], x[2]};
-    int low = 3;  // lowest ghost axis of this field at this point
-#pragma unroll
-    for (int b = 2; b >= 0; b--) {
-      const int o = (f >= 6 && f - 6 == b) ? 1 : 0;  // the face field along b
-      if (y[b] < NGH) {
-        y[b] += P.n[b];
-        low = b;
-      } else if (y[b] >= NGH + P.n[b] + o && y[b] < 2 * NGH + P.n[b] + o) {
-        y[b] -= P.n[b];
-        low = b;
-      }
-    }
-    on[f] = low == a && (f != PS || ps);
-    src[f] = lin(P, y[0], y[1], y[2]);
-    dst[f] = lin(P, x[0], x[1], x[2]);
-  }
+  const int dst = lin32(P, x[0], x[1], x[2]);
+  // all loads before the stores
   double v[9];
+  bool on[9];
+  {
+    int y[3] = {x[0], x[1], x[2]}, neg, fixed;
+    const bool any = ghost_source<PERIODIC>(P, G, G.gas, -1, y, neg, fixed);
+    const int src = lin32(P, y[0], y[1], y[2]);
 #pragma unroll
-  for (int f = 0; f < 9; f++) {
-    const double* q = f < 6 ? W + (size_t)f * P.fs : B + (size_t)(f - 6) * P.fs;
-    if (on[f]) v[f] = q[src[f]];
-  }
-#pragma unroll
-  for (int f = 0; f < 9; f++) {
-    double* q = f < 6 ? W + (size_t)f * P.fs : B + (size_t)(f - 6) * P.fs;
-    if (on[f]) q[dst[f]] = v[f];
-  }
-}
-
-// One face of the ghost-fill library (src/boundary_conditions.c): the 6 gas
-// primitives with kind `kind` (gas_bc_*) and the 3 face fields with kind
-// `gkind` (gem_bc_*); 0 skips that group.  t = (i, j, k) with the
-// component along `axis` replaced by the ghost layer 0..NGH-1.
-__device__ __forceinline__ void bcface_body(const Params& P, int axis, int side, int kind,
-                                            int gkind, int which, Pos t) {
-  int ijk[3] = {t.x, t.y, t.z};
-  const int l = ijk[axis];
-  for (int a = 0; a < 3; a++)
-    if (ijk[a] >= (a == axis ? NGH : P.N[a])) return;
-  const int bsel = which ? cur_buf(P) : 1 - cur_buf(P);
-  double* __restrict__ W = P.Wbuf[bsel];
-  double* __restrict__ B = P.Bbuf[bsel];
-  const int N = P.N[axis];
-  for (int f = 0; f < 9; f++) {
-    if (f == PS && !P.ps_live) continue;  // zero everywhere, and stays so
-    const bool gas = f < 6;
-    const int kd = gas ? kind : gkind;
-    if (kd == 0 || kd == 'n' || kd == 'p') continue;
-    if (!gas && kd == 'r') continue;  // gem_bc_reflective_* are empty
-    const int onface = (!gas && f - 6 == axis) ? 1 : 0;
-    double* a = gas ? W + (size_t)f * P.fs : B + (size_t)(f - 6) * P.fs;
-    const int dst = side == 0 ? l : N - 1 - NGH + l + onface;
-    double v;
-    if (kd == 'f') {
-      if (gas) {
-        if (f == PS) continue;
-        if (f == RHO) v = (axis == 1 && side == 0) ? 2.0 : 1.0;
-        else if (f == PR) v = (axis == 1 && side == 1) ? 2.5 : 1.0;
-        else v = 0.0;
-      } else {
-        v = 0.0;
+    for (int f = 0; f < PS; f++) {
+      on[f] = any;
+      if (!any) continue;
+      if (fixed < 0) {
+        v[f] = W[(size_t)f * P.fs + src];
+      } else {  // gas_bc_fixed_*
+        v[f] = f == RHO ? (fixed == 2 ? 2.0 : 1.0) : (f == PR ? (fixed == 3 ? 2.5 : 1.0) : 0.0);
       }
-    } else {
-      int src;
-      if (kd == 'e') src = side == 0 ? NGH : N - 1 - NGH - 1 + onface;
-      else src = side == 0 ? 2 * NGH - 1 - l + onface : N - 1 - NGH - 1 - l;
-      ijk[axis] = src;
-      const int k0 = ijk[2];
-      // pole ('o', j faces): mirrored across the axis half a turn away in
-      // phi, the theta and phi components negated
-      // (src/spherical/spherical_boundary.c:23-138)
-      if (kd == 'o') ijk[2] = NGH + (k0 - NGH + P.n[2] / 2) % P.n[2];
-      v = a[lin(P, ijk[0], ijk[1], ijk[2])];
-      ijk[2] = k0;
-      if (kd == 'r' && gas && f == V1 + axis) v = -v;
-      if (kd == 'o' && (gas ? (f == V2 || f == V3) : f != 6)) v = -v;
+      // a reflective fill turns the velocity along its axis, the pole fill
+      // theta and phi components
+      const bool flip = f >= V1 && f <= V3 && ((neg >> (f - V1) & 1) != (f != V1 && (neg & 8)));
+      if (flip) v[f] = -v[f];
     }
-    ijk[axis] = dst;
-    a[lin(P, ijk[0], ijk[1], ijk[2])] = v;
   }
+  on[PS] = false;
+  if (ps) {
+    int y[3] = {x[0], x[1], x[2]}, neg, fixed;
+    on[PS] = ghost_source<PERIODIC>(P, G, G.gas, -1, y, neg, fixed, true);
+    if (on[PS]) v[PS] = W[(size_t)PS * P.fs + lin32(P, y[0], y[1], y[2])];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    int y[3] = {x[0], x[1], x[2]}, neg, fixed;
+    on[6 + c] = ghost_source<PERIODIC>(P, G, G.gem, c, y, neg, fixed);
+    if (!on[6 + c]) continue;
+    v[6 + c] = fixed < 0 ? B[(size_t)c * P.fs + lin32(P, y[0], y[1], y[2])] : 0.0;
+    if (c != 0 && (neg & 8)) v[6 + c] = -v[6 + c];
+  }
+#pragma unroll
+  for (int f = 0; f < 9; f++)
+    if (on[f]) (f < 6 ? W + (size_t)f * P.fs : B + (size_t)(f - 6) * P.fs)[dst] = v[f];
 }
 
 // ------------------------------------------------- single-instance kernels
-
-// 1: a fully periodic grid fills its ghosts in one launch (k_wrap3) instead
-// of one per axis
-#ifndef GOP_WRAP3
-#define GOP_WRAP3 1
-#endif
 
 // Resident 256-thread blocks per SM each kernel is compiled for (caps its
 // registers at 65536 / (256 * n)), per stage and arithmetic type; the
@@ -1128,17 +1093,20 @@ __device__ __forceinline__ void bcface_body(const Params& P, int axis, int side,
 #define GOP_MINB(STAGE, R) (sizeof(R) == 8 ? GOP_MINB_##STAGE##_F64 : GOP_MINB_##STAGE##_F32)
 #define GOP_UPD_MINB(COORD, R) ((COORD) == 0 ? GOP_MINB(UPDATE, R) : GOP_MINB(UPDATE_SPH, R))
 
-__global__ void k_begin(Params P) {
-  pdl_enter();
-  begin_body(P);
-}
-__global__ void k_end(Params P) {
-  pdl_enter();
-  end_body(P);
-}
 __global__ void k_arm(Params P, double tstop, double budget) {
   pdl_enter();
   arm_body(P, tstop, budget);
+  begin_body(P);
+}
+// between two steps of a call: the buffer just written becomes the current
+// state, the next step is opened
+__device__ __forceinline__ void turn_body(const Params& P) {
+  end_body(P);
+  begin_body(P);
+}
+__global__ void k_turn(Params P) {
+  pdl_enter();
+  turn_body(P);
 }
 
 // S_PSNZ <- 1 if p_S of either state buffer is nonzero at a point the AB2
@@ -1247,20 +1215,25 @@ __global__ void __launch_bounds__(256, GOP_UPD_MINB(COORD, R)) k_update(Params P
   update_body<COORD, R, BG, PSL>(P, w, grid_pos(), dtc, db);
   block_commit(dtc, db, P.scal + S_NEXT_DT, P.scal + S_DIVB);
 }
-__global__ void k_wrap(Params P, int axis, int which) {
+// Ghost fill of the state just written (which 0) or of the current state.
+// After a step's fill the block that finishes last turns to the next step: a
+// launch of one thread for the end of the step and one for the begin of the
+// next took 2.4 us each.
+template <bool PERIODIC>
+__global__ void __launch_bounds__(256) k_ghost(Params P, GhostFill G, int which) {
   pdl_enter();
-  if (stopped(P)) return;
-  wrap_body(P, axis, which, grid_pos());
-}
-__global__ void k_wrap3(Params P, int which) {
-  pdl_enter();
-  if (stopped(P)) return;
-  wrap3_body(P, which, (long long)blockIdx.x * blockDim.x + threadIdx.x);
-}
-__global__ void k_bcface(Params P, int axis, int side, int kind, int gkind, int which) {
-  pdl_enter();
-  if (stopped(P)) return;
-  bcface_body(P, axis, side, kind, gkind, which, grid_pos());
+  if (!which && stopped(P)) return;
+  ghost_body<PERIODIC>(P, G, which, blockIdx.x * blockDim.x + threadIdx.x);
+  if (which) return;
+  // every thread of the block has read S_PAR and written its points
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  unsigned* done = reinterpret_cast<unsigned*>(P.scal + S_TILE) + 1;
+  __threadfence();
+  if (atomicAdd(done, 1u) == gridDim.x - 1) {
+    *done = 0;
+    turn_body(P);
+  }
 }
 
 // ------------------------------------------------------ layout transposes
@@ -1380,13 +1353,6 @@ Tune::Tune() {
 dim3 launch_space(const Params& P, int slot) {
   if (slot == K_AB2) return dim3(P.N[0], P.N[1], P.N[2]);
   if (slot == K_UPDATE) return dim3(P.n[0], P.n[1], P.n[2]);
-  if (slot >= K_WRAP0 && slot <= K_BC5) {  // (i, j, k) with the ghost layers along the axis
-    const bool wrap = slot <= K_WRAP2;
-    const int a = wrap ? slot - K_WRAP0 : (slot - K_BC0) / 2;
-    int e[3] = {P.N[0], P.N[1], P.N[2]};
-    e[a] = wrap ? 2 * NGH : NGH;
-    return dim3(e[0], e[1], e[2]);
-  }
   const int stage = (slot - K_C2C0) / 3, D = (slot - K_C2C0) % 3;
   const int p = (D + 1) % 3, q = (D + 2) % 3;
   int cnt[3];
@@ -1407,8 +1373,6 @@ dim3 launch_space(const Params& P, int slot) {
   return dim3(cnt[0], cnt[1], cnt[2]);
 }
 
-void launch_begin(const Params& P, cudaStream_t st) { LAUNCH(k_begin, 1, 1, st, P); }
-void launch_end(const Params& P, cudaStream_t st) { LAUNCH(k_end, 1, 1, st, P); }
 void launch_arm(const Params& P, double tstop, double budget, cudaStream_t st) {
   LAUNCH(k_arm, 1, 1, st, P, tstop, budget);
 }
@@ -1550,37 +1514,28 @@ template void launch_step_body<double>(const Params&, int, const Work<double>&, 
 template void launch_step_body<float>(const Params&, int, const Work<float>&, cudaStream_t,
                                       const Tune&, const SweepSet*, const Hook&);
 
-dim3 ghost_block(int slot) {
-  if (slot == K_WRAP0) return dim3(8, 16, 2);               // 8 layers along i
-  if (slot == K_BC0 || slot == K_BC1) return dim3(4, 32, 2);  // 4 layers along i
-  return dim3(32, 8, 1);
-}
-
 void launch_ghosts(const Params& P, const char bc[6], const char gem_bc[6], int which,
                    cudaStream_t st) {
-  bool periodic[3];
-  for (int a = 0; a < 3; a++) periodic[a] = bc[2 * a] == 'p' && bc[2 * a + 1] == 'p';
-  if (periodic[0] && periodic[1] && periodic[2] && GOP_WRAP3) {
-    const long long N0 = P.N[0], N1 = P.N[1], N2 = P.N[2];
-    const long long pts = 9 * (N1 * N2 + N0 * N2 + N0 * N1);
-    LAUNCH(k_wrap3, dim3((unsigned)((pts + 255) / 256)), dim3(256), st, P, which);
-    return;
+  GhostFill G;
+  bool any = false, all = true;
+  for (int f = 0; f < 6; f++) {
+    G.gas[f] = bc[f];
+    G.gem[f] = gem_bc[f];
+    any = any || bc[f] != 'n' || (gem_bc[f] != 'n' && gem_bc[f] != 'r');
   }
   for (int a = 0; a < 3; a++) {
-    if (!periodic[a]) continue;
-    const dim3 sp = launch_space(P, K_WRAP0 + a), blk = ghost_block(K_WRAP0 + a);
-    LAUNCH(k_wrap, grid3(sp.x, sp.y, sp.z, blk), blk, st, P, a, which);
+    G.per[a] = bc[2 * a] == 'p' && bc[2 * a + 1] == 'p';
+    all = all && G.per[a];
   }
-  for (int face = 0; face < 6; face++) {
-    const int a = face / 2, side = face % 2;
-    const char kind = bc[face], gkind = gem_bc[face];
-    if (periodic[a]) continue;
-    const bool gas_work = kind != 'n';
-    const bool gem_work = gkind != 'n' && gkind != 'r';
-    if (!gas_work && !gem_work) continue;
-    const dim3 sp = launch_space(P, K_BC0 + face), blk = ghost_block(K_BC0 + face);
-    LAUNCH(k_bcface, grid3(sp.x, sp.y, sp.z, blk), blk, st, P, a, side, (int)kind, (int)gkind, which);
+  if (!any) {
+    if (!which) LAUNCH(k_turn, 1, 1, st, P);
+    return;
   }
+  const long long N0 = P.N[0], N1 = P.N[1], N2 = P.N[2];
+  const long long pts = 9 * (N1 * N2 + N0 * N2 + N0 * N1);
+  const dim3 g((unsigned)((pts + 255) / 256));
+  if (all) LAUNCH(k_ghost<true>, g, dim3(256), st, P, G, which);
+  else LAUNCH(k_ghost<false>, g, dim3(256), st, P, G, which);
 }
 
 static dim3 transpose_grid(const Params& P) {

@@ -35,12 +35,9 @@ void count_launches(int64_t n);  // kernels run by graph replays
 enum Group : int { G_BEGIN = 0, G_AB2, G_C2C, G_EMF, G_FLUX, G_UPDATE, G_GHOST, G_END, NGROUP };
 
 // launch shapes of the tunable kernels: AB2, C2C x3, EMF x3, FLUX x3,
-// UPDATE; then the ghost launches (periodic wrap per axis, boundary fill
-// per face), whose shapes are fixed (ghost_block)
+// UPDATE
 enum TuneSlot : int { K_AB2 = 0, K_C2C0, K_C2C1, K_C2C2, K_EMF0, K_EMF1, K_EMF2,
-                      K_FLUX0, K_FLUX1, K_FLUX2, K_UPDATE, NTUNE,
-                      K_WRAP0 = NTUNE, K_WRAP1, K_WRAP2, K_BC0, K_BC1, K_BC2, K_BC3, K_BC4,
-                      K_BC5, NSLOT };
+                      K_FLUX0, K_FLUX1, K_FLUX2, K_UPDATE, NTUNE };
 struct Tune {
   dim3 blk[NTUNE];
   // the stage's fluxes / edge EMFs from the tile-staged sweep kernels
@@ -71,8 +68,6 @@ bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, con
 
 // points covered by the launch of one slot (x, y, z extents)
 dim3 launch_space(const Params& P, int slot);
-// thread-block shape of a ghost-fill slot (K_WRAP*, K_BC*)
-dim3 ghost_block(int slot);
 
 // launches one tunable kernel; pdl false: without programmatic dependent
 // launch
@@ -88,9 +83,8 @@ struct Hook {
     if (mark) mark(ctx, g, s);
   }
 };
-void launch_begin(const Params& P, cudaStream_t st);
-void launch_end(const Params& P, cudaStream_t st);
-// arm a gop_step call: stop after time tstop or after `budget` steps
+// arm a gop_step call: stop after time tstop or after `budget` steps; opens
+// the first step
 void launch_arm(const Params& P, double tstop, double budget, cudaStream_t st);
 // CFL dt (in the form and arithmetic of the step's own estimate) and
 // max|div B| of the current state
@@ -100,7 +94,14 @@ void launch_ps_check(const Params& P, cudaStream_t st);
 template <typename R>
 void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t st,
                       const Tune& tune, const SweepSet* sw, const Hook& hook = Hook());
-// which = 0: the buffer being written this step; 1: the current state
+// what fills the ghost layers of each face (gas_bc_*, gem_bc_*: GOP_BC_*) and
+// which axes are periodic
+struct GhostFill {
+  char gas[6], gem[6];
+  bool per[3];
+};
+// which = 0: the buffer being written this step, and the turn to the next
+// step; 1: the current state
 void launch_ghosts(const Params& P, const char bc[6], const char gem_bc[6], int which,
                    cudaStream_t st);
 // one field between the reference layout and the device's

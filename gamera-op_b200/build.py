@@ -26,7 +26,8 @@ SOURCES = [
 ]
 HEADERS = [ROOT / "include" / "gamera_op.h", PKG / "csrc" / "gop_device.cuh",
            PKG / "csrc" / "gop_kernels.h", PKG / "csrc" / "gop_internal.h",
-           PKG / "csrc" / "gop_stage.cuh", PKG / "csrc" / "gop_tma.cuh",
+           PKG / "csrc" / "gop_stage.cuh", PKG / "csrc" / "gop_update.cuh",
+           PKG / "csrc" / "gop_tma.cuh",
            PKG / "csrc" / "gop_fields.h", PKG / "csrc" / "gop_bgfield.h"]
 
 NVCC_FLAGS = [

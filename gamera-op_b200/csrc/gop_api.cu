@@ -130,6 +130,7 @@ void build_tables(const gop_desc& d, Tables& T) {
       dxv[a][c] = x[c + 1] - x[c];
       xcv[a][c] = 0.5 * (x[c] + x[c + 1]);
       T.at(a, T_DX, c) = dxv[a][c];
+      T.at(a, T_IDX, c) = 1.0 / dxv[a][c];
       double xc = xcv[a][c], dx = dxv[a][c];
       if (sph && a == 0)
         xctr[a][c] = xc + 2.0 * xc * dx * dx / (12.0 * xc * xc + dx * dx);

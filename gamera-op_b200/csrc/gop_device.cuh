@@ -29,6 +29,7 @@ constexpr double PDMB = 1.0;
 enum Tab : int {
   T_X = 0,     // face coordinate x[f]
   T_DX,        // x[f+1] - x[f]
+  T_IDX,       // 1 / T_DX
   T_MA,        // (x[c+1] - xctr[c]) / dx[c]: weight of the lower face in mags
   T_MB,        // (xctr[c] - x[c]) / dx[c]: weight of the upper face
   T_WL0,       // 7 left PDM weights at face f (applied to cells f-4..f+2)
@@ -122,10 +123,22 @@ __device__ __forceinline__ long long lin(const Params& P, int i, int j, int k) {
   return (long long)k * P.sk + (long long)j * P.sj + i;
 }
 
-// the same in 32 bits: a field has fewer than 2^31 points (an instance holds
-// at least 348 bytes per point, so one of 2^31 would not fit any GPU)
+// the same in 32 bits: a field has fewer than 2^29 points (an instance holds
+// at least 432 bytes per point, so one of 2^29 would not fit a GPU of 232 GB)
 __device__ __forceinline__ int lin32(const Params& P, int i, int j, int k) {
   return (k * P.N[1] + j) * P.pitch + i;
+}
+
+// base[off / sizeof(T)] of a field for a byte offset (below 2^32, see lin32):
+// one address register for all the fields a thread reads at a point, where an
+// index of 64 bits takes two additions per field
+template <typename T>
+__device__ __forceinline__ T at_byte(const T* base, unsigned off) {
+  return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + off));
+}
+template <typename T>
+__device__ __forceinline__ T& at_byte(T* base, unsigned off) {
+  return *reinterpret_cast<T*>(reinterpret_cast<char*>(base) + off);
 }
 
 __device__ __forceinline__ long long stride(const Params& P, int axis) {

@@ -29,6 +29,7 @@
 #include "gop_device.cuh"
 #include "gop_kernels.h"
 #include "gop_stage.cuh"
+#include "gop_update.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -37,87 +38,25 @@
 
 namespace gop {
 
-// Options of the mixed path's Cartesian update (0: FP32 as documented): run
-// the flux divergence, the Alfven/Boris correction or the CFL estimate in
-// FP64 instead
-#ifndef GOP_MX_DIV64
-#define GOP_MX_DIV64 0
-#endif
-#ifndef GOP_MX_ALF64
-#define GOP_MX_ALF64 0
-#endif
-#ifndef GOP_MX_CFL64
-#define GOP_MX_CFL64 0
-#endif
-
 // ------------------------------------------------------------------ utils
 
 
-__device__ __forceinline__ void atomic_min_pos(double* slot, double v) {
-  // positive doubles order like their bit patterns
-  atomicMin(reinterpret_cast<unsigned long long*>(slot), (unsigned long long)__double_as_longlong(v));
-}
-__device__ __forceinline__ void atomic_max_pos(double* slot, double v) {
-  atomicMax(reinterpret_cast<unsigned long long*>(slot), (unsigned long long)__double_as_longlong(v));
-}
-
-__device__ __forceinline__ double warp_min(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ double warp_max(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-// block-wide min and max of (a, b); one thread commits them with one atomic each
-__device__ __forceinline__ void block_commit(double a, double b, double* smin, double* smax) {
-  __shared__ double sa[32], sb[32];
-  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-  const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) / 32;
-  const int w = tid / 32, lane = tid & 31;
-  a = warp_min(a);
-  b = warp_max(b);
-  if (lane == 0) {
-    sa[w] = a;
-    sb[w] = b;
-  }
-  __syncthreads();
-  if (w == 0) {
-    a = lane < nw ? sa[lane] : DBL_MAX;
-    b = lane < nw ? sb[lane] : 0.0;
-    a = warp_min(a);
-    b = warp_max(b);
-    if (lane == 0) {
-      if (a < DBL_MAX) atomic_min_pos(smin, a);
-      if (b > 0.0) atomic_max_pos(smax, b);
-    }
-  }
-}
-
-// CFL time step of one cell (src/solver_func.c:255-298), in T arithmetic
-// (FP32 for the mixed path's estimate)
+// CFL rate (signal speed over the cell's lengths) of one cell of a
+// curvilinear grid, in T arithmetic (FP32 for the mixed path's estimate)
 template <int COORD, typename T = double>
 __device__ __forceinline__ double cfl_cell(const Params& P, int i, int j, int k, double rho,
                                            double u, double v, double w, double p, double b1,
                                            double b2, double b3) {
-  const T r = (T)rho, x1 = (T)b1, x2 = (T)b2, x3 = (T)b3, ut = (T)u, vt = (T)v, wt = (T)w;
-  T bsq = x1 * x1 + x2 * x2 + x3 * x3;
-  T va = sqrt(bsq / r);
-  T vae = va * (T)P.ca / sqrt(va * va + (T)P.ca2);
-  T vf = sqrt(ut * ut + vt * vt + wt * wt);
-  T vs = sqrt((T)P.gamma * (T)p / r);
-  T vc = vf + sqrt(vs * vs + vae * vae);
+  const T x1 = (T)b1, x2 = (T)b2, x3 = (T)b3;
+  const T vc = signal_speed(P, (T)rho, (T)u, (T)v, (T)w, (T)p, x1 * x1 + x2 * x2 + x3 * x3);
   T dk = (T)Geo<COORD>::dl(P, 2, i, j, k);
   // the phi length of the pole rings is nk / nchunk times longer (dxk_ring,
   // spherical_RingAverage.c:110-138; get_dt_ring, spherical_general.c:700-743)
   if (COORD == 2 && P.ring) dk = (T)P.ringtab[2 * P.n[2] + j] * dk;
-  T t = vc / (T)Geo<COORD>::dl(P, 0, i, j, k) + vc / (T)Geo<COORD>::dl(P, 1, i, j, k) + vc / dk;
-  return (double)((T)P.cfl / t);
+  const T di = (T)Geo<COORD>::dl(P, 0, i, j, k), dj = (T)Geo<COORD>::dl(P, 1, i, j, k);
+  if constexpr (sizeof(T) == 8) return vc * ((dj * dk + di * dk + di * dj) / (di * dj * dk));
+  return (double)(vc / di + vc / dj + vc / dk);
 }
-
 // rows of cells whose state or face field the pole ring average changes
 // (the ring rows and the rows of the faces its EMF-like field touches)
 __device__ __forceinline__ bool ring_band_row(const Params& P, int j) {
@@ -149,10 +88,6 @@ __device__ __forceinline__ void line8(const T* __restrict__ a, long long s, R v[
 
 
 
-// thread coordinates in a launch space
-struct Pos {
-  int x, y, z;
-};
 __device__ __forceinline__ Pos grid_pos() {
   return {(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(blockIdx.y * blockDim.y + threadIdx.y),
           (int)(blockIdx.z * blockDim.z + threadIdx.z)};
@@ -421,193 +356,6 @@ __device__ __forceinline__ double ct_face(const Params& P, const double* __restr
   return B[x + A * fs] - dt * (cq - cp) / Geo<COORD>::face(P, A, i, j, k);
 }
 
-// One active cell of a Cartesian grid (src/solver_solve.c:263-484 with the
-// Cartesian geometry of src/cartesian/cartesian_general.c): every face of
-// the cell has the area of its axis, every edge along axis a the length
-// dx_a, and the geometric sources vanish, so the whole cell needs dx_i,
-// dx_j, dx_k and one division.  Face fields, constrained transport, the
-// conservative update and the pressure recovery are FP64; with R = float
-// the flux divergence, the Alfven/Boris correction and the CFL estimate are
-// FP32.  Returns the cell's CFL dt and |div B| of the new state.
-template <typename R, bool BG, bool PSL>
-__device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, Pos t,
-                                            double& dtc, double& dbmax) {
-  // arithmetic of the stages the mixed path runs in FP32 (FP64 when their
-  // option is on, and always on the plain path)
-  using RD = typename std::conditional<sizeof(R) == 8 || GOP_MX_DIV64, double, R>::type;
-  using RA = typename std::conditional<sizeof(R) == 8 || GOP_MX_ALF64, double, R>::type;
-  using RC = typename std::conditional<sizeof(R) == 8 || GOP_MX_CFL64, double, R>::type;
-  const int i = NGH + t.x, j = NGH + t.y, k = NGH + t.z;
-  if (i >= NGH + P.n[0] || j >= NGH + P.n[1] || k >= NGH + P.n[2]) return;
-  const size_t fs = P.fs;
-  const double dt = P.scal[S_DT];
-  const int cb = cur_buf(P);
-  const double* __restrict__ W = P.Wbuf[cb];
-  const double* __restrict__ B = P.Bbuf[cb];
-  double* __restrict__ Wn = P.Wbuf[1 - cb];
-  double* __restrict__ Bn = P.Bbuf[1 - cb];
-  const long long x = lin(P, i, j, k), sj = P.sj, sk = P.sk;
-  const double dx[3] = {tb(P, 0, T_DX, i), tb(P, 1, T_DX, j), tb(P, 2, T_DX, k)};
-  const double A[3] = {dx[1] * dx[2], dx[0] * dx[2], dx[0] * dx[1]};
-  const double ivol = 1.0 / (dx[0] * dx[1] * dx[2]);
-  const double iA[3] = {dx[0] * ivol, dx[1] * ivol, dx[2] * ivol};  // 1/A_a
-  const double il[3] = {A[0] * ivol, A[1] * ivol, A[2] * ivol};     // 1/dx_a
-
-  // constrained transport: face A gets -dt (curl E)_A, from FP64 products
-  // of the edge EMFs and edge lengths (src/solver_solve.c:263-306)
-  const R* __restrict__ E = wk.E + x;
-  auto ed = [&](int a, long long off) { return (double)E[a * fs + off] * dx[a]; };
-  const double e0 = ed(0, 0), e1 = ed(1, 0), e2 = ed(2, 0);
-  const double e0j = ed(0, sj), e0k = ed(0, sk), e1i = ed(1, 1), e1k = ed(1, sk);
-  const double e2i = ed(2, 1), e2j = ed(2, sj);
-  double bl[3], bu[3], mo[3];
-  bl[0] = B[x] - dt * ((e2j - e2) - (e1k - e1)) * iA[0];
-  bl[1] = B[x + fs] - dt * ((e0k - e0) - (e2i - e2)) * iA[1];
-  bl[2] = B[x + 2 * fs] - dt * ((e1i - e1) - (e0j - e0)) * iA[2];
-  {
-    const double e1ik = ed(1, 1 + sk), e2ij = ed(2, 1 + sj), e0jk = ed(0, sj + sk);
-    bu[0] = B[x + 1] - dt * ((e2ij - e2i) - (e1ik - e1i)) * iA[0];
-    bu[1] = B[x + sj + fs] - dt * ((e0jk - e0j) - (e2ij - e2j)) * iA[1];
-    bu[2] = B[x + sk + 2 * fs] - dt * ((e1ik - e1k) - (e0jk - e0k)) * iA[2];
-  }
-  // mags^n for the time-centred field
-  mo[0] = B[x] * tb(P, 0, T_MA, i) + B[x + 1] * tb(P, 0, T_MB, i);
-  mo[1] = B[x + fs] * tb(P, 1, T_MA, j) + B[x + sj + fs] * tb(P, 1, T_MB, j);
-  mo[2] = B[x + 2 * fs] * tb(P, 2, T_MA, k) + B[x + sk + 2 * fs] * tb(P, 2, T_MB, k);
-  // (stored here: keeping the six face values until after the flux loads
-  // measured 8 % slower on B200, FP64 256^3, from the registers it holds)
-  Bn[x] = bl[0];
-  Bn[x + fs] = bl[1];
-  Bn[x + 2 * fs] = bl[2];
-  if (i == NGH + P.n[0] - 1) Bn[x + 1] = bu[0];
-  if (j == NGH + P.n[1] - 1) Bn[x + sj + fs] = bu[1];
-  if (k == NGH + P.n[2] - 1) Bn[x + sk + 2 * fs] = bu[2];
-  if constexpr (BG) {  // div of B + B0 (face-normal B0, src/solver_func.c:324-343)
-    const double* f0 = P.bg + (size_t)BG_FACE * fs + x;
-    const double* f1 = P.bg + (size_t)(BG_FACE + 4) * fs + x;
-    const double* f2 = P.bg + (size_t)(BG_FACE + 8) * fs + x;
-    const double dvb = ((bu[0] + f0[1]) * A[0] - (bl[0] + f0[0]) * A[0]) * ivol +
-                       ((bu[1] + f1[sj]) * A[1] - (bl[1] + f1[0]) * A[1]) * ivol +
-                       ((bu[2] + f2[sk]) * A[2] - (bl[2] + f2[0]) * A[2]) * ivol;
-    dbmax = fabs(dvb);
-  } else {
-    const double dvb = (bu[0] * A[0] - bl[0] * A[0]) * ivol + (bu[1] * A[1] - bl[1] * A[1]) * ivol +
-                       (bu[2] * A[2] - bl[2] * A[2]) * ivol;
-    dbmax = fabs(dvb);
-  }
-  // cell-centred B0 (magtot = mags + B0)
-  double c0[3] = {0.0, 0.0, 0.0};
-  if constexpr (BG) {
-#pragma unroll
-    for (int a = 0; a < 3; a++) c0[a] = P.bg[(size_t)(BG_B0 + a) * fs + x];
-  }
-  double mn[3], mt[3];
-  mn[0] = bl[0] * tb(P, 0, T_MA, i) + bu[0] * tb(P, 0, T_MB, i);
-  mn[1] = bl[1] * tb(P, 1, T_MA, j) + bu[1] * tb(P, 1, T_MB, j);
-  mn[2] = bl[2] * tb(P, 2, T_MA, k) + bu[2] * tb(P, 2, T_MB, k);
-#pragma unroll
-  for (int a = 0; a < 3; a++) mt[a] = BG ? 0.5 * (mn[a] + mo[a]) + c0[a] : 0.5 * (mn[a] + mo[a]);
-
-  // flux divergence: 6 hydro and 3 stress components (FP32 arithmetic on
-  // the mixed path; the reference's F_u A - F_l A over the volume otherwise)
-  RD du[6], dm[3];
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    const long long s = d == 0 ? 1LL : (d == 1 ? sj : sk);
-    const R* __restrict__ Fd = wk.F + (size_t)(9 * d) * fs + x;
-#pragma unroll
-    for (int m = 0; m < 9; m++) {
-      if (m == PS && !PSL) continue;
-      RD v;
-      if constexpr (sizeof(RD) == 4) {
-        v = (Fd[s + m * fs] - Fd[m * fs]) * (R)il[d];
-      } else {
-        v = ((double)Fd[s + m * fs] * A[d] - (double)Fd[m * fs] * A[d]) * ivol;
-      }
-      if (m < 6) du[m] = d == 0 ? v : du[m] + v;
-      else dm[m - 6] = d == 0 ? v : dm[m - 6] + v;
-    }
-  }
-  if constexpr (BG) {  // + the Lorentz force of B0 (src/solver_solve.c:312-324)
-#pragma unroll
-    for (int a = 0; a < 3; a++) dm[a] += (RD)P.bg[(size_t)(BG_LOR + a) * fs + x];
-  }
-
-  // U^n from W^n, conservative update, cons->prim in FP64
-  // (src/solver_func.c:356-382, src/solver_solve.c:326-377)
-  const double gm1 = P.gm1;
-  const double r0 = W[x], u0 = W[x + fs], v0 = W[x + 2 * fs], w0 = W[x + 3 * fs],
-               p0 = W[x + 4 * fs];
-  const double U0[3] = {r0 * u0, r0 * v0, r0 * w0};
-  const double E0 = 0.5 * r0 * (u0 * u0 + v0 * v0 + w0 * w0) + p0 * P.inv_gm1;
-  const double Ur = r0 - dt * (double)du[0];
-  double Um[3];
-#pragma unroll
-  for (int a = 0; a < 3; a++) Um[a] = U0[a] - dt * (double)du[1 + a];
-  const double Ue = E0 - dt * (double)du[4];
-  double rho = Ur;
-  const double irho = 1.0 / Ur;
-  double vv[3] = {Um[0] * irho, Um[1] * irho, Um[2] * irho};
-  double p = (Ue - 0.5 * (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]) * rho) * gm1;
-  double pS = 0.0;
-  if constexpr (PSL) {  // entropy S = p_S / rho^(gamma-1), updated and back
-    const double ps0 = W[x + 5 * fs];
-    const double S0 = (ps0 == 0.0 && r0 > 0.0) ? ps0 : ps0 / pow(r0, gm1);
-    const double Us = S0 - dt * (double)du[5];
-    pS = (Us == 0.0 && Ur > 0.0) ? Us : Us * pow(Ur, gm1);
-  }
-  // positivity floors (src/solver_func.c:2117-2135)
-  if (rho < P.rho_floor) {
-    rho = P.rho_floor;
-    p = P.p_floor;
-  }
-  if (p < P.p_floor) p = P.p_floor;
-
-  // Alfven/Boris correction of the momentum (src/solver_solve.c:385-484)
-  {
-    const RA bsq = (RA)(mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
-    const RA alf = bsq / ((RA)rho * (RA)P.ca2);
-    const RA perp = RA(1) / (RA(1) + alf);
-    const RA rdt = (RA)dt;
-    const RA drho = -rdt * (RA)du[0];
-    const RA dva = alf * drho;
-    RA tv[3], wv[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      wv[a] = (RA)W[x + (1 + a) * fs];
-      tv[a] = alf * (-rdt * (RA)du[1 + a] - drho * wv[a]);
-    }
-    RA bdv = (RA)mt[0] * tv[0] + (RA)mt[1] * tv[1] + (RA)mt[2] * tv[2];
-    bdv = bdv / (bsq + RA(1e-10));
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const RA inc = perp * ((-rdt * (RA)du[1 + a]) + (-rdt * (RA)dm[a]) + dva * wv[a] + (RA)mt[a] * bdv);
-      vv[a] = (U0[a] + (double)inc) * irho;
-    }
-  }
-  Wn[x] = rho;
-  Wn[x + fs] = vv[0];
-  Wn[x + 2 * fs] = vv[1];
-  Wn[x + 3 * fs] = vv[2];
-  Wn[x + 4 * fs] = p;
-  if constexpr (PSL) Wn[x + 5 * fs] = pS;  // else it stays zero in both buffers
-
-  // CFL dt of the new state with magtot = mags^{n+1} (src/solver_func.c:255-298)
-  {
-    const RC r = (RC)rho, u = (RC)vv[0], v = (RC)vv[1], w = (RC)vv[2];
-    const double t0 = mn[0] + c0[0], t1 = mn[1] + c0[1], t2 = mn[2] + c0[2];
-    const RC bsq = BG ? (RC)(t0 * t0 + t1 * t1 + t2 * t2) : (RC)(mn[0] * mn[0] + mn[1] * mn[1] + mn[2] * mn[2]);
-    const RC va = sqrt(bsq / r);
-    const RC vae = va * (RC)P.ca / sqrt(va * va + (RC)P.ca2);
-    const RC vf = sqrt(u * u + v * v + w * w);
-    const RC vs = sqrt((RC)P.gamma * (RC)p / r);
-    const RC vc = vf + sqrt(vs * vs + vae * vae);
-    dtc = (double)((RC)P.cfl / (vc * (RC)il[0] + vc * (RC)il[1] + vc * (RC)il[2]));
-  }
-  if (!(dtc > 0.0) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
-    P.scal[S_FLAGS] = 1.0;
-}
-
 // Constrained transport of a curvilinear grid (src/solver_solve.c:263-306),
 // its own launch before the update: every active cell writes its three lower
 // faces, the last cell along an axis also the upper boundary face, so each
@@ -649,15 +397,15 @@ __device__ __forceinline__ void ct_body(const Params& P, const Work<R>& wk, Pos 
   }
 }
 
-// one active cell: returns its CFL dt and |div B| of the new state.  The
+// one active cell: returns its CFL rate and |div B| of the new state.  The
 // flux divergence, the geometric sources, the Alfven/Boris correction and
 // the CFL estimate are in R (FP32 on the mixed path); the face fields, the
 // conservative update and the pressure recovery are FP64.
 template <int COORD, typename R, bool BG, bool PSL>
 __device__ __forceinline__ void update_body(const Params& P, const Work<R>& wk, Pos t,
-                                            double& dtc, double& dbmax) {
+                                            double& rate, double& dbmax) {
   if constexpr (COORD == 0) {
-    update_cart<R, BG, PSL>(P, wk, t, dtc, dbmax);
+    update_cart<R, BG, PSL>(P, wk, t, FluxPoint<R>{P, wk}, rate, dbmax);
     return;
   }
   const int i = NGH + t.x, j = NGH + t.y, k = NGH + t.z;
@@ -817,8 +565,8 @@ __device__ __forceinline__ void update_body(const Params& P, const Work<R>& wk, 
   Wn[x + 3 * fs] = vv[2];
   Wn[x + 4 * fs] = p;
   if constexpr (PSL) Wn[x + 5 * fs] = pS;
-  // CFL dt of the new state (magtot = mags^{n+1}) and max|div B^{n+1}|
-  dtc = cfl_cell<COORD, R>(P, i, j, k, rho, vv[0], vv[1], vv[2], p, mn[0], mn[1], mn[2]);
+  // CFL rate of the new state (magtot = mags^{n+1}) and max|div B^{n+1}|
+  rate = cfl_cell<COORD, R>(P, i, j, k, rho, vv[0], vv[1], vv[2], p, mn[0], mn[1], mn[2]);
   double b0l[3] = {0.0, 0.0, 0.0}, b0u[3] = {0.0, 0.0, 0.0};
   if constexpr (BG) {  // div of B + B0 (face-normal B0, src/solver_func.c:324-343)
 #pragma unroll
@@ -832,19 +580,18 @@ __device__ __forceinline__ void update_body(const Params& P, const Work<R>& wk, 
                      ((bu[1] + b0u[1]) * fu[1] - (bl[1] + b0l[1]) * fl[1]) * ivol +
                      ((bu[2] + b0u[2]) * fu[2] - (bl[2] + b0l[2]) * fl[2]) * ivol;
   dbmax = fabs(dvb);
-  if (!(dtc > 0.0) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
+  if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
     P.scal[S_FLAGS] = 1.0;
   if (COORD == 2 && P.ring && ring_band_row(P, j)) {
     // the ring average still changes this row: k_ring_dt takes its CFL dt
     // and div B afterwards
-    dtc = DBL_MAX;
+    rate = 0.0;
     dbmax = 0.0;
   }
 }
 
 // CFL dt and |div B| of one cell of the current state (prepare).  The dt
-// takes the form and arithmetic R of the step's own estimate (the
-// Cartesian update's 1/dx from the face area over the volume; the FP32
+// takes the form and arithmetic R of the step's own estimate (the FP32
 // estimate on the mixed path; FP64 in the rows of the pole ring average),
 // so a restarted run takes exactly the step the uninterrupted one would.
 template <int COORD, bool BG, typename R>
@@ -863,25 +610,15 @@ __device__ __forceinline__ void dt_body(const Params& P, Pos t, double& dtc, dou
   }
   if constexpr (COORD == 0) {  // as update_cart
     using RC = typename std::conditional<sizeof(R) == 8 || GOP_MX_CFL64, double, R>::type;
-    const double dx[3] = {tb(P, 0, T_DX, i), tb(P, 1, T_DX, j), tb(P, 2, T_DX, k)};
-    const double A[3] = {dx[1] * dx[2], dx[0] * dx[2], dx[0] * dx[1]};
-    const double ivol = 1.0 / (dx[0] * dx[1] * dx[2]);
-    const double il[3] = {A[0] * ivol, A[1] * ivol, A[2] * ivol};
-    const RC r = (RC)W[c], u = (RC)W[c + P.fs], v = (RC)W[c + 2 * P.fs], w = (RC)W[c + 3 * P.fs];
-    const RC p = (RC)W[c + 4 * P.fs];
-    const RC bsq = (RC)(b1 * b1 + b2 * b2 + b3 * b3);
-    const RC va = sqrt(bsq / r);
-    const RC vae = va * (RC)P.ca / sqrt(va * va + (RC)P.ca2);
-    const RC vf = sqrt(u * u + v * v + w * w);
-    const RC vs = sqrt((RC)P.gamma * p / r);
-    const RC vc = vf + sqrt(vs * vs + vae * vae);
-    dtc = (double)((RC)P.cfl / (vc * (RC)il[0] + vc * (RC)il[1] + vc * (RC)il[2]));
+    const double il[3] = {tb(P, 0, T_IDX, i), tb(P, 1, T_IDX, j), tb(P, 2, T_IDX, k)};
+    dtc = step_of<RC>(P, cfl_cart<RC>(P, il, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
+                                      W[c + 4 * P.fs], b1 * b1 + b2 * b2 + b3 * b3));
   } else if (P.ring && ring_band_row(P, j)) {  // as k_ring_dt
-    dtc = cfl_cell<COORD>(P, i, j, k, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
-                          W[c + 4 * P.fs], b1, b2, b3);
+    dtc = step_of<double>(P, cfl_cell<COORD>(P, i, j, k, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
+                                             W[c + 4 * P.fs], b1, b2, b3));
   } else {  // as the curvilinear update
-    dtc = cfl_cell<COORD, R>(P, i, j, k, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
-                             W[c + 4 * P.fs], b1, b2, b3);
+    dtc = step_of<R>(P, cfl_cell<COORD, R>(P, i, j, k, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
+                                           W[c + 4 * P.fs], b1, b2, b3));
   }
   const double vol = Geo<COORD>::vol(P, i, j, k);
   double d = 0.0;
@@ -1127,7 +864,12 @@ __global__ void k_dt(Params P) {
   pdl_enter();
   double dtc = DBL_MAX, db = 0.0;
   dt_body<COORD, BG, R>(P, grid_pos(), dtc, db);
-  block_commit(dtc, db, P.scal + S_NEXT_DT, P.scal + S_DIVB);
+  dtc = warp_min(dtc);
+  db = warp_max(db);
+  if (((threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31) == 0) {
+    if (dtc < DBL_MAX) atomic_min_pos(P.scal + S_NEXT_DT, dtc);
+    if (db > 0.0) atomic_max_pos(P.scal + S_DIVB, db);
+  }
 }
 
 // CFL dt and |div B| of the ring band rows of the new state, after the pole
@@ -1136,7 +878,7 @@ __global__ void k_dt(Params P) {
 // thread (i, band row, k)
 __global__ void k_ring_dt(Params P) {
   pdl_enter();
-  double dtc = DBL_MAX, db = 0.0;
+  double rate = 0.0, db = 0.0;
   const int i = NGH + blockIdx.x * blockDim.x + threadIdx.x;
   const int k = NGH + blockIdx.z * blockDim.z + threadIdx.z;
   const int slot = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1154,7 +896,7 @@ __global__ void k_ring_dt(Params P) {
       b[a] = mags_at(P, B, a, i, j, k);
       if (P.bg) b[a] += P.bg[(size_t)(BG_B0 + a) * P.fs + c];
     }
-    dtc = cfl_cell<2>(P, i, j, k, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
+    rate = cfl_cell<2>(P, i, j, k, W[c], W[c + P.fs], W[c + 2 * P.fs], W[c + 3 * P.fs],
                       W[c + 4 * P.fs], b[0], b[1], b[2]);
     const double vol = Geo<2>::vol(P, i, j, k);
     double d = 0.0;
@@ -1173,7 +915,7 @@ __global__ void k_ring_dt(Params P) {
     }
     db = fabs(d);
   }
-  block_commit(dtc, db, P.scal + S_NEXT_DT, P.scal + S_DIVB);
+  block_commit<double>(P, rate, db);
 }
 
 template <typename R, bool PSL>
@@ -1211,9 +953,9 @@ template <int COORD, typename R, bool BG, bool PSL>
 __global__ void __launch_bounds__(256, GOP_UPD_MINB(COORD, R)) k_update(Params P, Work<R> w) {
   pdl_enter();
   if (stopped(P)) return;
-  double dtc = DBL_MAX, db = 0.0;
-  update_body<COORD, R, BG, PSL>(P, w, grid_pos(), dtc, db);
-  block_commit(dtc, db, P.scal + S_NEXT_DT, P.scal + S_DIVB);
+  double rate = 0.0, db = 0.0;
+  update_body<COORD, R, BG, PSL>(P, w, grid_pos(), rate, db);
+  block_commit<typename std::conditional<COORD == 0 && GOP_MX_CFL64, double, R>::type>(P, rate, db);
 }
 // Ghost fill of the state just written (which 0) or of the current state.
 // After a step's fill the block that finishes last turns to the next step: a

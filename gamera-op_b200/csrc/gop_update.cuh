@@ -1,0 +1,308 @@
+// The cell update of a Cartesian grid and the reductions of the CFL step and
+// of |div B|, shared by the per-cell kernel (gop_kernels.cu) and the
+// tile-staged one (gop_sweep.cu).
+#pragma once
+
+#include <cfloat>
+#include <type_traits>
+
+#include "gop_stage.cuh"
+
+namespace gop {
+
+// Options of the mixed path's Cartesian update (0: FP32 as documented): run
+// the flux divergence, the Alfven/Boris correction or the CFL estimate in
+// FP64 instead
+#ifndef GOP_MX_DIV64
+#define GOP_MX_DIV64 0
+#endif
+#ifndef GOP_MX_ALF64
+#define GOP_MX_ALF64 0
+#endif
+#ifndef GOP_MX_CFL64
+#define GOP_MX_CFL64 0
+#endif
+
+// thread coordinates in a launch space
+struct Pos {
+  int x, y, z;
+};
+
+__device__ __forceinline__ void atomic_min_pos(double* slot, double v) {
+  // positive doubles order like their bit patterns
+  atomicMin(reinterpret_cast<unsigned long long*>(slot), (unsigned long long)__double_as_longlong(v));
+}
+__device__ __forceinline__ void atomic_max_pos(double* slot, double v) {
+  atomicMax(reinterpret_cast<unsigned long long*>(slot), (unsigned long long)__double_as_longlong(v));
+}
+
+__device__ __forceinline__ double warp_min(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// The block's largest CFL rate and |div B|; one thread commits the time step
+// of the rate (cfl / rate, in the arithmetic R of the rates: one division per
+// block instead of one per cell, the quotient being monotone) and |div B| with
+// one atomic each.  A rate of zero is no limit.
+template <typename R>
+__device__ __forceinline__ double step_of(const Params& P, double rate) {
+  return rate > 0.0 ? fmin((double)((R)P.cfl / (R)rate), DBL_MAX) : DBL_MAX;
+}
+template <typename R>
+__device__ __forceinline__ void block_commit(const Params& P, double a, double b) {
+  double* smin = P.scal + S_NEXT_DT;
+  double* smax = P.scal + S_DIVB;
+  __shared__ double sa[32], sb[32];
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) / 32;
+  const int w = tid / 32, lane = tid & 31;
+  a = warp_max(a);
+  b = warp_max(b);
+  if (lane == 0) {
+    sa[w] = a;
+    sb[w] = b;
+  }
+  __syncthreads();
+  if (w == 0) {
+    a = lane < nw ? sa[lane] : 0.0;
+    b = lane < nw ? sb[lane] : 0.0;
+    a = warp_max(a);
+    b = warp_max(b);
+    if (lane == 0) {
+      if (a > 0.0) atomic_min_pos(smin, step_of<R>(P, a));
+      if (b > 0.0) atomic_max_pos(smax, b);
+    }
+  }
+}
+
+// A rate that gives no positive time step
+__device__ __forceinline__ bool bad_rate(double rate) { return !(rate >= 0.0 && rate <= DBL_MAX); }
+
+// Fast signal speed |v| + sqrt(cs^2 + va^2) of a cell (src/solver_func.c:
+// 255-298): FP64 in the form of fast_speed, FP32 (the mixed path's estimate)
+// term by term
+__device__ __forceinline__ double signal_speed(const Params& P, double r, double u, double v, double w,
+                                               double p, double bsq) {
+  return sqrt(u * u + v * v + w * w) + fast_speed(P.gamma * p, r, bsq, P.ca2);
+}
+__device__ __forceinline__ float signal_speed(const Params& P, float r, float u, float v, float w, float p,
+                                              float bsq) {
+  const float va = sqrt(bsq / r);
+  const float vae = va * (float)P.ca / sqrt(va * va + (float)P.ca2);
+  const float vf = sqrt(u * u + v * v + w * w);
+  const float vs = sqrt((float)P.gamma * p / r);
+  return vf + sqrt(vs * vs + vae * vae);
+}
+
+// CFL rate (signal speed over the cell's lengths) of a cell of a Cartesian
+// grid, il the inverse lengths, in T arithmetic (FP32 for the mixed path's
+// estimate)
+template <typename T>
+__device__ __forceinline__ double cfl_cart(const Params& P, const double il[3], double rho, double u,
+                                           double v, double w, double p, double bsq) {
+  const T vc = signal_speed(P, (T)rho, (T)u, (T)v, (T)w, (T)p, (T)bsq);
+  return (double)(vc * (T)il[0] + vc * (T)il[1] + vc * (T)il[2]);
+}
+
+// the face fluxes from global memory
+template <typename R>
+struct FluxPoint {
+  const Params& P;
+  const Work<R>& wk;
+  __device__ __forceinline__ R operator()(const Pos& t, int d, int m, bool upper) const {
+    constexpr unsigned RS = sizeof(R);
+    const unsigned r = RS * (unsigned)lin32(P, NGH + t.x, NGH + t.y, NGH + t.z);
+    const unsigned s = d == 0 ? RS : RS * (unsigned)(d == 1 ? P.sj : P.sk);
+    return at_byte(wk.F + (size_t)(9 * d + m) * P.fs, upper ? r + s : r);
+  }
+};
+
+// One active cell of a Cartesian grid (src/solver_solve.c:263-484 with the
+// Cartesian geometry of src/cartesian/cartesian_general.c): every face of
+// the cell has the area of its axis, every edge along axis a the length
+// dx_a, and the geometric sources vanish, so the whole cell needs dx_i,
+// dx_j, dx_k and one division.  Face fields, constrained transport, the
+// conservative update and the pressure recovery are FP64; with R = float
+// the flux divergence, the Alfven/Boris correction and the CFL estimate are
+// FP32.  Returns the cell's CFL rate and |div B| of the new state.
+// flux(d, m, upper): flux m at the cell's lower or upper face along axis d.
+template <typename R, bool BG, bool PSL, class Flux>
+__device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, Pos t, const Flux& flux,
+                                            double& rate, double& dbmax) {
+  // arithmetic of the stages the mixed path runs in FP32 (FP64 when their
+  // option is on, and always on the plain path)
+  using RD = typename std::conditional<sizeof(R) == 8 || GOP_MX_DIV64, double, R>::type;
+  using RA = typename std::conditional<sizeof(R) == 8 || GOP_MX_ALF64, double, R>::type;
+  using RC = typename std::conditional<sizeof(R) == 8 || GOP_MX_CFL64, double, R>::type;
+  const int i = NGH + t.x, j = NGH + t.y, k = NGH + t.z;
+  if (i >= NGH + P.n[0] || j >= NGH + P.n[1] || k >= NGH + P.n[2]) return;
+  const size_t fs = P.fs;
+  const double dt = P.scal[S_DT];
+  const int cb = cur_buf(P);
+  const double* W = P.Wbuf[cb];
+  const double* B = P.Bbuf[cb];
+  double* Wn = P.Wbuf[1 - cb];
+  double* Bn = P.Bbuf[1 - cb];
+  // byte offsets of the cell and of its upper neighbours along j and k: o
+  // in the FP64 state, r in the stage arrays
+  const unsigned x = lin32(P, i, j, k), o = 8 * x, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
+  constexpr unsigned RS = sizeof(R);
+  const unsigned r = RS * x, rj = RS * (unsigned)P.sj, rk = RS * (unsigned)P.sk;
+  const double il[3] = {tb(P, 0, T_IDX, i), tb(P, 1, T_IDX, j), tb(P, 2, T_IDX, k)};
+
+  // flux divergence: 5 hydro (6 with the entropy channel) and 3 stress
+  // components, the difference of the two faces over the cell's length (every
+  // face of a Cartesian cell has the area of its axis).  First, so that its 48
+  // loads run ahead of everything else.
+  RD du[6], dm[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+#pragma unroll
+    for (int m = 0; m < 9; m++) {
+      if (m == PS && !PSL) continue;
+      const R fu = flux(t, d, m, true), fl = flux(t, d, m, false);
+      const RD v = ((RD)fu - (RD)fl) * (RD)il[d];
+      if (m < 6) du[m] = d == 0 ? v : du[m] + v;
+      else dm[m - 6] = d == 0 ? v : dm[m - 6] + v;
+    }
+  }
+  if constexpr (BG) {  // + the Lorentz force of B0 (src/solver_solve.c:312-324)
+#pragma unroll
+    for (int a = 0; a < 3; a++) dm[a] += (RD)P.bg[(size_t)(BG_LOR + a) * fs + x];
+  }
+
+  // constrained transport: face A gets -dt (curl E)_A from the differences of
+  // the edge EMFs, in FP64 (src/solver_solve.c:263-306; the edge lengths over
+  // the face area are inverse cell lengths)
+  const R *E0 = wk.E, *E1 = wk.E + fs, *E2 = wk.E + 2 * fs;
+  auto ld = [](const R* e, unsigned off) { return (double)at_byte(e, off); };
+  const double e0 = ld(E0, r), e0j = ld(E0, r + rj), e0k = ld(E0, r + rk), e0jk = ld(E0, r + rj + rk);
+  const double e1 = ld(E1, r), e1i = ld(E1, r + RS), e1k = ld(E1, r + rk), e1ik = ld(E1, r + RS + rk);
+  const double e2 = ld(E2, r), e2i = ld(E2, r + RS), e2j = ld(E2, r + rj), e2ij = ld(E2, r + RS + rj);
+  const double b0l = at_byte(B, o), b0u = at_byte(B, o + 8);
+  const double b1l = at_byte(B + fs, o), b1u = at_byte(B + fs, o + oj);
+  const double b2l = at_byte(B + 2 * fs, o), b2u = at_byte(B + 2 * fs, o + ok);
+  double bl[3], bu[3], mo[3];
+  bl[0] = b0l - dt * ((e2j - e2) * il[1] - (e1k - e1) * il[2]);
+  bl[1] = b1l - dt * ((e0k - e0) * il[2] - (e2i - e2) * il[0]);
+  bl[2] = b2l - dt * ((e1i - e1) * il[0] - (e0j - e0) * il[1]);
+  bu[0] = b0u - dt * ((e2ij - e2i) * il[1] - (e1ik - e1i) * il[2]);
+  bu[1] = b1u - dt * ((e0jk - e0j) * il[2] - (e2ij - e2j) * il[0]);
+  bu[2] = b2u - dt * ((e1ik - e1k) * il[0] - (e0jk - e0k) * il[1]);
+  // mags^n for the time-centred field
+  mo[0] = b0l * tb(P, 0, T_MA, i) + b0u * tb(P, 0, T_MB, i);
+  mo[1] = b1l * tb(P, 1, T_MA, j) + b1u * tb(P, 1, T_MB, j);
+  mo[2] = b2l * tb(P, 2, T_MA, k) + b2u * tb(P, 2, T_MB, k);
+  at_byte(Bn, o) = bl[0];
+  at_byte(Bn + fs, o) = bl[1];
+  at_byte(Bn + 2 * fs, o) = bl[2];
+  if (i == NGH + P.n[0] - 1) at_byte(Bn, o + 8) = bu[0];
+  if (j == NGH + P.n[1] - 1) at_byte(Bn + fs, o + oj) = bu[1];
+  if (k == NGH + P.n[2] - 1) at_byte(Bn + 2 * fs, o + ok) = bu[2];
+  if constexpr (BG) {  // div of B + B0 (face-normal B0, src/solver_func.c:324-343)
+    const double* f0 = P.bg + (size_t)BG_FACE * fs;
+    const double* f1 = P.bg + (size_t)(BG_FACE + 4) * fs;
+    const double* f2 = P.bg + (size_t)(BG_FACE + 8) * fs;
+    dbmax = fabs(((bu[0] + at_byte(f0, o + 8)) - (bl[0] + at_byte(f0, o))) * il[0] +
+                 ((bu[1] + at_byte(f1, o + oj)) - (bl[1] + at_byte(f1, o))) * il[1] +
+                 ((bu[2] + at_byte(f2, o + ok)) - (bl[2] + at_byte(f2, o))) * il[2]);
+  } else {
+    dbmax = fabs((bu[0] - bl[0]) * il[0] + (bu[1] - bl[1]) * il[1] + (bu[2] - bl[2]) * il[2]);
+  }
+  // cell-centred B0 (magtot = mags + B0)
+  double c0[3] = {0.0, 0.0, 0.0};
+  if constexpr (BG) {
+#pragma unroll
+    for (int a = 0; a < 3; a++) c0[a] = at_byte(P.bg + (size_t)(BG_B0 + a) * fs, o);
+  }
+  double mn[3], mt[3];
+  mn[0] = bl[0] * tb(P, 0, T_MA, i) + bu[0] * tb(P, 0, T_MB, i);
+  mn[1] = bl[1] * tb(P, 1, T_MA, j) + bu[1] * tb(P, 1, T_MB, j);
+  mn[2] = bl[2] * tb(P, 2, T_MA, k) + bu[2] * tb(P, 2, T_MB, k);
+#pragma unroll
+  for (int a = 0; a < 3; a++) mt[a] = BG ? 0.5 * (mn[a] + mo[a]) + c0[a] : 0.5 * (mn[a] + mo[a]);
+
+  // U^n from W^n, conservative update, cons->prim in FP64
+  // (src/solver_func.c:356-382, src/solver_solve.c:326-377)
+  const double gm1 = P.gm1;
+  const double r0 = at_byte(W, o), p0 = at_byte(W + 4 * fs, o);
+  double w0[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) w0[a] = at_byte(W + (1 + a) * fs, o);
+  const double U0[3] = {r0 * w0[0], r0 * w0[1], r0 * w0[2]};
+  const double E0n = 0.5 * r0 * (w0[0] * w0[0] + w0[1] * w0[1] + w0[2] * w0[2]) + p0 * P.inv_gm1;
+  const double Ur = r0 - dt * (double)du[0];
+  double Um[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) Um[a] = U0[a] - dt * (double)du[1 + a];
+  const double Ue = E0n - dt * (double)du[4];
+  double rho = Ur;
+  const double irho = 1.0 / Ur;
+  double vv[3] = {Um[0] * irho, Um[1] * irho, Um[2] * irho};
+  double p = (Ue - 0.5 * (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]) * rho) * gm1;
+  double pS = 0.0;
+  if constexpr (PSL) {  // entropy S = p_S / rho^(gamma-1), updated and back
+    const double ps0 = at_byte(W + 5 * fs, o);
+    const double S0 = (ps0 == 0.0 && r0 > 0.0) ? ps0 : ps0 / pow(r0, gm1);
+    const double Us = S0 - dt * (double)du[5];
+    pS = (Us == 0.0 && Ur > 0.0) ? Us : Us * pow(Ur, gm1);
+  }
+  // positivity floors (src/solver_func.c:2117-2135)
+  if (rho < P.rho_floor) {
+    rho = P.rho_floor;
+    p = P.p_floor;
+  }
+  if (p < P.p_floor) p = P.p_floor;
+
+  // Alfven/Boris correction of the momentum (src/solver_solve.c:385-484)
+  {
+    const RA bsq = (RA)(mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
+    RA alf, perp;
+    if constexpr (sizeof(RA) == 8) {  // b^2 / (rho ca^2) and 1 / (1 + that) by one division
+      const double rc = rho * P.ca2, q = rc + bsq, inv = 1.0 / (rc * q);
+      alf = bsq * q * inv;
+      perp = rc * rc * inv;
+    } else {
+      alf = bsq / ((RA)rho * (RA)P.ca2);
+      perp = RA(1) / (RA(1) + alf);
+    }
+    const RA rdt = (RA)dt;
+    const RA drho = -rdt * (RA)du[0];
+    const RA dva = alf * drho;
+    RA tv[3], wv[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      wv[a] = (RA)w0[a];
+      tv[a] = alf * (-rdt * (RA)du[1 + a] - drho * wv[a]);
+    }
+    RA bdv = (RA)mt[0] * tv[0] + (RA)mt[1] * tv[1] + (RA)mt[2] * tv[2];
+    bdv = bdv / (bsq + RA(1e-10));
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const RA inc = perp * ((-rdt * (RA)du[1 + a]) + (-rdt * (RA)dm[a]) + dva * wv[a] + (RA)mt[a] * bdv);
+      vv[a] = (U0[a] + (double)inc) * irho;
+    }
+  }
+  at_byte(Wn, o) = rho;
+#pragma unroll
+  for (int a = 0; a < 3; a++) at_byte(Wn + (1 + a) * fs, o) = vv[a];
+  at_byte(Wn + 4 * fs, o) = p;
+  if constexpr (PSL) at_byte(Wn + 5 * fs, o) = pS;  // else it stays zero in both buffers
+
+  // CFL rate of the new state with magtot = mags^{n+1} (src/solver_func.c:255-298)
+  {
+    const double t0 = mn[0] + c0[0], t1 = mn[1] + c0[1], t2 = mn[2] + c0[2];
+    rate = cfl_cart<RC>(P, il, rho, vv[0], vv[1], vv[2], p, t0 * t0 + t1 * t1 + t2 * t2);
+  }
+  if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
+    P.scal[S_FLAGS] = 1.0;
+}
+
+}  // namespace gop

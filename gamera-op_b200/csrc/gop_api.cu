@@ -1307,7 +1307,7 @@ int gop_set_sweep(gop_instance* h, int on) {
   if (!h) return fail(GOP_EINVAL, "instance is NULL");
   if (on && !h->sweep) return fail(GOP_ENODEV, "the tile-staged sweep kernels are not available");
   CK(cudaStreamSynchronize(h->st));
-  h->tune.flux_sweep = h->tune.emf_sweep = on != 0;
+  h->tune.flux_sweep = h->tune.emf_sweep = h->tune.update_sweep = on != 0;
   drop_step_graph(h);
   return GOP_OK;
 }
@@ -1488,7 +1488,7 @@ static int batch_pick_sweeps(gop_batch* b) {
     std::vector<Tune> pick(nm);
     for (size_t i = 0; i < nm; i++) pick[i] = b->m[i]->tune;
     for (gop_instance* h : b->m) {
-      h->tune.flux_sweep = h->tune.emf_sweep = false;
+      h->tune.flux_sweep = h->tune.emf_sweep = h->tune.update_sweep = false;
       drop_step_graph(h);
     }
     if (rc == GOP_OK) rc = batch_build(b);

@@ -405,7 +405,9 @@ template <int COORD, typename R, bool BG, bool PSL>
 __device__ __forceinline__ void update_body(const Params& P, const Work<R>& wk, Pos t,
                                             double& rate, double& dbmax) {
   if constexpr (COORD == 0) {
-    update_cart<R, BG, PSL>(P, wk, t, FluxPoint<R>{P, wk}, rate, dbmax);
+    const int ci = NGH + t.x, cj = NGH + t.y, ck = NGH + t.z;
+    if (ci >= NGH + P.n[0] || cj >= NGH + P.n[1] || ck >= NGH + P.n[2]) return;
+    update_cart<R, BG, PSL>(P, PointReader<R>(P, wk, ci, cj, ck), ci, cj, ck, rate, dbmax);
     return;
   }
   const int i = NGH + t.x, j = NGH + t.y, k = NGH + t.z;
@@ -1089,7 +1091,7 @@ Tune::Tune() {
   for (int d = 0; d < 3; d++) {
     flux_order[d] = emf_order[d] = d;
   }
-  flux_sweep = emf_sweep = true;
+  flux_sweep = emf_sweep = update_sweep = true;
 }
 
 dim3 launch_space(const Params& P, int slot) {
@@ -1240,7 +1242,8 @@ void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t
     const dim3 blk = tune.blk[K_UPDATE];
     LAUNCH_PDL(!after_emf_sweep, (k_ct<2, R>), grid3(P.n[0], P.n[1], P.n[2], blk), blk, st, P, w);
   }
-  launch_slot<R>(P, coord, w, K_UPDATE, tune.blk[K_UPDATE], st, coord != 0 || !after_emf_sweep);
+  if (!(coord == 0 && tune.update_sweep && launch_update_sweep<R>(sw, P, w, st)))
+    launch_slot<R>(P, coord, w, K_UPDATE, tune.blk[K_UPDATE], st, coord != 0 || !after_emf_sweep);
   // the work arrays are free after the update: 2 fields of doubles of scratch
   if (P.ring) {
     launch_ring_average(P, reinterpret_cast<double*>(w.Wh), st);

@@ -44,6 +44,7 @@ struct Tune {
   // (gop_sweep.cu) instead of the per-point kernels, where the sweeps apply
   bool flux_sweep;
   bool emf_sweep;
+  bool update_sweep;  // the Cartesian update from tiles as well
   // order of the axes (independent) in the flux and EMF stages
   int flux_order[3];
   int emf_order[3];
@@ -65,6 +66,10 @@ bool launch_flux_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, co
 template <typename R>
 bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, const int order[3],
                       cudaStream_t st);
+
+// the update of a Cartesian grid from TMA-filled tiles; false as above
+template <typename R>
+bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st);
 
 // points covered by the launch of one slot (x, y, z extents)
 dim3 launch_space(const Params& P, int slot);

@@ -46,6 +46,7 @@
 
 #include "gop_stage.cuh"
 #include "gop_tma.cuh"
+#include "gop_update.cuh"
 
 namespace gop {
 
@@ -180,39 +181,52 @@ __host__ __device__ constexpr uint64_t inverse_of(int d) { return d > 1 ? ~0ull 
 __device__ __forceinline__ int div_by(int n, int d, uint64_t inv) {
   return d > 1 ? (int)__umul64hi((uint64_t)n, inv) : n;
 }
-// Tile r of the nt[0] x nt[1] x nt[2] tiles of a sweep along D, x fastest.
-// The feeding thread works this out and the others read it from shared
-// memory; its warp is the last of the block at every tile, so the two
+// Tile r of the nt[0] x nt[1] x nt[2] tiles of a stage, x fastest, as its three
+// digits.  The feeding thread works this out and the others read the tile from
+// shared memory; its warp is the last of the block at every tile, so the two
 // divisions are products with the counts' inverses (FP64 EMF stage 1.81 ->
 // 1.76 ms per blast 256^3 step on B200).
-template <int D, bool EMF, int ROWS, class Maps>
-__device__ __forceinline__ Tile tile_of(const Params& P, const Maps& m, int r) {
+template <class Maps>
+__device__ __forceinline__ int3 tile_digits(const Maps& m, int r) {
   const int* nt = m.nt;
   const int q = div_by(r, nt[0], m.inv[0]), c = div_by(q, nt[1], m.inv[1]);
-  const int a = r - q * nt[0], b = q - c * nt[1];
+  return make_int3(r - q * nt[0], q - c * nt[1], c);
+}
+// a tile of a sweep along D
+template <int D, bool EMF, int ROWS, class Maps>
+__device__ __forceinline__ Tile sweep_tile(const Params& P, const Maps& m, int r) {
+  const int3 d = tile_digits(m, r);
   Tile T;
   T.D = D;
-  T.x0 = NGH + 32 * a;
+  T.x0 = NGH + 32 * d.x;
   // the rows of a tile run along k where its windows do (flux along k, EMFs
   // along i and j), along j otherwise
   if constexpr (EMF ? D != 2 : D == 2) {
-    T.y0 = NGH + c;
-    T.z0 = NGH + ROWS * b;
+    T.y0 = NGH + d.z;
+    T.z0 = NGH + ROWS * d.y;
   } else {
-    T.y0 = NGH + ROWS * b;
-    T.z0 = NGH + c;
+    T.y0 = NGH + ROWS * d.y;
+    T.z0 = NGH + d.z;
   }
   // the warp of the row-end pass rotates over the row sets
   constexpr bool ends = EMF ? D != 0 : D == 0;
-  T.end_warp = ends && row_end_face(P, T.x0) ? (short)((b + nt[1] * c) & (kWarps - 1)) : (short)-1;
+  T.end_warp = ends && row_end_face(P, T.x0) ? (short)((d.y + m.nt[1] * d.z) & (kWarps - 1)) : (short)-1;
   return T;
 }
+// what a thread gathers over its tiles (the update)
+struct Gather {
+  double rate = 0.0, divb = 0.0;
+};
 
 template <typename R, int D, bool BG>
 struct FluxStage {
   using F = FluxTile<D>;
   using Maps = FluxMaps;
   static constexpr int ELEMS = F::ELEMS, ROWS = F::ROWS;
+  static constexpr int BYTES = F::TX * (int)sizeof(R);
+  __device__ static Tile place(const Params& P, const Maps& m, int r) {
+    return sweep_tile<D, false, ROWS>(P, m, r);
+  }
   static constexpr int TX = F::TX;
 
   __device__ static void issue(const Params& P, const Maps& m, int par, const Tile& T, R* s,
@@ -233,7 +247,7 @@ struct FluxStage {
 
   // the face in tile row `row` (a warp's row), column `col` (a lane's face)
   __device__ __forceinline__ static void point(const Params& P, const Work<R>& wk, const R* s,
-                                               const Tile& T, int row, int col) {
+                                               const Tile& T, int row, int col, Gather&) {
     const int i = T.x0 + col, j = T.y0 + (D == 2 ? 0 : row), k = T.z0 + (D == 2 ? row : 0);
     if (!(i < NGH + P.n[0] + (D == 0) && j < NGH + P.n[1] + (D == 1) && k < NGH + P.n[2] + (D == 2)))
       return;
@@ -342,6 +356,10 @@ struct EmfStage {
   using E = EmfTile<D>;
   using Maps = EmfMaps;
   static constexpr int ELEMS = E::ELEMS, ROWS = E::ROWS;
+  static constexpr int BYTES = E::TX * (int)sizeof(R);
+  __device__ static Tile place(const Params& P, const Maps& m, int r) {
+    return sweep_tile<D, true, ROWS>(P, m, r);
+  }
   static constexpr int TX = E::TX;
   static constexpr int p = (D + 1) % 3, q = (D + 2) % 3;
 
@@ -380,7 +398,7 @@ struct EmfStage {
 
   // the edge in tile row `warp` (a warp's row), column `lane` (a lane's edge)
   __device__ __forceinline__ static void point(const Params& P, const Work<R>& wk, const R* s,
-                                               const Tile& T, int warp, int lane) {
+                                               const Tile& T, int warp, int lane, Gather&) {
     const int i = T.x0 + lane, j = T.y0 + (D == 2 ? warp : 0), k = T.z0 + (D == 2 ? 0 : warp);
     if (!(i < NGH + P.n[0] + (D != 0) && j < NGH + P.n[1] + (D != 1) && k < NGH + P.n[2] + (D != 2)))
       return;
@@ -473,7 +491,7 @@ struct EmfStage {
 // MASK: the axes it is compiled for (bit d).
 template <typename R, bool EMF_, bool BG, unsigned MASK_>
 struct Sweep {
-  static constexpr bool EMF = EMF_;
+  static constexpr bool EMF = EMF_, STATE = false;
   static constexpr unsigned MASK = MASK_;
   static constexpr bool H0 = MASK & 1, H1 = MASK >> 1 & 1, H2 = MASK >> 2 & 1;
   template <int D>
@@ -527,15 +545,15 @@ struct alignas(64) SweepMaps {
 // stage of a blast 256^3 step 3.16 ms, with the counter 2.40).  In a batch a block that starts late finds less work left.
 template <class SW, typename R>
 __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
-                                          const SweepMaps<typename SW::Maps>& maps) {
+                                          const SweepMaps<typename SW::Maps>& maps, Gather& gather) {
   // stop flag, or an earlier pipeline wait that timed out: do nothing
   if (stopped(P) || P.scal[S_FLAGS] == 2.0) return;
   constexpr int S = SW::S;
   using S0 = typename SW::template Stage<0>;
   using S1 = typename SW::template Stage<1>;
   using S2 = typename SW::template Stage<2>;
-  static_assert((!SW::H0 || S0::TX <= SW::ELEMS) && (!SW::H1 || S1::TX <= SW::ELEMS) &&
-                    (!SW::H2 || S2::TX <= SW::ELEMS),
+  static_assert((!SW::H0 || S0::BYTES <= SW::SLOT) && (!SW::H1 || S1::BYTES <= SW::SLOT) &&
+                    (!SW::H2 || S2::BYTES <= SW::SLOT),
                 "slot holds its boxes");
   extern __shared__ unsigned char smem_dyn[];
   // TMA destinations on 128-byte boundaries (the launch adds 128 bytes)
@@ -547,7 +565,7 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
   uint64_t* empty = full + S;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntiles = maps.first[3];
-  const int par = sizeof(R) == 8 ? cur_buf(P) : 0;
+  const int par = SW::STATE || sizeof(R) == 8 ? cur_buf(P) : 0;
   // the feeder: tile t into slot q
   auto issue = [&](int q, int t) {
     const int g = (t >= maps.first[1]) + (t >= maps.first[2]), r = t - maps.first[g];
@@ -557,9 +575,9 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
       using St = decltype(stage);
       constexpr int D = decltype(d)::value;
       if constexpr (!(SW::MASK >> D & 1)) return;
-      const Tile T = tile_of<D, SW::EMF, St::ROWS>(P, maps.m[D], r);
+      const Tile T = St::place(P, maps.m[D], r);
       tiles[q] = T;
-      mbar_arrive_expect_tx(bar, St::TX * (int)sizeof(R));
+      mbar_arrive_expect_tx(bar, St::BYTES);
       St::issue(P, maps.m[D], par, T, slot, bar);
     };
     const int D = maps.order[g];
@@ -612,7 +630,7 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
       int row = warp, col = lane;
 #pragma unroll 1
       for (;;) {
-        St::point(P, wk, slot, T, row, col);
+        St::point(P, wk, slot, T, row, col, gather);
         if (St::ROWS > kWarps && col < 32 && row + kWarps < St::ROWS) {
           row += kWarps;
           continue;
@@ -668,7 +686,160 @@ __global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, EMF>::CTAS))
     k_sweep(Params P, Work<R> wk,
             const __grid_constant__ SweepMaps<typename Sweep<R, EMF, BG, MASK>::Maps> maps) {
   pdl_enter();
-  sweep_run<Sweep<R, EMF, BG, MASK>, R>(P, wk, maps);
+  Gather none;
+  sweep_run<Sweep<R, EMF, BG, MASK>, R>(P, wk, maps, none);
+}
+
+// ---------------------------------------------------------------- update
+
+// The Cartesian update from tiles of 32 x 4 x 2 cells (a warp per row along
+// i): everything a cell reads -- 24 face fluxes with their upper neighbours, 12
+// edge EMFs, 6 face and 5 state values -- comes by the tile's 14 copies.  The
+// per-cell kernel waits for its 71 loads a few at a time (long-scoreboard
+// stalls 5.6 per instruction, 4.5 TB/s at 256^3 FP64).
+template <typename R>
+struct UpdTile {
+  // the faces along each axis, the edges along each axis
+  __host__ __device__ static constexpr Box F(int d) {
+    return d == 0 ? Box{36, 4, 2, 1} : (d == 1 ? Box{32, 5, 2, 1} : Box{32, 4, 3, 1});
+  }
+  __host__ __device__ static constexpr Box E(int d) {
+    return d == 0 ? Box{32, 5, 3, 1} : (d == 1 ? Box{36, 4, 3, 1} : Box{36, 5, 2, 1});
+  }
+  static constexpr Box W{32, 4, 2, 5};
+  __host__ __device__ static constexpr int up(int bytes) { return (bytes + 127) / 128 * 128; }
+  static constexpr int RS = sizeof(R);
+  // byte offsets in the slot: the 5 hydro and the 3 stress fluxes of each
+  // axis, the EMFs, the face field (FP64), the state (FP64)
+  __host__ __device__ static constexpr int f(int d) {
+    int o = 0;
+    for (int a = 0; a < d; a++) o += up(5 * F(a).elems() * RS) + up(3 * F(a).elems() * RS);
+    return o;
+  }
+  __host__ __device__ static constexpr int g(int d) { return f(d) + up(5 * F(d).elems() * RS); }
+  __host__ __device__ static constexpr int e(int d) {
+    int o = f(3);
+    for (int a = 0; a < d; a++) o += up(E(a).elems() * RS);
+    return o;
+  }
+  __host__ __device__ static constexpr int b(int d) {
+    int o = e(3);
+    for (int a = 0; a < d; a++) o += up(F(a).elems() * 8);
+    return o;
+  }
+  __host__ __device__ static constexpr int w() { return b(3); }
+  static constexpr int SLOT = w() + up(W.elems() * 8);
+  static constexpr int BYTES = 8 * (F(0).elems() + F(1).elems() + F(2).elems()) * (RS + 1) +
+                               (E(0).elems() + E(1).elems() + E(2).elems()) * RS + W.elems() * 8;
+};
+
+struct alignas(64) UpdMaps {
+  CUtensorMap f[3], g[3];  // fluxes along each axis: hydro, stress
+  CUtensorMap e[3];        // EMFs
+  CUtensorMap b[3][2];     // step-start face field, of either parity
+  CUtensorMap w[2];        // step-start state
+  int nt[3];
+  uint64_t inv[2];
+};
+
+// the reader of update_cart on a slot: column c, row (jj, kk) of the tile
+template <typename R>
+struct TileReader {
+  using U = UpdTile<R>;
+  const unsigned char* s;
+  int c, jj, kk;
+  template <typename T>
+  __device__ __forceinline__ T at(int off, int idx) const {
+    return reinterpret_cast<const T*>(s + off)[idx];
+  }
+  __device__ __forceinline__ int face_at(int d, int u) const {
+    return d == 0 ? (kk * 4 + jj) * 36 + c + u
+                  : (d == 1 ? (kk * 5 + jj + u) * 32 + c : ((kk + u) * 4 + jj) * 32 + c);
+  }
+  __device__ __forceinline__ R flux(int d, int m, int u) const {
+    constexpr int f[3] = {U::f(0), U::f(1), U::f(2)}, g[3] = {U::g(0), U::g(1), U::g(2)};
+    constexpr int n[3] = {U::F(0).elems(), U::F(1).elems(), U::F(2).elems()};
+    return m < 5 ? at<R>(f[d], m * n[d] + face_at(d, u)) : at<R>(g[d], (m - 6) * n[d] + face_at(d, u));
+  }
+  __device__ __forceinline__ double emf(int a, int di, int dj, int dk) const {
+    constexpr int e[3] = {U::e(0), U::e(1), U::e(2)};
+    const int idx = a == 0 ? ((kk + dk) * 5 + jj + dj) * 32 + c
+                           : (a == 1 ? ((kk + dk) * 4 + jj) * 36 + c + di : (kk * 5 + jj + dj) * 36 + c + di);
+    return (double)at<R>(e[a], idx);
+  }
+  __device__ __forceinline__ double face(int a, int u) const {
+    constexpr int b[3] = {U::b(0), U::b(1), U::b(2)};
+    return at<double>(b[a], face_at(a, u));
+  }
+  __device__ __forceinline__ double state(int m) const {
+    return at<double>(U::w(), ((m * 2 + kk) * 4 + jj) * 32 + c);
+  }
+};
+
+template <typename R, bool BG>
+struct UpdStage {
+  using U = UpdTile<R>;
+  using Maps = UpdMaps;
+  static constexpr int ELEMS = U::SLOT / (int)sizeof(R), ROWS = kWarps, BYTES = U::BYTES;
+  __device__ static Tile place(const Params& P, const Maps& m, int r) {
+    const int3 d = tile_digits(m, r);
+    return Tile{0, -1, NGH + 32 * d.x, NGH + 4 * d.y, NGH + 2 * d.z};
+  }
+  __device__ static void issue(const Params& P, const Maps& m, int par, const Tile& T, R* slot,
+                               uint64_t* bar) {
+    unsigned char* s = reinterpret_cast<unsigned char*>(slot);
+    const int x = T.x0, y = T.y0, z = T.z0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      tma_load_4d(s + U::f(d), &m.f[d], bar, x, y, z, 9 * d);
+      tma_load_4d(s + U::g(d), &m.g[d], bar, x, y, z, 9 * d + 6);
+      tma_load_4d(s + U::e(d), &m.e[d], bar, x, y, z, d);
+      tma_load_4d(s + U::b(d), &m.b[d][par], bar, x, y, z, d);
+    }
+    tma_load_4d(s + U::w(), &m.w[par], bar, x, y, z, 0);
+  }
+  __device__ __forceinline__ static void point(const Params& P, const Work<R>& wk, const R* slot,
+                                               const Tile& T, int row, int col, Gather& out) {
+    const int jj = row & 3, kk = row >> 2;
+    const int i = T.x0 + col, j = T.y0 + jj, k = T.z0 + kk;
+    if (!(i < NGH + P.n[0] && j < NGH + P.n[1] && k < NGH + P.n[2])) return;
+    double rate, divb;
+    update_cart<R, BG, false>(P, TileReader<R>{reinterpret_cast<const unsigned char*>(slot), col, jj, kk},
+                              i, j, k, rate, divb);
+    out.rate = fmax(out.rate, rate);
+    out.divb = fmax(out.divb, divb);
+  }
+};
+
+// Two slots, as many blocks per SM as then fit: one in FP64 (90 KB a slot, 8
+// warps of up to 255 registers), two in FP32.  What bounds it is that the
+// copies run ahead: with one slot a block loads and computes in turn.  Blast
+// 256^3 on B200, us a launch: FP64 one slot and two blocks 1256, two slots and
+// one block 1108 (per cell 1275); FP32 one slot and three or four blocks 930,
+// 1055, two slots and two blocks 854 (per cell 983).
+template <typename R, bool BG>
+struct UpdSweep {
+  static constexpr bool EMF = false, STATE = true;
+  static constexpr unsigned MASK = 1;
+  static constexpr bool H0 = true, H1 = false, H2 = false;
+  template <int D>
+  using Stage = UpdStage<R, BG>;
+  using Maps = UpdMaps;
+  static constexpr int ELEMS = Stage<0>::ELEMS, SLOT = UpdTile<R>::SLOT;
+  static constexpr int CTAS = sizeof(R) == 8 ? 1 : 2, S = 2;
+  static constexpr int SMEM = S * SLOT + S * (2 * 8 + (int)sizeof(Tile)) + 128;
+  static_assert((SMEM + 1024) * CTAS <= 228 * 1024, "update blocks per SM");
+};
+
+template <typename R, bool BG>
+__global__ void __launch_bounds__(kSweepThreads, (UpdSweep<R, BG>::CTAS))
+    k_update_sweep(Params P, Work<R> wk, const __grid_constant__ SweepMaps<UpdMaps> maps) {
+  pdl_enter();
+  if (stopped(P)) return;
+  Gather g;
+  sweep_run<UpdSweep<R, BG>, R>(P, wk, maps, g);
+  using RC = typename std::conditional<GOP_MX_CFL64, double, R>::type;
+  block_commit<RC>(P, g.rate, g.divb);
 }
 
 template <typename R, unsigned MASK>
@@ -806,9 +977,30 @@ static bool make_emf_maps(EmfMaps& m, const Params& P, const Work<R>& w) {
   return ok;
 }
 
+template <typename R>
+static bool make_upd_maps(UpdMaps& m, const Params& P, const Work<R>& w) {
+  using U = UpdTile<R>;
+  bool ok = true;
+  for (int d = 0; d < 3 && ok; d++) {
+    Box f = U::F(d), g = U::F(d);
+    f.f = 5;
+    g.f = 3;
+    ok = field_map<R>(&m.f[d], w.F, 27, P, f) && field_map<R>(&m.g[d], w.F, 27, P, g) &&
+         field_map<R>(&m.e[d], w.E, 3, P, U::E(d));
+    for (int b = 0; b < 2 && ok; b++) ok = field_map<double>(&m.b[d][b], P.Bbuf[b], 3, P, U::F(d));
+  }
+  for (int b = 0; b < 2 && ok; b++) ok = field_map<double>(&m.w[b], P.Wbuf[b], 6, P, U::W);
+  m.nt[0] = (P.n[0] + 31) / 32;
+  m.nt[1] = (P.n[1] + 3) / 4;
+  m.nt[2] = (P.n[2] + 1) / 2;
+  for (int a = 0; a < 2; a++) m.inv[a] = inverse_of(m.nt[a]);
+  return ok;
+}
+
 struct SweepSet {
   SweepMaps<FluxMaps> flux;
   SweepMaps<EmfMaps> emf;
+  SweepMaps<UpdMaps> upd;
   int sms = 0;
 };
 
@@ -820,7 +1012,9 @@ static bool allow_smem() {
 template <typename R, bool BG>
 static bool allow_smem() {
   return allow_smem<R, false, BG, 1>() && allow_smem<R, false, BG, 2>() && allow_smem<R, false, BG, 4>() &&
-         allow_smem<R, false, BG, 7>() && allow_smem<R, true, BG, 7>();
+         allow_smem<R, false, BG, 7>() && allow_smem<R, true, BG, 7>() &&
+         cudaFuncSetAttribute(k_update_sweep<R, BG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              UpdSweep<R, BG>::SMEM) == cudaSuccess;
 }
 
 template <typename R>
@@ -833,7 +1027,7 @@ SweepSet* sweep_create(const Params& P, const Work<R>& w) {
   ok = ok && make_flux_maps<R, 0>(s->flux.m[0], P, w) && make_flux_maps<R, 1>(s->flux.m[1], P, w) &&
        make_flux_maps<R, 2>(s->flux.m[2], P, w) && make_emf_maps<R, 0>(s->emf.m[0], P, w) &&
        make_emf_maps<R, 1>(s->emf.m[1], P, w) && make_emf_maps<R, 2>(s->emf.m[2], P, w);
-  ok = ok && allow_smem<R, false>() && allow_smem<R, true>();
+  ok = ok && make_upd_maps<R>(s->upd.m[0], P, w) && allow_smem<R, false>() && allow_smem<R, true>();
   if (!ok) {
     cudaGetLastError();
     delete s;
@@ -918,7 +1112,23 @@ bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, con
   else launch_axes<R, true, false>(sw, P, w, sw->emf, order, st);
   return true;
 }
+// Where a block has too few tiles to fill its ring before it ends, the per-cell
+// kernel is as fast or faster (B200, us, tiles / per cell: Orszag-Tang 64x64x4
+// FP64 11 / 9; blast 77x45x21 17 / 15; 64^3 FP64 30.9 / 31.2, FP32 29.4 / 28.3,
+// with 3.5 to 7 tiles a block; 128^3 150 / 171, 115 / 134).
+constexpr int kUpdTiles = 6;
+template <typename R>
+bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
+  if (!sw || P.ps_live) return false;
+  const int* nt = sw->upd.m[0].nt;
+  if ((long long)nt[0] * nt[1] * nt[2] < (long long)kUpdTiles * sw->sms * UpdSweep<R, false>::CTAS) return false;
+  static const int order[3] = {0, 1, 2};
+  if (P.bg) launch_persistent<UpdSweep<R, true>, R>(k_update_sweep<R, true>, sw, P, w, sw->upd, order, st);
+  else launch_persistent<UpdSweep<R, false>, R>(k_update_sweep<R, false>, sw, P, w, sw->upd, order, st);
+  return true;
+}
 #define GOP_INST(R)                                                                            \
+  template bool launch_update_sweep<R>(const SweepSet*, const Params&, const Work<R>&, cudaStream_t); \
   template bool launch_flux_sweep<R>(const SweepSet*, const Params&, const Work<R>&,            \
                                      const int[3], cudaStream_t);                     \
   template bool launch_emf_sweep<R>(const SweepSet*, const Params&, const Work<R>&,             \

@@ -111,17 +111,36 @@ __device__ __forceinline__ double cfl_cart(const Params& P, const double il[3], 
   return (double)(vc * (T)il[0] + vc * (T)il[1] + vc * (T)il[2]);
 }
 
-// the face fluxes from global memory
+// What a cell's update reads, from global memory: the fluxes of its faces,
+// the EMFs of its edges, its face field and its state
 template <typename R>
-struct FluxPoint {
+struct PointReader {
   const Params& P;
   const Work<R>& wk;
-  __device__ __forceinline__ R operator()(const Pos& t, int d, int m, bool upper) const {
-    constexpr unsigned RS = sizeof(R);
-    const unsigned r = RS * (unsigned)lin32(P, NGH + t.x, NGH + t.y, NGH + t.z);
-    const unsigned s = d == 0 ? RS : RS * (unsigned)(d == 1 ? P.sj : P.sk);
-    return at_byte(wk.F + (size_t)(9 * d + m) * P.fs, upper ? r + s : r);
+  const double *W, *B;  // step-start state
+  // byte offsets of the cell and of its upper neighbours along j and k: o
+  // in the FP64 state, r in the stage arrays
+  unsigned o, oj, ok, r, rj, rk;
+  static constexpr unsigned RS = sizeof(R);
+  __device__ __forceinline__ PointReader(const Params& p, const Work<R>& w, int i, int j, int k)
+      : P(p), wk(w), W(p.Wbuf[cur_buf(p)]), B(p.Bbuf[cur_buf(p)]) {
+    const unsigned x = lin32(P, i, j, k);
+    o = 8 * x, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
+    r = RS * x, rj = RS * (unsigned)P.sj, rk = RS * (unsigned)P.sk;
   }
+  // flux m at the lower (u = 0) or upper face along axis d
+  __device__ __forceinline__ R flux(int d, int m, int u) const {
+    const unsigned s = d == 0 ? RS : (d == 1 ? rj : rk);
+    return at_byte(static_cast<const R*>(wk.F) + (size_t)(9 * d + m) * P.fs, u ? r + s : r);
+  }
+  // EMF along a at the edge di, dj, dk cells up
+  __device__ __forceinline__ double emf(int a, int di, int dj, int dk) const {
+    return (double)at_byte(static_cast<const R*>(wk.E) + a * P.fs, r + di * RS + dj * rj + dk * rk);
+  }
+  __device__ __forceinline__ double face(int a, int u) const {
+    return at_byte(B + a * P.fs, u ? o + (a == 0 ? 8u : (a == 1 ? oj : ok)) : o);
+  }
+  __device__ __forceinline__ double state(int m) const { return at_byte(W + m * P.fs, o); }
 };
 
 // One active cell of a Cartesian grid (src/solver_solve.c:263-484 with the
@@ -132,29 +151,21 @@ struct FluxPoint {
 // conservative update and the pressure recovery are FP64; with R = float
 // the flux divergence, the Alfven/Boris correction and the CFL estimate are
 // FP32.  Returns the cell's CFL rate and |div B| of the new state.
-// flux(d, m, upper): flux m at the cell's lower or upper face along axis d.
-template <typename R, bool BG, bool PSL, class Flux>
-__device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, Pos t, const Flux& flux,
+// in: the PointReader of cell (i, j, k), or one like it.
+template <typename R, bool BG, bool PSL, class Reader>
+__device__ __forceinline__ void update_cart(const Params& P, const Reader& in, int i, int j, int k,
                                             double& rate, double& dbmax) {
   // arithmetic of the stages the mixed path runs in FP32 (FP64 when their
   // option is on, and always on the plain path)
   using RD = typename std::conditional<sizeof(R) == 8 || GOP_MX_DIV64, double, R>::type;
   using RA = typename std::conditional<sizeof(R) == 8 || GOP_MX_ALF64, double, R>::type;
   using RC = typename std::conditional<sizeof(R) == 8 || GOP_MX_CFL64, double, R>::type;
-  const int i = NGH + t.x, j = NGH + t.y, k = NGH + t.z;
-  if (i >= NGH + P.n[0] || j >= NGH + P.n[1] || k >= NGH + P.n[2]) return;
   const size_t fs = P.fs;
   const double dt = P.scal[S_DT];
-  const int cb = cur_buf(P);
-  const double* W = P.Wbuf[cb];
-  const double* B = P.Bbuf[cb];
-  double* Wn = P.Wbuf[1 - cb];
-  double* Bn = P.Bbuf[1 - cb];
-  // byte offsets of the cell and of its upper neighbours along j and k: o
-  // in the FP64 state, r in the stage arrays
+  const int nb = 1 - cur_buf(P);
+  double* Wn = P.Wbuf[nb];
+  double* Bn = P.Bbuf[nb];
   const unsigned x = lin32(P, i, j, k), o = 8 * x, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
-  constexpr unsigned RS = sizeof(R);
-  const unsigned r = RS * x, rj = RS * (unsigned)P.sj, rk = RS * (unsigned)P.sk;
   const double il[3] = {tb(P, 0, T_IDX, i), tb(P, 1, T_IDX, j), tb(P, 2, T_IDX, k)};
 
   // flux divergence: 5 hydro (6 with the entropy channel) and 3 stress
@@ -167,7 +178,7 @@ __device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, 
 #pragma unroll
     for (int m = 0; m < 9; m++) {
       if (m == PS && !PSL) continue;
-      const R fu = flux(t, d, m, true), fl = flux(t, d, m, false);
+      const R fu = in.flux(d, m, 1), fl = in.flux(d, m, 0);
       const RD v = ((RD)fu - (RD)fl) * (RD)il[d];
       if (m < 6) du[m] = d == 0 ? v : du[m] + v;
       else dm[m - 6] = d == 0 ? v : dm[m - 6] + v;
@@ -181,14 +192,15 @@ __device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, 
   // constrained transport: face A gets -dt (curl E)_A from the differences of
   // the edge EMFs, in FP64 (src/solver_solve.c:263-306; the edge lengths over
   // the face area are inverse cell lengths)
-  const R *E0 = wk.E, *E1 = wk.E + fs, *E2 = wk.E + 2 * fs;
-  auto ld = [](const R* e, unsigned off) { return (double)at_byte(e, off); };
-  const double e0 = ld(E0, r), e0j = ld(E0, r + rj), e0k = ld(E0, r + rk), e0jk = ld(E0, r + rj + rk);
-  const double e1 = ld(E1, r), e1i = ld(E1, r + RS), e1k = ld(E1, r + rk), e1ik = ld(E1, r + RS + rk);
-  const double e2 = ld(E2, r), e2i = ld(E2, r + RS), e2j = ld(E2, r + rj), e2ij = ld(E2, r + RS + rj);
-  const double b0l = at_byte(B, o), b0u = at_byte(B, o + 8);
-  const double b1l = at_byte(B + fs, o), b1u = at_byte(B + fs, o + oj);
-  const double b2l = at_byte(B + 2 * fs, o), b2u = at_byte(B + 2 * fs, o + ok);
+  const double e0 = in.emf(0, 0, 0, 0), e0j = in.emf(0, 0, 1, 0), e0k = in.emf(0, 0, 0, 1),
+               e0jk = in.emf(0, 0, 1, 1);
+  const double e1 = in.emf(1, 0, 0, 0), e1i = in.emf(1, 1, 0, 0), e1k = in.emf(1, 0, 0, 1),
+               e1ik = in.emf(1, 1, 0, 1);
+  const double e2 = in.emf(2, 0, 0, 0), e2i = in.emf(2, 1, 0, 0), e2j = in.emf(2, 0, 1, 0),
+               e2ij = in.emf(2, 1, 1, 0);
+  const double b0l = in.face(0, 0), b0u = in.face(0, 1);
+  const double b1l = in.face(1, 0), b1u = in.face(1, 1);
+  const double b2l = in.face(2, 0), b2u = in.face(2, 1);
   double bl[3], bu[3], mo[3];
   bl[0] = b0l - dt * ((e2j - e2) * il[1] - (e1k - e1) * il[2]);
   bl[1] = b1l - dt * ((e0k - e0) * il[2] - (e2i - e2) * il[0]);
@@ -232,10 +244,10 @@ __device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, 
   // U^n from W^n, conservative update, cons->prim in FP64
   // (src/solver_func.c:356-382, src/solver_solve.c:326-377)
   const double gm1 = P.gm1;
-  const double r0 = at_byte(W, o), p0 = at_byte(W + 4 * fs, o);
+  const double r0 = in.state(0), p0 = in.state(4);
   double w0[3];
 #pragma unroll
-  for (int a = 0; a < 3; a++) w0[a] = at_byte(W + (1 + a) * fs, o);
+  for (int a = 0; a < 3; a++) w0[a] = in.state(1 + a);
   const double U0[3] = {r0 * w0[0], r0 * w0[1], r0 * w0[2]};
   const double E0n = 0.5 * r0 * (w0[0] * w0[0] + w0[1] * w0[1] + w0[2] * w0[2]) + p0 * P.inv_gm1;
   const double Ur = r0 - dt * (double)du[0];
@@ -249,7 +261,7 @@ __device__ __forceinline__ void update_cart(const Params& P, const Work<R>& wk, 
   double p = (Ue - 0.5 * (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]) * rho) * gm1;
   double pS = 0.0;
   if constexpr (PSL) {  // entropy S = p_S / rho^(gamma-1), updated and back
-    const double ps0 = at_byte(W + 5 * fs, o);
+    const double ps0 = in.state(5);
     const double S0 = (ps0 == 0.0 && r0 > 0.0) ? ps0 : ps0 / pow(r0, gm1);
     const double Us = S0 - dt * (double)du[5];
     pS = (Us == 0.0 && Ur > 0.0) ? Us : Us * pow(Ur, gm1);

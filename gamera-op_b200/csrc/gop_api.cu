@@ -153,7 +153,14 @@ void build_tables(const gop_desc& d, Tables& T) {
         T.at(0, T_G1, i) = 1.0 / 3.0 * (std::pow(r[i + 1], 3) - std::pow(r[i], 3));
         T.at(0, T_G2, i) = 0.5 * (r[i + 1] * r[i + 1] - r[i] * r[i]);
         T.at(0, T_G3, i) = xcv[0][i];
+        const double V = T.at(0, T_G1, i);
+        T.at(0, T_U0, i) = r[i] * r[i] / V;
+        T.at(0, T_U1, i) = r[i + 1] * r[i + 1] / V;
+        T.at(0, T_U2, i) = T.at(0, T_G2, i) / V;
+        T.at(0, T_U3, i) = 0.5 * dxv[0][i] / xcv[0][i];
+        T.at(0, T_U5, i) = 1.0 / T.at(0, T_G2, i);
       }
+      T.at(0, T_U4, i) = 1.0 / r[i];
     }
     for (int j = 0; j < N[1]; j++) {
       T.at(1, T_G1, j) = std::sin(t[j]);
@@ -162,7 +169,13 @@ void build_tables(const gop_desc& d, Tables& T) {
         T.at(1, T_G2, j) = std::sin(xcv[1][j]);
         T.at(1, T_G3, j) = std::sin(t[j + 1]) - std::sin(t[j]);
         T.at(1, T_G4, j) = std::sin(t[j + 1]) + std::sin(t[j]);
+        const double C = -T.at(1, T_G0, j);
+        T.at(1, T_U0, j) = std::sin(t[j]) / C;
+        T.at(1, T_U1, j) = std::sin(t[j + 1]) / C;
+        T.at(1, T_U2, j) = dxv[1][j] / C;
+        T.at(1, T_U3, j) = T.at(1, T_G3, j) / T.at(1, T_G4, j);
       }
+      T.at(1, T_U4, j) = 1.0 / std::sin(t[j]);
     }
   }
 

@@ -43,6 +43,14 @@ enum Tab : int {
   T_G2,
   T_G3,
   T_G4,
+  // spherical: quotients of the factors above that the update takes (see
+  // update_sph); axis 0 | axis 1, with V = G1 of axis 0, C = cos(t0) - cos(t1)
+  T_U0,        // r^2 / V             | sin(t) / C
+  T_U1,        // r1^2 / V            | sin(t1) / C
+  T_U2,        // G2 / V              | (t1 - t0) / C
+  T_U3,        // dr / (2 r_c)        | G3 / G4
+  T_U4,        // 1 / r               | 1 / sin(t)
+  T_U5,        // 1 / G2              |
   NTAB
 };
 

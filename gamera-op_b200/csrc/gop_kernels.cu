@@ -41,22 +41,6 @@ namespace gop {
 // ------------------------------------------------------------------ utils
 
 
-// CFL rate (signal speed over the cell's lengths) of one cell of a
-// curvilinear grid, in T arithmetic (FP32 for the mixed path's estimate)
-template <int COORD, typename T = double>
-__device__ __forceinline__ double cfl_cell(const Params& P, int i, int j, int k, double rho,
-                                           double u, double v, double w, double p, double b1,
-                                           double b2, double b3) {
-  const T x1 = (T)b1, x2 = (T)b2, x3 = (T)b3;
-  const T vc = signal_speed(P, (T)rho, (T)u, (T)v, (T)w, (T)p, x1 * x1 + x2 * x2 + x3 * x3);
-  T dk = (T)Geo<COORD>::dl(P, 2, i, j, k);
-  // the phi length of the pole rings is nk / nchunk times longer (dxk_ring,
-  // spherical_RingAverage.c:110-138; get_dt_ring, spherical_general.c:700-743)
-  if (COORD == 2 && P.ring) dk = (T)P.ringtab[2 * P.n[2] + j] * dk;
-  const T di = (T)Geo<COORD>::dl(P, 0, i, j, k), dj = (T)Geo<COORD>::dl(P, 1, i, j, k);
-  if constexpr (sizeof(T) == 8) return vc * ((dj * dk + di * dk + di * dj) / (di * dj * dk));
-  return (double)(vc / di + vc / dj + vc / dk);
-}
 // rows of cells whose state or face field the pole ring average changes
 // (the ring rows and the rows of the faces its EMF-like field touches)
 __device__ __forceinline__ bool ring_band_row(const Params& P, int j) {
@@ -356,8 +340,10 @@ __device__ __forceinline__ double ct_face(const Params& P, const double* __restr
   return B[x + A * fs] - dt * (cq - cp) / Geo<COORD>::face(P, A, i, j, k);
 }
 
-// Constrained transport of a curvilinear grid (src/solver_solve.c:263-306),
-// its own launch before the update: every active cell writes its three lower
+// Constrained transport of a spherical grid (src/solver_solve.c:263-306) in a
+// launch of its own before the update: with the pole ring average, whose pole
+// faces take their field from faces half a turn away, and on the mixed path
+// (see update_sph).  Every active cell writes its three lower
 // faces, the last cell along an axis also the upper boundary face, so each
 // face (with its division by the face area) is computed once
 template <int COORD, typename R>
@@ -397,17 +383,23 @@ __device__ __forceinline__ void ct_body(const Params& P, const Work<R>& wk, Pos 
   }
 }
 
-// one active cell: returns its CFL rate and |div B| of the new state.  The
+// one active cell: returns its CFL rate and |div B| of the new state.  After
+// k_ct (spherical grids, see update_sph): the
 // flux divergence, the geometric sources, the Alfven/Boris correction and
 // the CFL estimate are in R (FP32 on the mixed path); the face fields, the
 // conservative update and the pressure recovery are FP64.
-template <int COORD, typename R, bool BG, bool PSL>
+template <int COORD, typename R, bool BG, bool PSL, bool CT>
 __device__ __forceinline__ void update_body(const Params& P, const Work<R>& wk, Pos t,
                                             double& rate, double& dbmax) {
   if constexpr (COORD == 0) {
     const int ci = NGH + t.x, cj = NGH + t.y, ck = NGH + t.z;
     if (ci >= NGH + P.n[0] || cj >= NGH + P.n[1] || ck >= NGH + P.n[2]) return;
     update_cart<R, BG, PSL>(P, PointReader<R>(P, wk, ci, cj, ck), ci, cj, ck, rate, dbmax);
+    return;
+  } else if constexpr (COORD == 2 && !CT && sizeof(R) == 8) {
+    const int ci = NGH + t.x, cj = NGH + t.y, ck = NGH + t.z;
+    if (ci >= NGH + P.n[0] || cj >= NGH + P.n[1] || ck >= NGH + P.n[2]) return;
+    update_sph<BG, PSL>(P, wk, PointReader<R>(P, wk, ci, cj, ck), ci, cj, ck, rate, dbmax);
     return;
   }
   const int i = NGH + t.x, j = NGH + t.y, k = NGH + t.z;
@@ -951,12 +943,14 @@ __global__ void __launch_bounds__(256, GOP_MINB_CT) k_ct(Params P, Work<R> w) {
   if (stopped(P)) return;
   ct_body<COORD, R>(P, w, grid_pos());
 }
-template <int COORD, typename R, bool BG, bool PSL>
+// CT: k_ct has transported the face field (spherical grids, but for FP64 without
+// the pole ring average)
+template <int COORD, typename R, bool BG, bool PSL, bool CT = false>
 __global__ void __launch_bounds__(256, GOP_UPD_MINB(COORD, R)) k_update(Params P, Work<R> w) {
   pdl_enter();
   if (stopped(P)) return;
   double rate = 0.0, db = 0.0;
-  update_body<COORD, R, BG, PSL>(P, w, grid_pos(), rate, db);
+  update_body<COORD, R, BG, PSL, CT>(P, w, grid_pos(), rate, db);
   block_commit<typename std::conditional<COORD == 0 && GOP_MX_CFL64, double, R>::type>(P, rate, db);
 }
 // Ghost fill of the state just written (which 0) or of the current state.
@@ -1146,6 +1140,12 @@ void launch_dt(const Params& P, int coord, bool mixed, cudaStream_t st) {
   else launch_dt_r<double>(P, coord, st);
 }
 
+// the face field of this grid is transported by k_ct before the update
+template <typename R>
+static bool ct_apart(const Params& P) {
+  return P.coord != 0 && (P.ring || sizeof(R) == 4);
+}
+
 template <typename R, bool BG>
 static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slot, dim3 blk,
                            cudaStream_t st, bool pdl) {
@@ -1179,8 +1179,12 @@ static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slo
         if (P.ps_live) LAUNCH_PDL(pdl, (k_update<0, R, BG, true>), g, blk, st, P, w);
         else LAUNCH_PDL(pdl, (k_update<0, R, BG, false>), g, blk, st, P, w);
       } else {
-        if (P.ps_live) LAUNCH_PDL(pdl, (k_update<2, R, BG, true>), g, blk, st, P, w);
-        else LAUNCH_PDL(pdl, (k_update<2, R, BG, false>), g, blk, st, P, w);
+        if (ct_apart<R>(P) && P.ps_live) LAUNCH_PDL(pdl, (k_update<2, R, BG, true, true>), g, blk, st, P, w);
+        else if (ct_apart<R>(P)) LAUNCH_PDL(pdl, (k_update<2, R, BG, false, true>), g, blk, st, P, w);
+        else if constexpr (sizeof(R) == 8) {
+          if (P.ps_live) LAUNCH_PDL(pdl, (k_update<2, R, BG, true>), g, blk, st, P, w);
+          else LAUNCH_PDL(pdl, (k_update<2, R, BG, false>), g, blk, st, P, w);
+        }
       }
       break;
     default: break;
@@ -1238,12 +1242,12 @@ void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t
   hook(G_UPDATE, 1);
   const bool after_emf_sweep = after_sweep && !GOP_PDL_AFTER_SWEEP;
   launch_pole_emf<R>(P, w, st);  // pole ring average only
-  if (coord != 0) {  // curvilinear: the face fields in their own launch
+  if (ct_apart<R>(P)) {  // the face fields in their own launch
     const dim3 blk = tune.blk[K_UPDATE];
     LAUNCH_PDL(!after_emf_sweep, (k_ct<2, R>), grid3(P.n[0], P.n[1], P.n[2], blk), blk, st, P, w);
   }
-  if (!(coord == 0 && tune.update_sweep && launch_update_sweep<R>(sw, P, w, st)))
-    launch_slot<R>(P, coord, w, K_UPDATE, tune.blk[K_UPDATE], st, coord != 0 || !after_emf_sweep);
+  if (!(tune.update_sweep && launch_update_sweep<R>(sw, P, w, st)))
+    launch_slot<R>(P, coord, w, K_UPDATE, tune.blk[K_UPDATE], st, ct_apart<R>(P) || !after_emf_sweep);
   // the work arrays are free after the update: 2 fields of doubles of scratch
   if (P.ring) {
     launch_ring_average(P, reinterpret_cast<double*>(w.Wh), st);

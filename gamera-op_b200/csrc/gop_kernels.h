@@ -44,7 +44,7 @@ struct Tune {
   // (gop_sweep.cu) instead of the per-point kernels, where the sweeps apply
   bool flux_sweep;
   bool emf_sweep;
-  bool update_sweep;  // the Cartesian update from tiles as well
+  bool update_sweep;  // the update from tiles as well
   // order of the axes (independent) in the flux and EMF stages
   int flux_order[3];
   int emf_order[3];
@@ -67,7 +67,8 @@ template <typename R>
 bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, const int order[3],
                       cudaStream_t st);
 
-// the update of a Cartesian grid from TMA-filled tiles; false as above
+// the update from TMA-filled tiles; false as above, on small grids, and on
+// spherical ones with the pole ring average or on the mixed path
 template <typename R>
 bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st);
 

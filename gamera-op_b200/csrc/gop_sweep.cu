@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, EMF>::CTAS))
 
 // ---------------------------------------------------------------- update
 
-// The Cartesian update from tiles of 32 x 4 x 2 cells (a warp per row along
+// The update (Cartesian, or as update_sph) from tiles of 32 x 4 x 2 cells (a warp per row along
 // i): everything a cell reads -- 24 face fluxes with their upper neighbours, 12
 // edge EMFs, 6 face and 5 state values -- comes by the tile's 14 copies.  The
 // per-cell kernel waits for its 71 loads a few at a time (long-scoreboard
@@ -742,7 +742,7 @@ struct alignas(64) UpdMaps {
   uint64_t inv[2];
 };
 
-// the reader of update_cart on a slot: column c, row (jj, kk) of the tile
+// the reader of update_cart and update_sph on a slot: column c, row (jj, kk) of the tile
 template <typename R>
 struct TileReader {
   using U = UpdTile<R>;
@@ -776,7 +776,7 @@ struct TileReader {
   }
 };
 
-template <typename R, bool BG>
+template <typename R, bool BG, int COORD>
 struct UpdStage {
   using U = UpdTile<R>;
   using Maps = UpdMaps;
@@ -804,8 +804,9 @@ struct UpdStage {
     const int i = T.x0 + col, j = T.y0 + jj, k = T.z0 + kk;
     if (!(i < NGH + P.n[0] && j < NGH + P.n[1] && k < NGH + P.n[2])) return;
     double rate, divb;
-    update_cart<R, BG, false>(P, TileReader<R>{reinterpret_cast<const unsigned char*>(slot), col, jj, kk},
-                              i, j, k, rate, divb);
+    const TileReader<R> in{reinterpret_cast<const unsigned char*>(slot), col, jj, kk};
+    if constexpr (COORD == 0) update_cart<R, BG, false>(P, in, i, j, k, rate, divb);
+    else update_sph<BG, false>(P, wk, in, i, j, k, rate, divb);
     out.rate = fmax(out.rate, rate);
     out.divb = fmax(out.divb, divb);
   }
@@ -817,13 +818,13 @@ struct UpdStage {
 // 256^3 on B200, us a launch: FP64 one slot and two blocks 1256, two slots and
 // one block 1108 (per cell 1275); FP32 one slot and three or four blocks 930,
 // 1055, two slots and two blocks 854 (per cell 983).
-template <typename R, bool BG>
+template <typename R, bool BG, int COORD>
 struct UpdSweep {
   static constexpr bool EMF = false, STATE = true;
   static constexpr unsigned MASK = 1;
   static constexpr bool H0 = true, H1 = false, H2 = false;
   template <int D>
-  using Stage = UpdStage<R, BG>;
+  using Stage = UpdStage<R, BG, COORD>;
   using Maps = UpdMaps;
   static constexpr int ELEMS = Stage<0>::ELEMS, SLOT = UpdTile<R>::SLOT;
   static constexpr int CTAS = sizeof(R) == 8 ? 1 : 2, S = 2;
@@ -831,14 +832,14 @@ struct UpdSweep {
   static_assert((SMEM + 1024) * CTAS <= 228 * 1024, "update blocks per SM");
 };
 
-template <typename R, bool BG>
-__global__ void __launch_bounds__(kSweepThreads, (UpdSweep<R, BG>::CTAS))
+template <typename R, bool BG, int COORD>
+__global__ void __launch_bounds__(kSweepThreads, (UpdSweep<R, BG, COORD>::CTAS))
     k_update_sweep(Params P, Work<R> wk, const __grid_constant__ SweepMaps<UpdMaps> maps) {
   pdl_enter();
   if (stopped(P)) return;
   Gather g;
-  sweep_run<UpdSweep<R, BG>, R>(P, wk, maps, g);
-  using RC = typename std::conditional<GOP_MX_CFL64, double, R>::type;
+  sweep_run<UpdSweep<R, BG, COORD>, R>(P, wk, maps, g);
+  using RC = typename std::conditional<COORD == 0 && GOP_MX_CFL64, double, R>::type;
   block_commit<RC>(P, g.rate, g.divb);
 }
 
@@ -1013,8 +1014,11 @@ template <typename R, bool BG>
 static bool allow_smem() {
   return allow_smem<R, false, BG, 1>() && allow_smem<R, false, BG, 2>() && allow_smem<R, false, BG, 4>() &&
          allow_smem<R, false, BG, 7>() && allow_smem<R, true, BG, 7>() &&
-         cudaFuncSetAttribute(k_update_sweep<R, BG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              UpdSweep<R, BG>::SMEM) == cudaSuccess;
+         cudaFuncSetAttribute(k_update_sweep<R, BG, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              UpdSweep<R, BG, 0>::SMEM) == cudaSuccess &&
+         (sizeof(R) == 4 ||
+          cudaFuncSetAttribute(k_update_sweep<double, BG, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               UpdSweep<double, BG, 2>::SMEM) == cudaSuccess);
 }
 
 template <typename R>
@@ -1117,14 +1121,21 @@ bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, con
 // FP64 11 / 9; blast 77x45x21 17 / 15; 64^3 FP64 30.9 / 31.2, FP32 29.4 / 28.3,
 // with 3.5 to 7 tiles a block; 128^3 150 / 171, 115 / 134).
 constexpr int kUpdTiles = 6;
+template <typename R, bool BG, int COORD>
+static void launch_update_c(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
+  static const int order[3] = {0, 1, 2};
+  launch_persistent<UpdSweep<R, BG, COORD>, R>(k_update_sweep<R, BG, COORD>, sw, P, w, sw->upd, order, st);
+}
 template <typename R>
 bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
-  if (!sw || P.ps_live) return false;
+  if (!sw || P.ps_live || P.ring || (P.coord != 0 && sizeof(R) == 4)) return false;
   const int* nt = sw->upd.m[0].nt;
-  if ((long long)nt[0] * nt[1] * nt[2] < (long long)kUpdTiles * sw->sms * UpdSweep<R, false>::CTAS) return false;
-  static const int order[3] = {0, 1, 2};
-  if (P.bg) launch_persistent<UpdSweep<R, true>, R>(k_update_sweep<R, true>, sw, P, w, sw->upd, order, st);
-  else launch_persistent<UpdSweep<R, false>, R>(k_update_sweep<R, false>, sw, P, w, sw->upd, order, st);
+  if ((long long)nt[0] * nt[1] * nt[2] < (long long)kUpdTiles * sw->sms * UpdSweep<R, false, 0>::CTAS)
+    return false;
+  const bool bg = P.bg != nullptr;
+  if (P.coord == 0) bg ? launch_update_c<R, true, 0>(sw, P, w, st) : launch_update_c<R, false, 0>(sw, P, w, st);
+  else if constexpr (sizeof(R) == 8)
+    bg ? launch_update_c<R, true, 2>(sw, P, w, st) : launch_update_c<R, false, 2>(sw, P, w, st);
   return true;
 }
 #define GOP_INST(R)                                                                            \

@@ -1,5 +1,5 @@
-// The cell update of a Cartesian grid and the reductions of the CFL step and
-// of |div B|, shared by the per-cell kernel (gop_kernels.cu) and the
+// The cell update of a Cartesian or spherical grid and the reductions of the
+// CFL step and of |div B|, shared by the per-cell kernel (gop_kernels.cu) and the
 // tile-staged one (gop_sweep.cu).
 #pragma once
 
@@ -101,6 +101,22 @@ __device__ __forceinline__ float signal_speed(const Params& P, float r, float u,
   return vf + sqrt(vs * vs + vae * vae);
 }
 
+// CFL rate (signal speed over the cell's lengths) of one cell of a
+// curvilinear grid, in T arithmetic (FP32 for the mixed path's estimate)
+template <int COORD, typename T = double>
+__device__ __forceinline__ double cfl_cell(const Params& P, int i, int j, int k, double rho,
+                                           double u, double v, double w, double p, double b1,
+                                           double b2, double b3) {
+  const T x1 = (T)b1, x2 = (T)b2, x3 = (T)b3;
+  const T vc = signal_speed(P, (T)rho, (T)u, (T)v, (T)w, (T)p, x1 * x1 + x2 * x2 + x3 * x3);
+  T dk = (T)Geo<COORD>::dl(P, 2, i, j, k);
+  // the phi length of the pole rings is nk / nchunk times longer (dxk_ring,
+  // spherical_RingAverage.c:110-138; get_dt_ring, spherical_general.c:700-743)
+  if (COORD == 2 && P.ring) dk = (T)P.ringtab[2 * P.n[2] + j] * dk;
+  const T di = (T)Geo<COORD>::dl(P, 0, i, j, k), dj = (T)Geo<COORD>::dl(P, 1, i, j, k);
+  if constexpr (sizeof(T) == 8) return vc * ((dj * dk + di * dk + di * dj) / (di * dj * dk));
+  return (double)(vc / di + vc / dj + vc / dk);
+}
 // CFL rate (signal speed over the cell's lengths) of a cell of a Cartesian
 // grid, il the inverse lengths, in T arithmetic (FP32 for the mixed path's
 // estimate)
@@ -313,6 +329,203 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
     const double t0 = mn[0] + c0[0], t1 = mn[1] + c0[1], t2 = mn[2] + c0[2];
     rate = cfl_cart<RC>(P, il, rho, vv[0], vv[1], vv[2], p, t0 * t0 + t1 * t1 + t2 * t2);
   }
+  if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
+    P.scal[S_FLAGS] = 1.0;
+}
+
+// One active cell of a spherical grid without the pole ring average
+// (src/solver_solve.c:263-484, src/spherical/spherical_general.c:42-316,
+// 605-698).  The areas, edges and volumes are separable, and what the update
+// takes of them are quotients: an edge over a face in the transport, a face
+// over the volume in the divergence.  They come from tables (T_U0..T_U5), so
+// there is no division for the geometry and the cell transports its six
+// faces itself (k_ct, a launch of its own, moved the new face field to memory
+// and back to save the divisions): 192x128x128 on B200, transport and update
+// 469 -> 327 us.  FP64 only: the mixed path's FP32 roundings follow the last
+// bits of areas, volumes and face field, and it keeps the reference's products
+// and quotients in k_ct and the kernel after it.
+template <bool BG, bool PSL, class Reader>
+__device__ __forceinline__ void update_sph(const Params& P, const Work<double>& wk, const Reader& in, int i, int j,
+                                           int k, double& rate, double& dbmax) {
+  using R = double;
+  const size_t fs = P.fs;
+  const double dt = P.scal[S_DT];
+  const int nb = 1 - cur_buf(P);
+  double* Wn = P.Wbuf[nb];
+  double* Bn = P.Bbuf[nb];
+  const unsigned x = lin32(P, i, j, k), o = 8 * x, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
+  // half-step values of the geometric sources
+  const R *Wh = wk.Wh, *Mh = wk.Msh;
+  const R rh = at_byte(Wh + RHO * fs, o), v2h = at_byte(Wh + V2 * fs, o), v3h = at_byte(Wh + V3 * fs, o),
+          ph = at_byte(Wh + PR * fs, o);
+  const R m1h = at_byte(Mh, o), m2h = at_byte(Mh + fs, o), m3h = at_byte(Mh + 2 * fs, o);
+  // face over volume: radial lower and upper, h times the theta factors, h w
+  // idp in phi
+  const double a0 = tb(P, 0, T_U0, i), a1 = tb(P, 0, T_U1, i), h = tb(P, 0, T_U2, i);
+  const double s0 = tb(P, 1, T_U0, j), s1 = tb(P, 1, T_U1, j), w = tb(P, 1, T_U2, j);
+  const double idp = tb(P, 2, T_IDX, k);
+
+  // flux divergence and the geometric sources (spherical_general.c:605-681)
+  R du[6], dm[3], sh[3], sb[3];
+  const R m22 = ph + rh * v2h * v2h, m33 = ph + rh * v3h * v3h;
+  R bsqh = m1h * m1h + m2h * m2h + m3h * m3h;
+  R n22 = R(0.5) * bsqh - m2h * m2h, n33 = R(0.5) * bsqh - m3h * m3h;
+  if constexpr (BG) {  // with the B0 cross terms (spherical_general.c:634-638)
+    const double* c0 = P.bg + (size_t)BG_B0 * fs;
+    const R g1 = (R)at_byte(c0, o), g2 = (R)at_byte(c0 + fs, o), g3 = (R)at_byte(c0 + 2 * fs, o);
+    bsqh = m1h * m1h + m2h * m2h + m3h * m3h + R(2) * (m1h * g1 + m2h * g2 + m3h * g3);
+    n22 = R(0.5) * bsqh - (m2h + g2) * m2h - m2h * g2;
+    n33 = R(0.5) * bsqh - (m3h + g3) * m3h - m3h * g3;
+  }
+  const R up[3] = {a1, h * s1, h * w * idp}, lo[3] = {a0, h * s0, h * w * idp};
+  const R gr = tb(P, 0, T_U3, i), gt = tb(P, 1, T_U3, j);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+#pragma unroll
+    for (int m = 0; m < 9; m++) {
+      if (m == PS && !PSL) continue;
+      const R fu = in.flux(d, m, 1) * up[d], fl = in.flux(d, m, 0) * lo[d], v = fu - fl;
+      if (m < 6) du[m] = d == 0 ? v : du[m] + v;
+      else dm[m - 6] = d == 0 ? v : dm[m - 6] + v;
+      if (d == 0 && (m == 2 || m == 3)) sh[m - 1] = -(fl + fu) * gr;
+      if (d == 0 && (m == 7 || m == 8)) sb[m - 6] = -(fl + fu) * gr;
+      if (d == 1 && m == 3) sh[2] -= (fl + fu) * gt;
+      if (d == 1 && m == 8) sb[2] -= (fl + fu) * gt;
+    }
+  }
+  const R dr = R(0.5) * (a1 - a0), dth = h * (s1 - s0);
+  sh[0] = (m22 + m33) * dr;
+  sh[1] += dth * m33;
+  sb[0] = (n22 + n33) * dr;
+  sb[1] += dth * n33;
+  if constexpr (BG) {  // + the Lorentz force of B0 (src/solver_solve.c:312-324)
+#pragma unroll
+    for (int a = 0; a < 3; a++) dm[a] += (R)P.bg[(size_t)(BG_LOR + a) * fs + x];
+  }
+
+  // constrained transport of the six faces, FP64: curl E over the face from
+  // edge over face lengths
+  const double b0l = in.face(0, 0), b0u = in.face(0, 1);
+  const double b1l = in.face(1, 0), b1u = in.face(1, 1);
+  const double b2l = in.face(2, 0), b2u = in.face(2, 1);
+  double bl[3], bu[3];
+  {
+    const double e0 = in.emf(0, 0, 0, 0), e0j = in.emf(0, 0, 1, 0), e0k = in.emf(0, 0, 0, 1),
+                 e0jk = in.emf(0, 0, 1, 1);
+    const double e1 = in.emf(1, 0, 0, 0), e1i = in.emf(1, 1, 0, 0), e1k = in.emf(1, 0, 0, 1),
+                 e1ik = in.emf(1, 1, 0, 1);
+    const double e2 = in.emf(2, 0, 0, 0), e2i = in.emf(2, 1, 0, 0), e2j = in.emf(2, 0, 1, 0),
+                 e2ij = in.emf(2, 1, 1, 0);
+    const double r0 = tb(P, 0, T_X, i), r1 = tb(P, 0, T_X, i + 1), dr = tb(P, 0, T_DX, i);
+    const double ir0 = tb(P, 0, T_U4, i), ir1 = tb(P, 0, T_U4, i + 1), ig = tb(P, 0, T_U5, i);
+    const double drt = dr * tb(P, 1, T_IDX, j), wp = w * idp;
+    const double q0 = dr * idp * tb(P, 1, T_U4, j), q1 = dr * idp * tb(P, 1, T_U4, j + 1);
+    bl[0] = b0l - dt * ir0 * ((e2j * s1 - e2 * s0) - (e1k - e1) * wp);
+    bu[0] = b0u - dt * ir1 * ((e2ij * s1 - e2i * s0) - (e1ik - e1i) * wp);
+    bl[1] = b1l - dt * ig * ((e0k - e0) * q0 - (e2i * r1 - e2 * r0));
+    bu[1] = b1u - dt * ig * ((e0jk - e0j) * q1 - (e2ij * r1 - e2j * r0));
+    bl[2] = b2l - dt * ig * ((e1i * r1 - e1 * r0) - (e0j - e0) * drt);
+    bu[2] = b2u - dt * ig * ((e1ik * r1 - e1k * r0) - (e0jk - e0k) * drt);
+  }
+  double mo[3], mn[3], mt[3];
+  {
+    const double ma0 = tb(P, 0, T_MA, i), mb0 = tb(P, 0, T_MB, i), ma1 = tb(P, 1, T_MA, j),
+                 mb1 = tb(P, 1, T_MB, j), ma2 = tb(P, 2, T_MA, k), mb2 = tb(P, 2, T_MB, k);
+    mo[0] = b0l * ma0 + b0u * mb0;
+    mo[1] = b1l * ma1 + b1u * mb1;
+    mo[2] = b2l * ma2 + b2u * mb2;
+    mn[0] = bl[0] * ma0 + bu[0] * mb0;
+    mn[1] = bl[1] * ma1 + bu[1] * mb1;
+    mn[2] = bl[2] * ma2 + bu[2] * mb2;
+  }
+  at_byte(Bn, o) = bl[0];
+  at_byte(Bn + fs, o) = bl[1];
+  at_byte(Bn + 2 * fs, o) = bl[2];
+  if (i == NGH + P.n[0] - 1) at_byte(Bn, o + 8) = bu[0];
+  if (j == NGH + P.n[1] - 1) at_byte(Bn + fs, o + oj) = bu[1];
+  if (k == NGH + P.n[2] - 1) at_byte(Bn + 2 * fs, o + ok) = bu[2];
+  if constexpr (BG) {  // div of B + B0 (face-normal B0, src/solver_func.c:324-343)
+    const double* f0 = P.bg + (size_t)BG_FACE * fs;
+    const double* f1 = P.bg + (size_t)(BG_FACE + 4) * fs;
+    const double* f2 = P.bg + (size_t)(BG_FACE + 8) * fs;
+    const double l0 = bl[0] + at_byte(f0, o), u0 = bu[0] + at_byte(f0, o + 8);
+    const double l1 = bl[1] + at_byte(f1, o), u1 = bu[1] + at_byte(f1, o + oj);
+    const double l2 = bl[2] + at_byte(f2, o), u2 = bu[2] + at_byte(f2, o + ok);
+    dbmax = fabs((u0 * a1 - l0 * a0) + h * (u1 * s1 - l1 * s0) + h * w * idp * (u2 - l2));
+  } else {
+    dbmax = fabs((bu[0] * a1 - bl[0] * a0) + h * (bu[1] * s1 - bl[1] * s0) + h * w * idp * (bu[2] - bl[2]));
+  }
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    mt[a] = 0.5 * (mn[a] + mo[a]);
+    if constexpr (BG) {  // magtot = mags + B0
+      const double c0 = at_byte(P.bg + (size_t)(BG_B0 + a) * fs, o);
+      mt[a] += c0;
+      mn[a] += c0;  // the next step's magtot, for its CFL rate
+    }
+  }
+
+  // U^n from W^n, conservative update, cons->prim in FP64
+  // (src/solver_func.c:356-382, src/solver_solve.c:326-377)
+  const double gm1 = P.gm1;
+  const double rn = in.state(0), pn = in.state(4);
+  const double wn[3] = {in.state(1), in.state(2), in.state(3)};
+  const double U0[3] = {rn * wn[0], rn * wn[1], rn * wn[2]};
+  const double Ur = rn - dt * (double)du[0];
+  double Um[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) Um[a] = U0[a] - dt * (double)du[1 + a] + dt * (double)sh[a];
+  const double Ue = 0.5 * rn * (wn[0] * wn[0] + wn[1] * wn[1] + wn[2] * wn[2]) + pn * P.inv_gm1 -
+                    dt * (double)du[4];
+  double rho = Ur;
+  const double irho = 1.0 / Ur;
+  double vv[3] = {Um[0] * irho, Um[1] * irho, Um[2] * irho};
+  double p = (Ue - 0.5 * (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]) * rho) * gm1;
+  double pS = 0.0;
+  if constexpr (PSL) {  // entropy S = p_S / rho^(gamma-1), updated and back
+    const double ps0 = in.state(5);
+    const double S0 = (ps0 == 0.0 && rn > 0.0) ? ps0 : ps0 / pow(rn, gm1);
+    const double Us = S0 - dt * (double)du[5];
+    pS = (Us == 0.0 && Ur > 0.0) ? Us : Us * pow(Ur, gm1);
+  }
+  // positivity floors (src/solver_func.c:2117-2135)
+  if (rho < P.rho_floor) {
+    rho = P.rho_floor;
+    p = P.p_floor;
+  }
+  if (p < P.p_floor) p = P.p_floor;
+  // Alfven/Boris correction (src/solver_solve.c:385-484)
+  const R mr[3] = {(R)mt[0], (R)mt[1], (R)mt[2]};
+  const R bsq = mr[0] * mr[0] + mr[1] * mr[1] + mr[2] * mr[2];
+  R alf, perp;
+  // b^2 / (rho ca^2) and 1 / (1 + that) by one division
+  const double rc = rho * P.ca2, q = rc + bsq, inv = 1.0 / (rc * q);
+  alf = bsq * q * inv;
+  perp = rc * rc * inv;
+  const R rdt = (R)dt;
+  const R drho = -rdt * du[0];
+  const R dva = alf * drho;
+  R tv[3], wv[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    wv[a] = (R)wn[a];
+    tv[a] = alf * (-rdt * du[1 + a] + rdt * sh[a] - drho * wv[a]);
+  }
+  R bdv = mr[0] * tv[0] + mr[1] * tv[1] + mr[2] * tv[2];
+  bdv = bdv / (bsq + R(1e-10));
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const R inc = perp * ((-rdt * du[1 + a] + rdt * sh[a]) + (-rdt * dm[a] + rdt * sb[a]) +
+                          dva * wv[a] + mr[a] * bdv);
+    vv[a] = (U0[a] + (double)inc) * irho;
+  }
+  at_byte(Wn, o) = rho;
+#pragma unroll
+  for (int a = 0; a < 3; a++) at_byte(Wn + (1 + a) * fs, o) = vv[a];
+  at_byte(Wn + 4 * fs, o) = p;
+  if constexpr (PSL) at_byte(Wn + 5 * fs, o) = pS;
+  // CFL rate of the new state (magtot = mags^{n+1})
+  rate = cfl_cell<2, R>(P, i, j, k, rho, vv[0], vv[1], vv[2], p, mn[0], mn[1], mn[2]);
   if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
     P.scal[S_FLAGS] = 1.0;
 }

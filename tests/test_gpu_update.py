@@ -1,9 +1,12 @@
-"""The Cartesian update from shared-memory tiles against the per-cell kernel:
+"""The update from shared-memory tiles against the per-cell kernel:
 the same arithmetic on the same values, so the states agree to the rounding of
 a multiply-add contracted differently (1e-13 relative L1, as for the flux and
 EMF sweeps).  Grids large enough for the tiles (6 a resident block) whose last
 tiles are partly filled on every axis, in both precisions, and one with a
-background field."""
+background field; spherical shells in FP64 (the mixed path has the per-cell
+kernel only)."""
+import math
+
 import numpy as np
 import pytest
 
@@ -14,14 +17,18 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-13
 
 
-@pytest.mark.parametrize("prec", [0, 1])
-@pytest.mark.parametrize("n,bg", [((64, 96, 96), False), ((97, 99, 83), False), ((4, 250, 401), False),
-                                  ((72, 90, 81), True)])
-def test_tiled_update_equals_the_per_cell_update(n, bg, prec):
+GRIDS = [((64, 96, 96), False), ((97, 99, 83), False), ((4, 250, 401), False), ((72, 90, 81), True)]
+SHELLS = [((64, 56, 64), False), ((33, 59, 61), False), ((40, 61, 66), True)]
+CASES = [(n, bg, p, 0) for n, bg in GRIDS for p in (0, 1)] + [(n, bg, 0, 2) for n, bg in SHELLS]
+
+
+@pytest.mark.parametrize("n,bg,prec,coord", CASES)
+def test_tiled_update_equals_the_per_cell_update(n, bg, prec, coord):
     import gop
 
     rng = np.random.default_rng(sum(n) + prec)
-    xs = [gop.grid_uniform(m, 1.0, 1.0 + m / 64.0) for m in n]
+    dom = ((1.0, 2.0), (0.25 * math.pi, 0.75 * math.pi), (-0.8, 0.8))
+    xs = [gop.grid_uniform(m, *(dom[a] if coord else (1.0, 1.0 + m / 64.0))) for a, m in enumerate(n)]
     N = tuple(m + 2 * NG + 1 for m in n)
     W, B = np.zeros((6,) + N), np.zeros((3,) + N)
     W[0] = 1.0 + 0.2 * rng.random(N)
@@ -30,7 +37,7 @@ def test_tiled_update_equals_the_per_cell_update(n, bg, prec):
     B[:] = 0.5 + 0.1 * rng.standard_normal((3,) + N)
     out = []
     for sweep in (True, False):
-        inst = gop.Instance(n, *xs, bc="eeeeee", precision=prec)
+        inst = gop.Instance(n, *xs, coord=coord, bc="eeeeee", precision=prec)
         if bg:
             inst.set_background_device(gop.BG_DIPOLE, moment=0.2)
         inst.set_sweep(sweep)

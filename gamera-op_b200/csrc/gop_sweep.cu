@@ -694,10 +694,11 @@ __global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, EMF>::CTAS))
 
 // The update (Cartesian, or as update_sph) from tiles of 32 x 4 x 2 cells (a warp per row along
 // i): everything a cell reads -- 24 face fluxes with their upper neighbours, 12
-// edge EMFs, 6 face and 5 state values -- comes by the tile's 14 copies.  The
+// edge EMFs, 6 face and 5 state values, the axes' tables (beside 220 KB of slots
+// the L1 keeps little) -- comes by the tile's 16 copies.  The
 // per-cell kernel waits for its 71 loads a few at a time (long-scoreboard
 // stalls 5.6 per instruction, 4.5 TB/s at 256^3 FP64).
-template <typename R>
+template <typename R, int COORD>
 struct UpdTile {
   // the faces along each axis, the edges along each axis
   __host__ __device__ static constexpr Box F(int d) {
@@ -728,9 +729,24 @@ struct UpdTile {
     return o;
   }
   __host__ __device__ static constexpr int w() { return b(3); }
-  static constexpr int SLOT = w() + up(W.elems() * 8);
+  // the axes' tables at the tile's columns, rows and planes (spherical: and
+  // the next ones): 1 / dx and the centring weights of a Cartesian grid, all
+  // but the reconstruction's of a spherical one (two groups of rows)
+  static constexpr int T0 = COORD == 0 ? T_IDX : T_X, TN = T_MB + 1 - T0;
+  static constexpr int TG = COORD == 0 ? 0 : NTAB - T_G0;
+  __host__ __device__ static constexpr int tw(int d) {
+    return COORD == 0 ? (d == 0 ? 32 : (d == 1 ? 4 : 2)) : (d == 0 ? 36 : (d == 1 ? 6 : 2));
+  }
+  __host__ __device__ static constexpr int t(int d) {
+    int o = w() + up(W.elems() * 8);
+    for (int a = 0; a < d; a++) o += up(tw(a) * TN * 8) + up(tw(a) * TG * 8);
+    return o;
+  }
+  __host__ __device__ static constexpr int tg(int d) { return t(d) + up(tw(d) * TN * 8); }
+  static constexpr int SLOT = t(3);
   static constexpr int BYTES = 8 * (F(0).elems() + F(1).elems() + F(2).elems()) * (RS + 1) +
-                               (E(0).elems() + E(1).elems() + E(2).elems()) * RS + W.elems() * 8;
+                               (E(0).elems() + E(1).elems() + E(2).elems()) * RS + W.elems() * 8 +
+                               (tw(0) + tw(1) + tw(2)) * (TN + TG) * 8;
 };
 
 struct alignas(64) UpdMaps {
@@ -738,14 +754,15 @@ struct alignas(64) UpdMaps {
   CUtensorMap e[3];        // EMFs
   CUtensorMap b[3][2];     // step-start face field, of either parity
   CUtensorMap w[2];        // step-start state
+  CUtensorMap t[3], g2[3]; // tables: T0.., T_G0..
   int nt[3];
   uint64_t inv[2];
 };
 
 // the reader of update_cart and update_sph on a slot: column c, row (jj, kk) of the tile
-template <typename R>
+template <typename R, int COORD>
 struct TileReader {
-  using U = UpdTile<R>;
+  using U = UpdTile<R, COORD>;
   const unsigned char* s;
   int c, jj, kk;
   template <typename T>
@@ -774,11 +791,16 @@ struct TileReader {
   __device__ __forceinline__ double state(int m) const {
     return at<double>(U::w(), ((m * 2 + kk) * 4 + jj) * 32 + c);
   }
+  __device__ __forceinline__ double tab(int a, int t, int up = 0) const {
+    constexpr int o[3] = {U::t(0), U::t(1), U::t(2)}, g[3] = {U::tg(0), U::tg(1), U::tg(2)};
+    const int x = (a == 0 ? c : (a == 1 ? jj : kk)) + up;
+    return t <= T_MB ? at<double>(o[a], (t - U::T0) * U::tw(a) + x) : at<double>(g[a], (t - T_G0) * U::tw(a) + x);
+  }
 };
 
 template <typename R, bool BG, int COORD>
 struct UpdStage {
-  using U = UpdTile<R>;
+  using U = UpdTile<R, COORD>;
   using Maps = UpdMaps;
   static constexpr int ELEMS = U::SLOT / (int)sizeof(R), ROWS = kWarps, BYTES = U::BYTES;
   __device__ static Tile place(const Params& P, const Maps& m, int r) {
@@ -795,6 +817,9 @@ struct UpdStage {
       tma_load_4d(s + U::g(d), &m.g[d], bar, x, y, z, 9 * d + 6);
       tma_load_4d(s + U::e(d), &m.e[d], bar, x, y, z, d);
       tma_load_4d(s + U::b(d), &m.b[d][par], bar, x, y, z, d);
+      const int at = d == 0 ? x : (d == 1 ? y : z);
+      tma_load_4d(s + U::t(d), &m.t[d], bar, at, U::T0, d, 0);
+      if constexpr (COORD != 0) tma_load_4d(s + U::tg(d), &m.g2[d], bar, at, T_G0, d, 0);
     }
     tma_load_4d(s + U::w(), &m.w[par], bar, x, y, z, 0);
   }
@@ -804,7 +829,7 @@ struct UpdStage {
     const int i = T.x0 + col, j = T.y0 + jj, k = T.z0 + kk;
     if (!(i < NGH + P.n[0] && j < NGH + P.n[1] && k < NGH + P.n[2])) return;
     double rate, divb;
-    const TileReader<R> in{reinterpret_cast<const unsigned char*>(slot), col, jj, kk};
+    const TileReader<R, COORD> in{reinterpret_cast<const unsigned char*>(slot), col, jj, kk};
     if constexpr (COORD == 0) update_cart<R, BG, false>(P, in, i, j, k, rate, divb);
     else update_sph<BG, false>(P, wk, in, i, j, k, rate, divb);
     out.rate = fmax(out.rate, rate);
@@ -817,7 +842,8 @@ struct UpdStage {
 // copies run ahead: with one slot a block loads and computes in turn.  Blast
 // 256^3 on B200, us a launch: FP64 one slot and two blocks 1256, two slots and
 // one block 1108 (per cell 1275); FP32 one slot and three or four blocks 930,
-// 1055, two slots and two blocks 854 (per cell 983).
+// 1055, two slots and two blocks 886 (per cell 983).  The tables in the slot
+// instead of the little L1 beside it: 1089 and 752.
 template <typename R, bool BG, int COORD>
 struct UpdSweep {
   static constexpr bool EMF = false, STATE = true;
@@ -826,7 +852,7 @@ struct UpdSweep {
   template <int D>
   using Stage = UpdStage<R, BG, COORD>;
   using Maps = UpdMaps;
-  static constexpr int ELEMS = Stage<0>::ELEMS, SLOT = UpdTile<R>::SLOT;
+  static constexpr int ELEMS = Stage<0>::ELEMS, SLOT = UpdTile<R, COORD>::SLOT;
   static constexpr int CTAS = sizeof(R) == 8 ? 1 : 2, S = 2;
   static constexpr int SMEM = S * SLOT + S * (2 * 8 + (int)sizeof(Tile)) + 128;
   static_assert((SMEM + 1024) * CTAS <= 228 * 1024, "update blocks per SM");
@@ -978,9 +1004,9 @@ static bool make_emf_maps(EmfMaps& m, const Params& P, const Work<R>& w) {
   return ok;
 }
 
-template <typename R>
+template <typename R, int COORD>
 static bool make_upd_maps(UpdMaps& m, const Params& P, const Work<R>& w) {
-  using U = UpdTile<R>;
+  using U = UpdTile<R, COORD>;
   bool ok = true;
   for (int d = 0; d < 3 && ok; d++) {
     Box f = U::F(d), g = U::F(d);
@@ -988,6 +1014,10 @@ static bool make_upd_maps(UpdMaps& m, const Params& P, const Work<R>& w) {
     g.f = 3;
     ok = field_map<R>(&m.f[d], w.F, 27, P, f) && field_map<R>(&m.g[d], w.F, 27, P, g) &&
          field_map<R>(&m.e[d], w.E, 3, P, U::E(d));
+    const cuuint64_t tm = (cuuint64_t)P.tmax, td[4] = {tm, (cuuint64_t)NTAB, 3, 1};
+    const cuuint64_t ts[3] = {tm * 8, tm * NTAB * 8, tm * NTAB * 3 * 8};
+    ok = ok && encode<double>(&m.t[d], P.tab, td, ts, Box{U::tw(d), U::TN, 1, 1});
+    if constexpr (COORD != 0) ok = ok && encode<double>(&m.g2[d], P.tab, td, ts, Box{U::tw(d), U::TG, 1, 1});
     for (int b = 0; b < 2 && ok; b++) ok = field_map<double>(&m.b[d][b], P.Bbuf[b], 3, P, U::F(d));
   }
   for (int b = 0; b < 2 && ok; b++) ok = field_map<double>(&m.w[b], P.Wbuf[b], 6, P, U::W);
@@ -1031,7 +1061,8 @@ SweepSet* sweep_create(const Params& P, const Work<R>& w) {
   ok = ok && make_flux_maps<R, 0>(s->flux.m[0], P, w) && make_flux_maps<R, 1>(s->flux.m[1], P, w) &&
        make_flux_maps<R, 2>(s->flux.m[2], P, w) && make_emf_maps<R, 0>(s->emf.m[0], P, w) &&
        make_emf_maps<R, 1>(s->emf.m[1], P, w) && make_emf_maps<R, 2>(s->emf.m[2], P, w);
-  ok = ok && make_upd_maps<R>(s->upd.m[0], P, w) && allow_smem<R, false>() && allow_smem<R, true>();
+  ok = ok && (P.coord == 0 ? make_upd_maps<R, 0>(s->upd.m[0], P, w) : make_upd_maps<R, 2>(s->upd.m[0], P, w)) &&
+       allow_smem<R, false>() && allow_smem<R, true>();
   if (!ok) {
     cudaGetLastError();
     delete s;

@@ -101,6 +101,10 @@ __device__ __forceinline__ float signal_speed(const Params& P, float r, float u,
   return vf + sqrt(vs * vs + vae * vae);
 }
 
+// vc (1/di + 1/dj + 1/dk)
+__device__ __forceinline__ double cfl_sph(double vc, double di, double dj, double dk) {
+  return vc * ((dj * dk + di * dk + di * dj) / (di * dj * dk));
+}
 // CFL rate (signal speed over the cell's lengths) of one cell of a
 // curvilinear grid, in T arithmetic (FP32 for the mixed path's estimate)
 template <int COORD, typename T = double>
@@ -114,7 +118,7 @@ __device__ __forceinline__ double cfl_cell(const Params& P, int i, int j, int k,
   // spherical_RingAverage.c:110-138; get_dt_ring, spherical_general.c:700-743)
   if (COORD == 2 && P.ring) dk = (T)P.ringtab[2 * P.n[2] + j] * dk;
   const T di = (T)Geo<COORD>::dl(P, 0, i, j, k), dj = (T)Geo<COORD>::dl(P, 1, i, j, k);
-  if constexpr (sizeof(T) == 8) return vc * ((dj * dk + di * dk + di * dj) / (di * dj * dk));
+  if constexpr (sizeof(T) == 8) return cfl_sph(vc, di, dj, dk);
   return (double)(vc / di + vc / dj + vc / dk);
 }
 // CFL rate (signal speed over the cell's lengths) of a cell of a Cartesian
@@ -137,12 +141,13 @@ struct PointReader {
   // byte offsets of the cell and of its upper neighbours along j and k: o
   // in the FP64 state, r in the stage arrays
   unsigned o, oj, ok, r, rj, rk;
+  int x[3];
   static constexpr unsigned RS = sizeof(R);
   __device__ __forceinline__ PointReader(const Params& p, const Work<R>& w, int i, int j, int k)
-      : P(p), wk(w), W(p.Wbuf[cur_buf(p)]), B(p.Bbuf[cur_buf(p)]) {
-    const unsigned x = lin32(P, i, j, k);
-    o = 8 * x, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
-    r = RS * x, rj = RS * (unsigned)P.sj, rk = RS * (unsigned)P.sk;
+      : P(p), wk(w), W(p.Wbuf[cur_buf(p)]), B(p.Bbuf[cur_buf(p)]), x{i, j, k} {
+    const unsigned c = lin32(P, i, j, k);
+    o = 8 * c, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
+    r = RS * c, rj = RS * (unsigned)P.sj, rk = RS * (unsigned)P.sk;
   }
   // flux m at the lower (u = 0) or upper face along axis d
   __device__ __forceinline__ R flux(int d, int m, int u) const {
@@ -157,6 +162,8 @@ struct PointReader {
     return at_byte(B + a * P.fs, u ? o + (a == 0 ? 8u : (a == 1 ? oj : ok)) : o);
   }
   __device__ __forceinline__ double state(int m) const { return at_byte(W + m * P.fs, o); }
+  // table t of axis a at the cell, or at the next one
+  __device__ __forceinline__ double tab(int a, int t, int up = 0) const { return tb(P, a, t, x[a] + up); }
 };
 
 // One active cell of a Cartesian grid (src/solver_solve.c:263-484 with the
@@ -182,7 +189,7 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
   double* Wn = P.Wbuf[nb];
   double* Bn = P.Bbuf[nb];
   const unsigned x = lin32(P, i, j, k), o = 8 * x, oj = 8 * (unsigned)P.sj, ok = 8 * (unsigned)P.sk;
-  const double il[3] = {tb(P, 0, T_IDX, i), tb(P, 1, T_IDX, j), tb(P, 2, T_IDX, k)};
+  const double il[3] = {in.tab(0, T_IDX), in.tab(1, T_IDX), in.tab(2, T_IDX)};
 
   // flux divergence: 5 hydro (6 with the entropy channel) and 3 stress
   // components, the difference of the two faces over the cell's length (every
@@ -225,9 +232,9 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
   bu[1] = b1u - dt * ((e0jk - e0j) * il[2] - (e2ij - e2j) * il[0]);
   bu[2] = b2u - dt * ((e1ik - e1k) * il[0] - (e0jk - e0k) * il[1]);
   // mags^n for the time-centred field
-  mo[0] = b0l * tb(P, 0, T_MA, i) + b0u * tb(P, 0, T_MB, i);
-  mo[1] = b1l * tb(P, 1, T_MA, j) + b1u * tb(P, 1, T_MB, j);
-  mo[2] = b2l * tb(P, 2, T_MA, k) + b2u * tb(P, 2, T_MB, k);
+  mo[0] = b0l * in.tab(0, T_MA) + b0u * in.tab(0, T_MB);
+  mo[1] = b1l * in.tab(1, T_MA) + b1u * in.tab(1, T_MB);
+  mo[2] = b2l * in.tab(2, T_MA) + b2u * in.tab(2, T_MB);
   at_byte(Bn, o) = bl[0];
   at_byte(Bn + fs, o) = bl[1];
   at_byte(Bn + 2 * fs, o) = bl[2];
@@ -251,9 +258,9 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
     for (int a = 0; a < 3; a++) c0[a] = at_byte(P.bg + (size_t)(BG_B0 + a) * fs, o);
   }
   double mn[3], mt[3];
-  mn[0] = bl[0] * tb(P, 0, T_MA, i) + bu[0] * tb(P, 0, T_MB, i);
-  mn[1] = bl[1] * tb(P, 1, T_MA, j) + bu[1] * tb(P, 1, T_MB, j);
-  mn[2] = bl[2] * tb(P, 2, T_MA, k) + bu[2] * tb(P, 2, T_MB, k);
+  mn[0] = bl[0] * in.tab(0, T_MA) + bu[0] * in.tab(0, T_MB);
+  mn[1] = bl[1] * in.tab(1, T_MA) + bu[1] * in.tab(1, T_MB);
+  mn[2] = bl[2] * in.tab(2, T_MA) + bu[2] * in.tab(2, T_MB);
 #pragma unroll
   for (int a = 0; a < 3; a++) mt[a] = BG ? 0.5 * (mn[a] + mo[a]) + c0[a] : 0.5 * (mn[a] + mo[a]);
 
@@ -361,9 +368,9 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
   const R m1h = at_byte(Mh, o), m2h = at_byte(Mh + fs, o), m3h = at_byte(Mh + 2 * fs, o);
   // face over volume: radial lower and upper, h times the theta factors, h w
   // idp in phi
-  const double a0 = tb(P, 0, T_U0, i), a1 = tb(P, 0, T_U1, i), h = tb(P, 0, T_U2, i);
-  const double s0 = tb(P, 1, T_U0, j), s1 = tb(P, 1, T_U1, j), w = tb(P, 1, T_U2, j);
-  const double idp = tb(P, 2, T_IDX, k);
+  const double a0 = in.tab(0, T_U0), a1 = in.tab(0, T_U1), h = in.tab(0, T_U2);
+  const double s0 = in.tab(1, T_U0), s1 = in.tab(1, T_U1), w = in.tab(1, T_U2);
+  const double idp = in.tab(2, T_IDX);
 
   // flux divergence and the geometric sources (spherical_general.c:605-681)
   R du[6], dm[3], sh[3], sb[3];
@@ -378,7 +385,7 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
     n33 = R(0.5) * bsqh - (m3h + g3) * m3h - m3h * g3;
   }
   const R up[3] = {a1, h * s1, h * w * idp}, lo[3] = {a0, h * s0, h * w * idp};
-  const R gr = tb(P, 0, T_U3, i), gt = tb(P, 1, T_U3, j);
+  const R gr = in.tab(0, T_U3), gt = in.tab(1, T_U3);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
 #pragma unroll
@@ -416,10 +423,10 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
                  e1ik = in.emf(1, 1, 0, 1);
     const double e2 = in.emf(2, 0, 0, 0), e2i = in.emf(2, 1, 0, 0), e2j = in.emf(2, 0, 1, 0),
                  e2ij = in.emf(2, 1, 1, 0);
-    const double r0 = tb(P, 0, T_X, i), r1 = tb(P, 0, T_X, i + 1), dr = tb(P, 0, T_DX, i);
-    const double ir0 = tb(P, 0, T_U4, i), ir1 = tb(P, 0, T_U4, i + 1), ig = tb(P, 0, T_U5, i);
-    const double drt = dr * tb(P, 1, T_IDX, j), wp = w * idp;
-    const double q0 = dr * idp * tb(P, 1, T_U4, j), q1 = dr * idp * tb(P, 1, T_U4, j + 1);
+    const double r0 = in.tab(0, T_X), r1 = in.tab(0, T_X, 1), dr = in.tab(0, T_DX);
+    const double ir0 = in.tab(0, T_U4), ir1 = in.tab(0, T_U4, 1), ig = in.tab(0, T_U5);
+    const double drt = dr * in.tab(1, T_IDX), wp = w * idp;
+    const double q0 = dr * idp * in.tab(1, T_U4), q1 = dr * idp * in.tab(1, T_U4, 1);
     bl[0] = b0l - dt * ir0 * ((e2j * s1 - e2 * s0) - (e1k - e1) * wp);
     bu[0] = b0u - dt * ir1 * ((e2ij * s1 - e2i * s0) - (e1ik - e1i) * wp);
     bl[1] = b1l - dt * ig * ((e0k - e0) * q0 - (e2i * r1 - e2 * r0));
@@ -429,8 +436,8 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
   }
   double mo[3], mn[3], mt[3];
   {
-    const double ma0 = tb(P, 0, T_MA, i), mb0 = tb(P, 0, T_MB, i), ma1 = tb(P, 1, T_MA, j),
-                 mb1 = tb(P, 1, T_MB, j), ma2 = tb(P, 2, T_MA, k), mb2 = tb(P, 2, T_MB, k);
+    const double ma0 = in.tab(0, T_MA), mb0 = in.tab(0, T_MB), ma1 = in.tab(1, T_MA),
+                 mb1 = in.tab(1, T_MB), ma2 = in.tab(2, T_MA), mb2 = in.tab(2, T_MB);
     mo[0] = b0l * ma0 + b0u * mb0;
     mo[1] = b1l * ma1 + b1u * mb1;
     mo[2] = b2l * ma2 + b2u * mb2;
@@ -525,7 +532,10 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
   at_byte(Wn + 4 * fs, o) = p;
   if constexpr (PSL) at_byte(Wn + 5 * fs, o) = pS;
   // CFL rate of the new state (magtot = mags^{n+1})
-  rate = cfl_cell<2, R>(P, i, j, k, rho, vv[0], vv[1], vv[2], p, mn[0], mn[1], mn[2]);
+  // (lengths dr, r_c dtheta, r_c sin(theta_c) dphi, as cfl_cell)
+  const double vc = signal_speed(P, rho, vv[0], vv[1], vv[2], p, mn[0] * mn[0] + mn[1] * mn[1] + mn[2] * mn[2]);
+  const double rctr = in.tab(0, T_G3);
+  rate = cfl_sph(vc, in.tab(0, T_DX), rctr * in.tab(1, T_DX), rctr * in.tab(1, T_G2) * in.tab(2, T_DX));
   if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
     P.scal[S_FLAGS] = 1.0;
 }

@@ -1147,11 +1147,15 @@ bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, con
   else launch_axes<R, true, false>(sw, P, w, sw->emf, order, st);
   return true;
 }
-// Where a block has too few tiles to fill its ring before it ends, the per-cell
-// kernel is as fast or faster (B200, us, tiles / per cell: Orszag-Tang 64x64x4
-// FP64 11 / 9; blast 77x45x21 17 / 15; 64^3 FP64 30.9 / 31.2, FP32 29.4 / 28.3,
-// with 3.5 to 7 tiles a block; 128^3 150 / 171, 115 / 134).
-constexpr int kUpdTiles = 6;
+// Tiles a block needs: with fewer its ring is hardly filled before it ends and
+// the per-cell kernel is as fast or faster (B200, us, tiles / per cell.  FP64, by
+// tiles a block: 2.7 (blast 77x45x21) 16.9 / 15.2, 3.2 23.0 / 20.7, 6.9 (64^3) 27.5
+// / 31, 55 (128^3) 144 / 171; FP32: 1.7 15.0 / 15.2, 3.5 (64^3) 27.2 / 29.1,
+// (Orszag-Tang 256x256x4) 23.7 / 26.7, 28 105 / 134).
+template <typename R>
+constexpr int upd_tiles() {
+  return sizeof(R) == 8 ? 6 : 3;
+}
 template <typename R, bool BG, int COORD>
 static void launch_update_c(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
   static const int order[3] = {0, 1, 2};
@@ -1161,7 +1165,7 @@ template <typename R>
 bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
   if (!sw || P.ps_live || P.ring || (P.coord != 0 && sizeof(R) == 4)) return false;
   const int* nt = sw->upd.m[0].nt;
-  if ((long long)nt[0] * nt[1] * nt[2] < (long long)kUpdTiles * sw->sms * UpdSweep<R, false, 0>::CTAS)
+  if ((long long)nt[0] * nt[1] * nt[2] < (long long)upd_tiles<R>() * sw->sms * UpdSweep<R, false, 0>::CTAS)
     return false;
   const bool bg = P.bg != nullptr;
   if (P.coord == 0) bg ? launch_update_c<R, true, 0>(sw, P, w, st) : launch_update_c<R, false, 0>(sw, P, w, st);

@@ -1212,6 +1212,7 @@ int gop_autotune(gop_instance* h, int reps, int* chosen) {
   };
   for (int slot = 0; slot < NTUNE; slot++) {
     float best = 1e30f;
+    if (slot >= K_C2C0 && slot <= K_C2C2) continue;  // one launch of a fixed shape: candidate 0
     for (int c = 0; c < ncand; c++) {
       if (cand[c].x * cand[c].y * cand[c].z > 256) continue;
       float ms = 0.f;

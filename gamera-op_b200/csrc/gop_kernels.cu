@@ -918,11 +918,26 @@ __global__ void __launch_bounds__(256, GOP_MINB(AB2, R)) k_ab2(Params P, Work<R>
   if (stopped(P)) return;
   ab2_body<R, PSL>(P, w, grid_pos());
 }
-template <typename R, int D>
-__global__ void __launch_bounds__(256, GOP_MINB(C2C, R)) k_c2c(Params P, Work<R> w) {
+// The ghost layers of the axes that are not periodic, for the edges of all
+// three directions in one launch: threads first[D] .. first[D + 1] - 1 take the
+// edges along D.  (Three launches of a few thousand points each took 3 to 5 us
+// a step apiece: shell 96x64x48 on B200, stage 13.9 -> 8.6 us.)
+struct C2cRange {
+  unsigned first[4];
+};
+template <typename R>
+__global__ void __launch_bounds__(256, GOP_MINB(C2C, R)) k_c2c(Params P, Work<R> w, C2cRange G) {
   pdl_enter();
   if (stopped(P)) return;
-  c2c_body<R, D>(P, w, grid_pos());
+  const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
+  // r = x + ex (y + ey z) over the points of a direction
+  auto at = [](unsigned r, unsigned ex, unsigned ey) {
+    const unsigned q = r / ex;
+    return Pos{(int)(r - q * ex), (int)(q % ey), (int)(q / ey)};
+  };
+  if (g < G.first[1]) c2c_body<R, 0>(P, w, at(g, P.n[0], P.n[1] + 1));
+  else if (g < G.first[2]) c2c_body<R, 1>(P, w, at(g - G.first[1], 2 * NGH, P.n[1]));
+  else if (g < G.first[3]) c2c_body<R, 2>(P, w, at(g - G.first[2], P.n[0] + 1, 2 * NGH));
 }
 // BG: with the background-field terms (Params::bg set)
 template <typename R, int D, bool BG>
@@ -1079,9 +1094,7 @@ Tune::Tune() {
   // block's longer transverse side so neighbouring rows share L1 lines
   for (int t = 0; t < NTUNE; t++) blk[t] = dim3(32, 4, 2);
   blk[K_EMF1] = blk[K_FLUX1] = dim3(32, 8, 1);
-  blk[K_C2C2] = blk[K_EMF2] = blk[K_FLUX2] = dim3(32, 1, 8);
-  // the first edge sweep of edges along j covers only the 8 ghost layers of i
-  blk[K_C2C1] = dim3(8, 32, 1);
+  blk[K_EMF2] = blk[K_FLUX2] = dim3(32, 1, 8);
   for (int d = 0; d < 3; d++) {
     flux_order[d] = emf_order[d] = d;
   }
@@ -1091,21 +1104,13 @@ Tune::Tune() {
 dim3 launch_space(const Params& P, int slot) {
   if (slot == K_AB2) return dim3(P.N[0], P.N[1], P.N[2]);
   if (slot == K_UPDATE) return dim3(P.n[0], P.n[1], P.n[2]);
-  const int stage = (slot - K_C2C0) / 3, D = (slot - K_C2C0) % 3;
-  const int p = (D + 1) % 3, q = (D + 2) % 3;
-  int cnt[3];
-  if (stage == 0) {  // ghost layers of q only (see c2c_body)
-    cnt[D] = P.n[D];
-    cnt[p] = P.n[p] + 1;
-    cnt[q] = 2 * NGH;
-  } else if (stage == 1) {
-    cnt[D] = P.n[D];
-    cnt[p] = P.n[p] + 1;
-    cnt[q] = P.n[q] + 1;
+  const bool emf = slot < K_FLUX0;
+  const int D = emf ? slot - K_EMF0 : slot - K_FLUX0;
+  int cnt[3] = {P.n[0], P.n[1], P.n[2]};
+  if (emf) {  // D cells, faces of the other two axes
+    cnt[(D + 1) % 3] += 1;
+    cnt[(D + 2) % 3] += 1;
   } else {
-    cnt[0] = P.n[0];
-    cnt[1] = P.n[1];
-    cnt[2] = P.n[2];
     cnt[D] += 1;
   }
   return dim3(cnt[0], cnt[1], cnt[2]);
@@ -1156,9 +1161,6 @@ static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slo
       if (P.ps_live) LAUNCH((k_ab2<R, true>), g, blk, st, P, w);
       else LAUNCH((k_ab2<R, false>), g, blk, st, P, w);
       break;
-    case K_C2C0: LAUNCH_PDL(pdl, (k_c2c<R, 0>), g, blk, st, P, w); break;
-    case K_C2C1: LAUNCH_PDL(pdl, (k_c2c<R, 1>), g, blk, st, P, w); break;
-    case K_C2C2: LAUNCH_PDL(pdl, (k_c2c<R, 2>), g, blk, st, P, w); break;
     case K_EMF0: LAUNCH_PDL(pdl, (k_emf<R, 0, BG>), g, blk, st, P, w); break;
     case K_EMF1: LAUNCH_PDL(pdl, (k_emf<R, 1, BG>), g, blk, st, P, w); break;
     case K_EMF2: LAUNCH_PDL(pdl, (k_emf<R, 2, BG>), g, blk, st, P, w); break;
@@ -1222,10 +1224,18 @@ void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t
     }
   hook(G_FLUX, 0);
   hook(G_C2C, 1);
-  for (int d = 0; d < 3; d++) {
-    if (P.per[(d + 2) % 3]) continue;  // the flux stage has written those ghost layers
-    launch_slot<R>(P, coord, w, K_C2C0 + d, tune.blk[K_C2C0 + d], st, !after_sweep || GOP_PDL_AFTER_SWEEP);
-    after_sweep = false;
+  {
+    C2cRange G;
+    G.first[0] = 0;
+    const unsigned n0 = P.n[0], n1 = P.n[1], n2 = P.n[2];
+    const unsigned pts[3] = {n0 * (n1 + 1) * 2 * NGH, 2 * NGH * n1 * (n2 + 1), (n0 + 1) * 2 * NGH * n2};
+    for (int d = 0; d < 3; d++)  // (where q is periodic the flux stage has written the layers)
+      G.first[d + 1] = G.first[d] + (P.per[(d + 2) % 3] ? 0u : pts[d]);
+    if (G.first[3]) {
+      LAUNCH_PDL(!after_sweep || GOP_PDL_AFTER_SWEEP, k_c2c<R>, dim3((G.first[3] + 255) / 256), dim3(256), st,
+                 P, w, G);
+      after_sweep = false;
+    }
   }
   hook(G_C2C, 0);
   hook(G_EMF, 1);

@@ -156,7 +156,8 @@ int gop_get_stats(gop_instance *h, gop_stats *out);
  * they are independent, so no result changes), timing two whole steps per
  * rotation with the state restored after each.  reps: timed launches per
  * candidate (0 = 3); chosen (optional, 11 ints) receives the picked
- * candidate index per launch. */
+ * candidate index per launch (0 for the three centre-to-edge entries, which
+ * are one launch of a fixed shape). */
 #define GOP_NTUNE 11
 #define GOP_TUNE_SWEEP 14 /* chosen[] value of a flux or EMF launch: the tile-staged sweep kernel */
 int gop_autotune(gop_instance *h, int reps, int *chosen);

@@ -38,6 +38,8 @@ METRIC = "Mcell-updates/s vs plain FP64 GPU at fixed L1 err; %HBM peak; p50/p99 
 UNIT = "Mcell-updates/s"
 BYTES_PER_CELL_UPDATE = 216  # algorithmic bytes of one cell-update (FP64)
 REF_BUDGET_S = 120  # seconds of timed steps the reference arm may spend
+# directions a group covers per step: the bytes and times below are of one
+# direction (the three go out in one launch or three, by stage and grid)
 GROUP_LAUNCHES = {"ab2": 1, "c2c": 3, "emf": 3, "flux": 3, "update": 1}
 # thread-block shapes the library's autotuner chooses from (gop_autotune)
 BLOCK_CANDIDATES = ["32x4x2", "32x8x1", "32x1x8", "32x2x4", "64x2x2", "64x4x1", "64x1x4",
@@ -54,7 +56,7 @@ def peaks():
 
 
 def algorithmic_bytes(group, n, mixed=False, ps_live=False):
-    """Compulsory DRAM bytes of one launch of a kernel group (each input
+    """Compulsory DRAM bytes of one direction of a kernel group (each input
     array element read once, each output written once).  Work arrays are
     FP32 on the mixed path (4 bytes), the state and its AB2 history FP64.
     ps_live False: the entropy channel p_S is identically zero (every

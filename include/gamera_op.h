@@ -166,8 +166,8 @@ int gop_get_launch_order(gop_instance *h, int *flux_order, int *emf_order);
 
 /* Kernel choice for the face fluxes and edge EMFs: on (the default) runs
  * the tile-staged sweep kernels (shared-memory tiles filled by the Tensor
- * Memory Accelerator, persistent blocks) wherever they apply, off the
- * per-point kernels; both give the same results.  With the entropy channel
+ * Memory Accelerator, persistent blocks) wherever they apply, and the update
+ * in the same form on grids large enough, off the per-point kernels; both give the same results.  With the entropy channel
  * live the per-face flux kernels always run.  GOP_ENODEV if the sweep
  * kernels could not be set up for this instance. */
 int gop_set_sweep(gop_instance *h, int on);
@@ -175,7 +175,8 @@ int gop_set_sweep(gop_instance *h, int on);
 /* Diagnostics: time every kernel group of every step with CUDA events on
  * the instance's stream (off by default; switching resets the totals).
  * Groups: 0 begin, 1 ab2, 2 centre-to-edge, 3 edge EMF, 4 face flux,
- * 5 update, 6 ghost fill, 7 end.  ms[g] and count[g] (GOP_NGROUP entries)
+ * 5 update, 6 ghost fill (its last block ends the step and opens the next),
+ * 7 end; 0 and 7 hold no launch.  ms[g] and count[g] (GOP_NGROUP entries)
  * are the summed milliseconds and the number of timed occurrences. */
 #define GOP_NGROUP 8
 int gop_set_profiling(gop_instance *h, int on);

@@ -6,9 +6,11 @@
 // synchronisation:
 //
 //   ab2       W_h, mags, mags_h, B_h over the ghost-extended grid
-//   c2c       centre-to-edge velocity, first sweep (3 edge directions)
+//   flux      PDM reconstruction + Rusanov flux + Maxwell stress per face; the
+//             first centre-to-edge sweep where it has the face's states
+//   c2c       centre-to-edge velocity, first sweep, in the ghost layers of
+//             axes that are not periodic (3 edge directions)
 //   emf       centre-to-edge second sweep, face-B reconstruction, edge EMF
-//   flux      PDM reconstruction + Rusanov flux + Maxwell stress per face
 //   update    divergence, sources, constrained transport, cons->prim,
 //             floors, Alfven/Boris correction, next CFL dt, max|div B|
 //   ghost     periodic wrap and boundary fills of the new state; its last

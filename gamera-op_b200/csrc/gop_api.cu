@@ -446,6 +446,7 @@ struct gop_instance {
   cudaStream_t st = nullptr;   // where its work goes (own, or the caller's)
   cudaStream_t copy = nullptr; // host copies of gop_upload and gop_download (made at first use)
   cudaEvent_t field_ev[6] = {};  // the last use of each staging slot
+  cudaEvent_t order_ev = nullptr;  // what st held when an upload began
   double* state = nullptr;   // 2 x (6 + 3) fields
   void* work = nullptr;      // WORK_FIELDS x R
   double* tab = nullptr;
@@ -489,10 +490,13 @@ static int copy_stream(gop_instance* h) {
   if (h->copy) return GOP_OK;
   for (cudaEvent_t& e : h->field_ev)
     if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!h->order_ev) CK(cudaEventCreateWithFlags(&h->order_ev, cudaEventDisableTiming));
   CK(cudaStreamCreateWithFlags(&h->copy, cudaStreamNonBlocking));
   return GOP_OK;
 }
-// nf <= 6 fields from the host; ends with the kernels enqueued on h->st
+// nf <= 6 fields from the host; ends with the kernels enqueued on h->st.  The
+// copies follow what h->st holds already, on either stream: the caller's own
+// work on it may be what fills the array.
 static int upload_fields(gop_instance* h, int nf, const double* host, double* dev) {
   const Params& P = h->P;
   const size_t ref = (size_t)P.N[0] * P.N[1] * P.N[2], bytes = ref * sizeof(double);
@@ -502,6 +506,8 @@ static int upload_fields(gop_instance* h, int nf, const double* host, double* de
   } else {
     const int rc = copy_stream(h);
     if (rc) return rc;
+    CK(cudaEventRecord(h->order_ev, h->st));
+    CK(cudaStreamWaitEvent(h->copy, h->order_ev, 0));
   }
   for (int f = 0; f < nf; f++) {
     double* slot = h->staging + f * ref;
@@ -804,6 +810,7 @@ int gop_destroy(gop_instance* h) {
   if (h->copy) cudaStreamDestroy(h->copy);
   for (cudaEvent_t e : h->field_ev)
     if (e) cudaEventDestroy(e);
+  if (h->order_ev) cudaEventDestroy(h->order_ev);
   sweep_destroy(h->sweep);
   delete[] h->hscal;
   prof_collect(h);

@@ -548,10 +548,14 @@ static int download_fields(gop_instance* h, int nf, const double* dev, double* h
   }
   return GOP_OK;
 }
-// the copies of download_fields have ended
-static int wait_fields(gop_instance* h) {
-  if (h->copy) CK(cudaStreamSynchronize(h->copy));
-  CK(cudaStreamSynchronize(h->st));
+// The end of a call that copied the caller's arrays: waits for every copy, after
+// a failure too (rc), so that the arrays are the caller's again.
+static int wait_fields(gop_instance* h, int rc) {
+  const cudaError_t a = h->copy ? cudaStreamSynchronize(h->copy) : cudaSuccess;
+  const cudaError_t b = cudaStreamSynchronize(h->st);
+  if (rc) return rc;
+  CK(a);
+  CK(b);
   return GOP_OK;
 }
 
@@ -837,9 +841,9 @@ int gop_upload(gop_instance* h, const double* gas, const double* face_b, const d
   if (!rc) rc = upload_fields(h, 3, face_b, P.Bbuf[0]);
   if (!rc && gas_p) rc = upload_fields(h, 6, gas_p, P.Wbuf[1]);
   if (!rc && gas_p) rc = upload_fields(h, 3, face_b_p, P.Bbuf[1]);
+  rc = wait_fields(h, rc);
   if (rc) return rc;
   double* s = h->hscal;
-  CK(cudaStreamSynchronize(h->st));
   for (int t = 0; t < NSCAL; t++) s[t] = 0.0;
   s[S_TIME] = time;
   s[S_DT0] = dt0;
@@ -877,11 +881,9 @@ int gop_set_background(gop_instance* h, const double* b0, const double* lorentz,
                           b0_edge, b0_edge + 3 * ref, b0_edge + 6 * ref};
   const int dst[8] = {BG_B0, BG_LOR, BG_FACE, BG_FACE + 3, BG_FACE + 6,
                       BG_EDGE, BG_EDGE + 3, BG_EDGE + 6};
-  for (int g = 0; g < 8; g++) {
-    rc = upload_fields(h, 3, src[g], h->bg + (size_t)dst[g] * P.fs);
-    if (rc) return rc;
-  }
-  CK(cudaStreamSynchronize(h->st));
+  for (int g = 0; g < 8 && !rc; g++) rc = upload_fields(h, 3, src[g], h->bg + (size_t)dst[g] * P.fs);
+  rc = wait_fields(h, rc);
+  if (rc) return rc;
   CK(cudaGetLastError());
   P.bg = h->bg;
   return GOP_OK;
@@ -916,12 +918,10 @@ int gop_get_background(gop_instance* h, double* b0, double* lorentz, double* b0_
                     b0_edge ? b0_edge + 3 * ref : nullptr, b0_edge ? b0_edge + 6 * ref : nullptr};
   const int src[8] = {BG_B0, BG_LOR, BG_FACE, BG_FACE + 3, BG_FACE + 6,
                       BG_EDGE, BG_EDGE + 3, BG_EDGE + 6};
-  for (int g = 0; g < 8; g++) {
-    if (!dst[g]) continue;
-    const int rc = download_fields(h, 3, h->bg + (size_t)src[g] * P.fs, dst[g]);
-    if (rc) return rc;
-  }
-  return wait_fields(h);
+  int rc = GOP_OK;
+  for (int g = 0; g < 8 && !rc; g++)
+    if (dst[g]) rc = download_fields(h, 3, h->bg + (size_t)src[g] * P.fs, dst[g]);
+  return wait_fields(h, rc);
 }
 
 int gop_problem_init_device(gop_instance* h, const gop_problem* p) {
@@ -1115,8 +1115,7 @@ int gop_step(gop_instance* h, int nsteps, double time_stop, double* time_out) {
 
 // download_fields, and the wait for its copies
 static int download_field(gop_instance* h, int nf, const double* dev, double* host) {
-  const int rc = download_fields(h, nf, dev, host);
-  return rc ? rc : wait_fields(h);
+  return wait_fields(h, download_fields(h, nf, dev, host));
 }
 
 template <typename R>
@@ -1148,8 +1147,8 @@ int gop_download(gop_instance* h, double* gas, double* face_b, double* gas_h, do
   if (!rc && face_b) rc = download_fields(h, 3, P.Bbuf[cur], face_b);
   if (!rc && gas_p) rc = download_fields(h, 6, P.Wbuf[1 - cur], gas_p);
   if (!rc && face_b_p) rc = download_fields(h, 3, P.Bbuf[1 - cur], face_b_p);
-  const int waited = wait_fields(h);  // also where a call failed: the arrays are the caller's again
-  if (rc || waited) return rc ? rc : waited;
+  rc = wait_fields(h, rc);
+  if (rc) return rc;
   if (mags) {
     double* tmp = nullptr;
     CK(device_alloc((void**)&tmp, (size_t)P.fs * 3 * sizeof(double), h->st));

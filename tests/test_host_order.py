@@ -90,3 +90,39 @@ def test_host_arrays_are_read_in_the_callers_stream_order(fake, n, call):
     before, _ = _order(ops)
     reads = [k for k, o in enumerate(ops) if o[0] == "h2d"]
     assert reads and all(0 in before[k] for k in reads)
+
+
+@pytest.mark.parametrize("copy", [1, 2, 4, 8])
+@pytest.mark.parametrize("call", ["upload", "background", "get_background", "download"])
+@pytest.mark.parametrize("n", SIZES)
+def test_a_failed_call_leaves_no_copy_of_the_callers_arrays_running(fake, n, call, copy):
+    """A call that returns with an error has waited for the copies it had
+    started: the arrays are the caller's again."""
+    code, ops = _run(fake, """
+        inst = instance(A["n"])
+        W, B, E = np.zeros(inst.shape(6)), np.zeros(inst.shape(3)), np.zeros(inst.shape(9))
+        bg = dict(b0=B, lorentz=B, b0_face=E, b0_edge=E)
+        if A["call"] == "get_background":
+            inst.set_background(bg)
+        F.fake_clear()
+        F.fake_fail_copy(A["copy"])
+        code = 0
+        try:
+            if A["call"] == "upload":
+                inst.upload(W, B, W, B)
+            elif A["call"] == "background":
+                inst.set_background(bg)
+            elif A["call"] == "get_background":
+                inst.get_background()
+            else:
+                inst.download(("gas", "face_b", "gas_p", "face_b_p"))
+        except gop.GopError as e:
+            code = e.code
+        out = [code, journal()]
+        """, n=n, call=call, copy=copy)
+    if "failed" not in [o[0] for o in ops]:  # the call makes fewer copies
+        assert code == 0
+        return
+    assert code == -5
+    _, done = _order(ops)
+    assert all(k in done for k, o in enumerate(ops) if o[0] in ("h2d", "d2h"))

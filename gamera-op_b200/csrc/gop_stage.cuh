@@ -39,6 +39,14 @@ __device__ __forceinline__ double sqrt_ratio(double n, double d) {
   return n == 0.0 ? 0.0 : __hiloint2double(__double2hiint(r) | nan_bits, __double2loint(r));
 }
 
+// The upper word of a density that is zero, negative, infinite or no number
+// (one comparison: below zero wraps round), where a speed over a common
+// denominator may have a value that the reference's separate roots do not have
+__device__ __forceinline__ bool odd_density(double rho) {
+  return (unsigned)(__double2hiint(rho) - 1) >= 0x7fefffffu;
+}
+__device__ __forceinline__ double no_number() { return __hiloint2double(0x7ff80000, 0); }
+
 // Fast magnetosonic speed sqrt(cs^2 + va^2) with the Boris-limited Alfven
 // speed va^2 = v^2 ca^2 / (v^2 + ca^2), v^2 = b2 / rho, from gp = gamma p, in
 // FP64: over the common denominator rho (b2 + ca^2 rho) it is one reciprocal
@@ -217,9 +225,13 @@ __device__ __forceinline__ R emf_finish(const Params& P, R vp, R vq, R bpl, R bp
   R e = -(vp * bq - vq * bp);
   R vz;
   if constexpr (sizeof(R) == 8) {
-    // Boris-limited Alfven speed as in fast_speed, cs = 0
+    // Boris-limited Alfven speed as in fast_speed, cs = 0.  The half-step
+    // densities are extrapolated and may be negative: no speed then, as
+    // sqrt(b^2 / rho) has none, but for b = 0.
     const R b2 = bp * bp + bq * bq, ca2 = (R)P.ca2;
-    vz = sqrt_ratio(b2 * ca2, b2 + R(0.25) * ca2 * rho4) + sqrt(vp * vp + vq * vq);
+    R va = sqrt_ratio(b2 * ca2, b2 + R(0.25) * ca2 * rho4);
+    if (odd_density(rho4) && !(rho4 > 0.0 || (rho4 < 0.0 && b2 == 0.0))) va = no_number();
+    vz = va + sqrt(vp * vp + vq * vq);
   } else {
     const R ca = (R)P.ca;
     vz = sqrt((bp * bp + bq * bq) / (R(0.25) * rho4));

@@ -30,13 +30,11 @@ __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
 // comparison and a select, where fmax(double) is twice that)
 __device__ __forceinline__ double max2(double a, double b) { return a > b || b != b ? a : b; }
 
-// sqrt(n / d) for d > 0 as n rsqrt(n d): one special function where the
-// division and the root take two of about 25 instructions each.  Not a number
-// for n or d below zero (a negative density, say), both included.
+// sqrt(n / d) for n, d > 0 (zero for n = 0) as n rsqrt(n d): one special
+// function where the division and the root take two of about 25 instructions
+// each
 __device__ __forceinline__ double sqrt_ratio(double n, double d) {
-  const double r = n * rsqrt(n * d);
-  const int nan_bits = (__double2hiint(d) >> 31) & 0x7ff80000;
-  return n == 0.0 ? 0.0 : __hiloint2double(__double2hiint(r) | nan_bits, __double2loint(r));
+  return n == 0.0 ? 0.0 : n * rsqrt(n * d);
 }
 
 // The upper word of a density that is zero, negative, infinite or no number
@@ -53,9 +51,16 @@ __device__ __forceinline__ double no_number() { return __hiloint2double(0x7ff800
 // root.  The reference's order (src/solver_func.c:1005-1018) takes three
 // roots, a reciprocal root and a division per state.  Blast 256^3 on B200:
 // flux stage 2.56 -> 2.34 ms per step, the EMFs' form of it 1.72 -> 1.58 ms.
+// What decides whether there is a speed is what the separate roots decide by:
+// no number for a negative pressure, however strong the field, nor for a
+// density of zero or below (but for -rho and -p without a field, whose ratio
+// is that of rho and p).
 __device__ __forceinline__ double fast_speed(double gp, double rho, double b2, double ca2) {
   const double q = b2 + ca2 * rho, r = ca2 * rho;
-  return sqrt_ratio(gp * q + b2 * r, rho * q);
+  double v = sqrt_ratio(gp * q + b2 * r, rho * q);
+  if (odd_density(rho) || __double2hiint(gp) < 0)
+    if (!(rho > 0.0 ? gp >= 0.0 : rho < 0.0 && gp <= 0.0 && b2 == 0.0)) v = no_number();
+  return v;
 }
 
 // The step-start state the PDM limiters compare against, in the stage type:

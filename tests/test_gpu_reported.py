@@ -53,3 +53,35 @@ def test_negative_density_around_an_edge(b, prec, sweep):
     Wp = W.copy()
     Wp[(0,) + PATCH] = 1.0
     assert _step(W, B, (Wp, B), prec, sweep) == (0 if b == 0.0 else -34)
+
+
+@pytest.mark.parametrize("sweep", [True, False])
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("rho,p", [(1.0, -0.5), (-1.0, 1.0), (-1.0, -0.5), (0.0, 1.0)])
+@pytest.mark.parametrize("b", [0.0, 0.3, 5.0, 30.0])
+def test_states_without_a_signal_speed(b, rho, p, prec, sweep):
+    """A patch of negative pressure (in a field strong enough, the common
+    denominator's numerator is positive there), of negative density, of both,
+    of no density."""
+    W, B = _state(1.0, 1.0, b)
+    W[(0,) + PATCH], W[(4,) + PATCH] = rho, p
+    assert _step(W, B, None, prec, sweep) == -34
+
+
+@pytest.mark.parametrize("b", [0.0, 0.3, 5.0, 30.0])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_cells_without_a_signal_speed_set_no_time_step(b, prec):
+    """The CFL minimum of the prepared state skips a cell of negative pressure."""
+    import gop
+
+    W, B = _state(1.0, 1.0, b)
+    dt = []
+    for bad in (False, True):
+        if bad:  # would be the fastest cell by far
+            W[0, NG + 3, NG + 3, NG + 3], W[4, NG + 3, NG + 3, NG + 3] = 1e-6, -1e-9
+        inst = gop.Instance(N3, *[gop.grid_uniform(m, 0.0, 1.0) for m in N3], precision=prec)
+        inst.upload(W, B)
+        inst.prepare()
+        dt.append(inst.stats()["dt0"])
+        inst.close()
+    assert dt[0] == dt[1]

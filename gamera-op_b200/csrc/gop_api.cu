@@ -981,6 +981,7 @@ int gop_prepare(gop_instance* h, int restart) {
   s[S_FLAGS] = 0.0;
   s[S_PAR] = 0.0;
   s[S_PSNZ] = 0.0;
+  s[S_TILE] = 0.0;  // a pipeline that gave up may leave its counters above zero
   CK(cudaMemcpyAsync(h->scal, s, NSCAL * sizeof(double), cudaMemcpyHostToDevice, h->st));
   // CFL dt and div B of the initial state (src/solver_solve.c:94-98)
   launch_dt(P, h->d.coord, h->d.precision == GOP_PREC_MIXED, h->st);

@@ -6,6 +6,7 @@ is what the graph says.  Fields below and above the size from which they travel
 on a stream of their own."""
 import json
 import os
+import re
 import subprocess
 import sys
 import textwrap
@@ -126,3 +127,31 @@ def test_a_failed_call_leaves_no_copy_of_the_callers_arrays_running(fake, n, cal
     assert code == -5
     _, done = _order(ops)
     assert all(k in done for k, o in enumerate(ops) if o[0] in ("h2d", "d2h"))
+
+
+def _scalars():
+    """Places of the instance's device scalars by name (and their number)."""
+    src = (ROOT / "gamera-op_b200/csrc/gop_device.cuh").read_text()
+    body = re.sub(r"//[^\n]*", "", re.search(r"enum Scal : int \{(.*?)\}", src, re.S).group(1))
+    return {m.split("=")[0].strip(): k for k, m in enumerate(x for x in body.split(",") if x.strip())}
+
+
+@pytest.mark.parametrize("restart", [False, True])
+def test_prepare_clears_what_a_failed_step_left(fake, restart):
+    """A step whose pipeline gave up may leave its tile counters above zero: a
+    prepared instance starts from clear flags and counters all the same."""
+    sc = _scalars()
+    left = _run(fake, """
+        inst = instance((16, 16, 16))
+        inst.upload(np.zeros(inst.shape(6)), np.zeros(inst.shape(3)))
+        s = (C.c_double * A["count"]).from_address(F.fake_block(8 * A["count"]))
+        for k in A["names"]:
+            s[k] = 3.0
+        try:
+            inst.prepare(restart=A["restart"])
+        except gop.GopError:  # (no kernel has set a time step)
+            pass
+        out = [s[k] for k in A["names"]]
+        """, names=[sc[k] for k in ("S_STOP", "S_STEPS", "S_FLAGS", "S_PAR", "S_TILE")], count=sc["NSCAL"],
+        restart=restart)
+    assert left == [0.0] * 5

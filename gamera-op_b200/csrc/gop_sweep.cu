@@ -546,8 +546,7 @@ struct alignas(64) SweepMaps {
 template <class SW, typename R>
 __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
                                           const SweepMaps<typename SW::Maps>& maps, Gather& gather) {
-  // stop flag, or an earlier pipeline wait that timed out: do nothing
-  if (stopped(P) || P.scal[S_FLAGS] == 2.0) return;
+  if (stopped(P)) return;
   constexpr int S = SW::S;
   using S0 = typename SW::template Stage<0>;
   using S1 = typename SW::template Stage<1>;
@@ -605,19 +604,25 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
       more = false;
     }
   };
+  // After a pipeline wait that timed out (flag 2, which another block may be
+  // setting now) a block has no work.  The feeder looks for all of the block, so
+  // that no thread waits for a ring that was not set up, and the block counts
+  // itself like the others, so that the counters end at zero.
+  bool leave = false;
   if (feeder) {
+    leave = P.scal[S_FLAGS] == 2.0;
     for (int q = 0; q < S; q++) {
       mbar_init(&full[q], 1);
       mbar_init(&empty[q], kWarps);
     }
     fence_mbar_init();
-    for (int q = 0; q < S && more; q++) feed(q);
+    for (int q = 0; q < S && more && !leave; q++) feed(q);
   }
-  __syncthreads();
+  leave = __syncthreads_or(leave) != 0;
   bool ok = true;
   int q = 0;
   uint32_t ph = 0;
-  for (;;) {
+  while (!leave) {
     if (!mbar_wait(&full[q], ph)) {
       ok = false;
       break;

@@ -74,7 +74,8 @@ enum Scal : int {
   S_STEPS,       // steps taken (as double)
   S_STOP,        // nonzero: time_stop reached, kernels return at once
   S_TSTOP,       // time_stop of the current gop_step call
-  S_FLAGS,       // bit 0: non-finite / non-positive state seen
+  S_FLAGS,       // 1: non-finite / non-positive state seen; 2: a pipeline wait
+                 // timed out (stays, whatever is seen after it)
   S_PAR,         // which of the two state buffers holds the current state
   S_BUDGET,      // steps left in the current gop_step call
   S_PSNZ,        // gop_prepare's check: nonzero if some p_S of the state or

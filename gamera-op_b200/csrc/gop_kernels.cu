@@ -92,7 +92,7 @@ __device__ __forceinline__ void begin_body(const Params& P) {
   }
   s[S_BUDGET] = s[S_BUDGET] - 1.0;
   const double dt = s[S_NEXT_DT];
-  if (!(dt > 0.0) || !isfinite(dt)) s[S_FLAGS] = 1.0;
+  if (!(dt > 0.0) || !isfinite(dt)) flag_numeric(P);
   s[S_DT] = dt;
   s[S_TIME] = s[S_TIME] + dt;
   s[S_CAB2] = 0.5 * dt / s[S_DT0];
@@ -577,7 +577,7 @@ __device__ __forceinline__ void update_body(const Params& P, const Work<R>& wk, 
                      ((bu[2] + b0u[2]) * fu[2] - (bl[2] + b0l[2]) * fl[2]) * ivol;
   dbmax = fabs(dvb);
   if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
-    P.scal[S_FLAGS] = 1.0;
+    flag_numeric(P);
   if (COORD == 2 && P.ring && ring_band_row(P, j)) {
     // the ring average still changes this row: k_ring_dt takes its CFL dt
     // and div B afterwards

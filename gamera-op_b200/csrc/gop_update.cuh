@@ -82,6 +82,11 @@ __device__ __forceinline__ void block_commit(const Params& P, double a, double b
   }
 }
 
+// a non-finite or non-positive state was seen (1; the flag of a timed-out wait,
+// 2, says that the state is none at all and stays)
+__device__ __forceinline__ void flag_numeric(const Params& P) {
+  if (P.scal[S_FLAGS] == 0.0) atomic_max_pos(P.scal + S_FLAGS, 1.0);
+}
 // A rate that gives no positive time step
 __device__ __forceinline__ bool bad_rate(double rate) { return !(rate >= 0.0 && rate <= DBL_MAX); }
 
@@ -340,7 +345,7 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
     rate = cfl_cart<RC>(P, il, rho, vv[0], vv[1], vv[2], p, t0 * t0 + t1 * t1 + t2 * t2);
   }
   if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
-    P.scal[S_FLAGS] = 1.0;
+    flag_numeric(P);
 }
 
 // One active cell of a spherical grid without the pole ring average
@@ -541,7 +546,7 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
   const double rctr = in.tab(0, T_G3);
   rate = cfl_sph(vc, in.tab(0, T_DX), rctr * in.tab(1, T_DX), rctr * in.tab(1, T_G2) * in.tab(2, T_DX));
   if (bad_rate(rate) || !isfinite(p) || !isfinite(rho) || !isfinite(vv[0] + vv[1] + vv[2]))
-    P.scal[S_FLAGS] = 1.0;
+    flag_numeric(P);
 }
 
 }  // namespace gop

@@ -1,8 +1,8 @@
 """Steps of an instance whose error flag says that a pipeline wait has timed out
 (the flag is written from outside; nothing waits): the tile-staged launches leave
 without work, every block counts itself so that the tile counters end at zero
-even if they did not begin so, and the instance is whole again after an
-upload."""
+even if they did not begin so, the step reports the timeout and nothing else, and
+the instance is whole again after an upload."""
 import json
 import os
 import subprocess
@@ -91,4 +91,13 @@ def _run(blocks, n, prec, nan):
 @pytest.mark.parametrize("n", [(32, 24, 20), (64, 96, 96)])
 def test_flagged_steps_leave_the_counters_at_zero(blocks, n, prec):
     out = _run(blocks, n, prec, False)
+    assert out == dict(clean=0, flagged=-5, flags=2, counters=0.0, again=0, same=True)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("n", [(32, 24, 20), (64, 96, 96)])
+def test_a_timed_out_step_is_not_taken_for_a_bad_state(blocks, n, prec):
+    """The per-cell update runs on what the sweeps have left undone and finds a
+    state that is no number."""
+    out = _run(blocks, n, prec, True)
     assert out == dict(clean=0, flagged=-5, flags=2, counters=0.0, again=0, same=True)

@@ -589,6 +589,12 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
   unsigned* counters = reinterpret_cast<unsigned*>(P.scal + S_TILE);
   const bool feeder = threadIdx.x == 0;
   int next = blockIdx.x;  // feeder only: the next tile to issue
+  // After a pipeline wait that timed out (flag 2, which another block may be
+  // setting now) there is no work.  The feeder looks for all of the block: the
+  // ring is set up and carries the end at once, so that no thread reads a tile or
+  // waits at a barrier that nobody has written, and the block counts itself like
+  // the others, so that the counters end at zero.
+  if (feeder && P.scal[S_FLAGS] == 2.0) next = ntiles;
   int issued = 0;         // feeder only: tiles whose copies were issued
   bool more = true;       // feeder only: the end has not been passed on
   // the feeder: the next tile into slot q, or the end of the work
@@ -604,25 +610,19 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
       more = false;
     }
   };
-  // After a pipeline wait that timed out (flag 2, which another block may be
-  // setting now) a block has no work.  The feeder looks for all of the block, so
-  // that no thread waits for a ring that was not set up, and the block counts
-  // itself like the others, so that the counters end at zero.
-  bool leave = false;
   if (feeder) {
-    leave = P.scal[S_FLAGS] == 2.0;
     for (int q = 0; q < S; q++) {
       mbar_init(&full[q], 1);
       mbar_init(&empty[q], kWarps);
     }
     fence_mbar_init();
-    for (int q = 0; q < S && more && !leave; q++) feed(q);
+    for (int q = 0; q < S && more; q++) feed(q);
   }
-  leave = __syncthreads_or(leave) != 0;
+  __syncthreads();
   bool ok = true;
   int q = 0;
   uint32_t ph = 0;
-  while (!leave) {
+  for (;;) {
     if (!mbar_wait(&full[q], ph)) {
       ok = false;
       break;

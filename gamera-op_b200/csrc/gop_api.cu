@@ -691,6 +691,7 @@ int gop_create(const gop_desc* desc, gop_instance** out) {
   P.cfl = d.cfl;
   P.ca = d.ca;
   P.ca2 = d.ca * d.ca;
+  split_ca2(d.ca, P.ca2m, P.ca2s);
   P.rho_floor = d.rho_floor;
   P.p_floor = d.p_floor;
   P.inv_gm1 = 1.0 / P.gm1;

@@ -96,6 +96,7 @@ struct Params {
   const double* tab;  // [3][NTAB][tmax]
   int tmax;
   double gamma, gm1, cfl, ca, ca2, rho_floor, p_floor;
+  double ca2m, ca2s;      // ca^2 = ca2m / ca2s (split_ca2)
   double inv_gm1;         // 1/(gamma-1)
   double q_ca;            // 1/(4 CA): Boris diffusion coefficient of the stress
   double* scal;           // device scalars

@@ -43,7 +43,8 @@ constexpr int kThreads = 256;
 struct Args {
   int n[3], N[3];
   int sph;
-  double gamma, cfl, ca, ca2;
+  double gamma, cfl;
+  double ca2m, ca2s;  // ca^2 = ca2m / ca2s (split_ca2)
   const double* gas;  // [6][NI][NJ][NK], k fastest (reference layout)
   const double* fb;   // [3][NI][NJ][NK]
   const double* b0;   // background field at the cell centroid [3][NI][NJ][NK], or null
@@ -143,7 +144,7 @@ __device__ __forceinline__ void cell_rate_divb(const Args& A, size_t c, size_t s
   // |v| + sqrt(cs^2 + va^2) with va^2 = v^2 ca^2 / (v^2 + ca^2), v^2 = b^2 /
   // rho, over the common denominator; no number where the density or the
   // pressure is negative, as the roots of the separate terms give
-  const double b2 = m1 * m1 + m2 * m2 + m3 * m3, r = A.ca2 * rho, q = b2 + r;
+  const double b2 = m1 * m1 + m2 * m2 + m3 * m3, r = A.ca2m * rho, q = fma(A.ca2m, rho, b2 * A.ca2s);
   const double num = A.gamma * p * q + b2 * r, den = rho * q;
   double f = num == 0.0 ? 0.0 : num * rsqrt(num * den);
   if (!(rho > 0.0) || p < 0.0) f = nan("");
@@ -297,8 +298,7 @@ extern "C" int gop_cfl_dt_noalloc(const gop_desc* desc, const double* gas, const
   A.sph = desc->coord == GOP_COORD_SPHERICAL;
   A.gamma = desc->gamma != 0 ? desc->gamma : 5.0 / 3.0;
   A.cfl = desc->cfl != 0 ? desc->cfl : 0.3;
-  A.ca = desc->ca != 0 ? desc->ca : 10.0;
-  A.ca2 = A.ca * A.ca;
+  gop::split_ca2(desc->ca != 0 ? desc->ca : 10.0, A.ca2m, A.ca2s);
   A.gas = gas;
   A.fb = face_b;
   A.b0 = b0;

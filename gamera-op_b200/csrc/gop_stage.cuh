@@ -55,8 +55,8 @@ __device__ __forceinline__ double no_number() { return __hiloint2double(0x7ff800
 // no number for a negative pressure, however strong the field, nor for a
 // density of zero or below (but for -rho and -p without a field, whose ratio
 // is that of rho and p).
-__device__ __forceinline__ double fast_speed(double gp, double rho, double b2, double ca2) {
-  const double q = b2 + ca2 * rho, r = ca2 * rho;
+__device__ __forceinline__ double fast_speed(const Params& P, double gp, double rho, double b2) {
+  const double r = P.ca2m * rho, q = fma(b2, P.ca2s, r);
   double v = sqrt_ratio(gp * q + b2 * r, rho * q);
   if (odd_density(rho) || __double2hiint(gp) < 0)
     if (!(rho > 0.0 ? gp >= 0.0 : rho < 0.0 && gp <= 0.0 && b2 == 0.0)) v = no_number();
@@ -112,7 +112,7 @@ __device__ __forceinline__ void flux_out(const Params& P, const Work<R>& wk, int
   const R vnl = L[V1 + D], vnr = Rt[V1 + D];
   R vf;
   if constexpr (sizeof(R) == 8) {
-    vf = max2(fabs(vnl) + fast_speed(gm * pl, rl, ttl, ca2), fabs(vnr) + fast_speed(gm * pr, rr, ttr, ca2));
+    vf = max2(fabs(vnl) + fast_speed(P, gm * pl, rl, ttl), fabs(vnr) + fast_speed(P, gm * pr, rr, ttr));
   } else {
     const R irl = R(1) / rl, irr = R(1) / rr;
     const R csl = sqrt(gm * pl * irl), csr = sqrt(gm * pr * irr);
@@ -233,8 +233,8 @@ __device__ __forceinline__ R emf_finish(const Params& P, R vp, R vq, R bpl, R bp
     // Boris-limited Alfven speed as in fast_speed, cs = 0.  The half-step
     // densities are extrapolated and may be negative: no speed then, as
     // sqrt(b^2 / rho) has none, but for b = 0.
-    const R b2 = bp * bp + bq * bq, ca2 = (R)P.ca2;
-    R va = sqrt_ratio(b2 * ca2, b2 + R(0.25) * ca2 * rho4);
+    const R b2 = bp * bp + bq * bq;
+    R va = sqrt_ratio(b2 * P.ca2m, fma(R(0.25) * P.ca2m, rho4, b2 * P.ca2s));
     if (odd_density(rho4) && !(rho4 > 0.0 || (rho4 < 0.0 && b2 == 0.0))) va = no_number();
     vz = va + sqrt(vp * vp + vq * vq);
   } else {

@@ -95,7 +95,7 @@ __device__ __forceinline__ bool bad_rate(double rate) { return !(rate >= 0.0 && 
 // term by term
 __device__ __forceinline__ double signal_speed(const Params& P, double r, double u, double v, double w,
                                                double p, double bsq) {
-  return sqrt(u * u + v * v + w * w) + fast_speed(P.gamma * p, r, bsq, P.ca2);
+  return sqrt(u * u + v * v + w * w) + fast_speed(P, P.gamma * p, r, bsq);
 }
 __device__ __forceinline__ float signal_speed(const Params& P, float r, float u, float v, float w, float p,
                                               float bsq) {
@@ -309,8 +309,8 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
     const RA bsq = (RA)(mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
     RA alf, perp;
     if constexpr (sizeof(RA) == 8) {  // b^2 / (rho ca^2) and 1 / (1 + that) by one division
-      const double rc = rho * P.ca2, q = rc + bsq, inv = 1.0 / (rc * q);
-      alf = bsq * q * inv;
+      const double rc = rho * P.ca2m, bs = bsq * P.ca2s, q = fma(bsq, P.ca2s, rc), inv = 1.0 / (rc * q);
+      alf = bs * q * inv;
       perp = rc * rc * inv;
     } else {
       alf = bsq / ((RA)rho * (RA)P.ca2);
@@ -515,8 +515,8 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
   const R bsq = mr[0] * mr[0] + mr[1] * mr[1] + mr[2] * mr[2];
   R alf, perp;
   // b^2 / (rho ca^2) and 1 / (1 + that) by one division
-  const double rc = rho * P.ca2, q = rc + bsq, inv = 1.0 / (rc * q);
-  alf = bsq * q * inv;
+  const double rc = rho * P.ca2m, bs = bsq * P.ca2s, q = fma(bsq, P.ca2s, rc), inv = 1.0 / (rc * q);
+  alf = bs * q * inv;
   perp = rc * rc * inv;
   const R rdt = (R)dt;
   const R drho = -rdt * du[0];

@@ -280,7 +280,7 @@ struct FluxStage {
       for (int u = 0; u < 8; u++) v[u] = wh[f * F::SB + u * TS];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = wl[f * F::LB + u * TS];
-      recon_lr(v, lim, Wt, L[f], Rt[f]);
+      recon_lr<D>(v, lim, Wt, L[f], Rt[f]);
     }
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -289,7 +289,7 @@ struct FluxStage {
       for (int u = 0; u < 8; u++) v[u] = msh[a * F::SB + u * TS];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = ms[a * F::LB + u * TS];
-      recon_lr(v, lim, Wt, mL[a], mR[a]);
+      recon_lr<D>(v, lim, Wt, mL[a], mR[a]);
     }
     flux_out<R, D, BG, false>(P, wk, lin32(P, i, j, k), D == 0 ? j : (D == 1 ? k : i), L, Rt, mL, mR,
                               bn);
@@ -453,7 +453,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = v0[cc * E::VF + u * tq];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = v[u + 2];
-      recon_lr(v, lim, Wq, L, Rr);
+      recon_lr<q>(v, lim, Wq, L, Rr);
       vav[cc] = R(0.5) * (L + Rr);
     }
     {  // B_p along q
@@ -462,7 +462,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = bp[u * tq];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = bpl[u * tq];
-      recon_lr(v, lim, Wq, bpL, bpR);
+      recon_lr<q>(v, lim, Wq, bpL, bpR);
     }
     {  // B_q along p
       R v[8], lim[4];
@@ -470,7 +470,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = bq[u * tp];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = bql[u * tp];
-      recon_lr(v, lim, Wp, bqL, bqR);
+      recon_lr<p>(v, lim, Wp, bqL, bqR);
     }
     const int x = lin32(P, i, j, k);
     const size_t fs = P.fs;

@@ -78,7 +78,7 @@ def _lines(rng, n, whole):
 
 def _check(lib, v, lim, w):
     ref = _reference(v, lim, w)
-    size = np.maximum(np.nan_to_num(np.abs(v)).max(1), np.abs(lim).max(1))[:, None]
+    size = np.maximum(np.nan_to_num(np.abs(v), posinf=0.0).max(1), np.abs(lim).max(1))[:, None]
     for bits, tol in ((64, 1e-14), (32, 6e-6)):
         got = _device(lib, bits, v, lim, w)
         ok = np.abs(got - ref) <= tol * size
@@ -104,3 +104,16 @@ def test_face_without_an_area(libs, signs, whole):
     w[:, 14], w[:, 15] = signs[0] * np.inf, signs[1] * np.inf
     w[:, 16], w[:, 17] = signs[1] * np.inf, signs[0] * np.inf
     _check(libs[1], v, lim, w)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("taps", [(0,), (7,), (3, 4), range(8)])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("whole", [False, True])
+def test_lost_taps(libs, axis, taps, value, whole):
+    """A half-step value that is no number: the clamp's fmin leaves the larger of
+    the two neighbours, on either side of the face and for either direction.  An
+    infinite one is clamped."""
+    v, lim, w = _lines(np.random.default_rng(11), 20000, whole)
+    v[:, list(taps)] = value
+    _check(libs[axis], v, lim, w)

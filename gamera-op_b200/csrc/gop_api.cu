@@ -419,6 +419,8 @@ cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
+int periodic(const gop_desc& d, int a) { return d.bc[2 * a] == 'p' && d.bc[2 * a + 1] == 'p'; }
+
 struct Layout {
   int N[3];
   int pitch;
@@ -678,7 +680,7 @@ int gop_create(const gop_desc* desc, gop_instance** out) {
   P.n[2] = d.nk;
   for (int a = 0; a < 3; a++) {
     P.N[a] = L.N[a];
-    P.per[a] = d.bc[2 * a] == 'p' && d.bc[2 * a + 1] == 'p';
+    P.per[a] = periodic(d, a);
   }
   P.pitch = L.pitch;
   P.coord = d.coord;
@@ -964,6 +966,7 @@ int gop_prepare(gop_instance* h, int restart) {
   // every field: the state may be new
   Params Pall = P;
   Pall.ps_live = 1;
+  for (int a = 0; a < 3; a++) Pall.per[a] = periodic(h->d, a);
   launch_ghosts(Pall, h->d.bc, h->d.gem_bc, 1, h->st);
   if (!restart) {
     // AB2 history <- current state (src/solver_solve.c:55-92)
@@ -982,19 +985,29 @@ int gop_prepare(gop_instance* h, int restart) {
   s[S_FLAGS] = 0.0;
   s[S_PAR] = 0.0;
   s[S_PSNZ] = 0.0;
+  s[S_HISTG] = 0.0;
   s[S_TILE] = 0.0;  // a pipeline that gave up may leave its counters above zero
   CK(cudaMemcpyAsync(h->scal, s, NSCAL * sizeof(double), cudaMemcpyHostToDevice, h->st));
   // CFL dt and div B of the initial state (src/solver_solve.c:94-98)
   launch_dt(P, h->d.coord, h->d.precision == GOP_PREC_MIXED, h->st);
   // is the entropy channel live?  A p_S that is zero in the state and its
-  // history stays zero in every later step, and the flux kernels skip it
-  launch_ps_check(P, h->st);
+  // history stays zero in every later step, and the flux kernels skip it.  And
+  // do the periodic ghost layers of an uploaded history repeat the active cells?
+  // Where they do not, the flux stage's edge velocities are not those of the
+  // layers, which k_c2c then reconstructs from what was uploaded.
+  launch_state_check(Pall, restart != 0, h->st);
   CK(cudaMemcpyAsync(s, h->scal, NSCAL * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
   const int live = s[S_PSNZ] != 0.0 ? 1 : 0;
   if (live != h->P.ps_live) {
     drop_step_graph(h);
     h->P.ps_live = live;
+  }
+  for (int a = 0; a < 3; a++) {
+    const int per = s[S_HISTG] == 0.0 ? Pall.per[a] : 0;
+    if (per == h->P.per[a]) continue;
+    drop_step_graph(h);
+    h->P.per[a] = per;
   }
   if (!restart) s[S_DT0] = s[S_NEXT_DT];
   CK(cudaMemcpyAsync(h->scal, s, NSCAL * sizeof(double), cudaMemcpyHostToDevice, h->st));

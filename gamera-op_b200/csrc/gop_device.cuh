@@ -80,6 +80,9 @@ enum Scal : int {
   S_BUDGET,      // steps left in the current gop_step call
   S_PSNZ,        // gop_prepare's check: nonzero if some p_S of the state or
                  // of its AB2 history is nonzero
+  S_HISTG,       // gop_prepare's check of an uploaded AB2 history: nonzero if a
+                 // velocity in a periodic ghost layer is not that of the cell
+                 // the layer repeats
   S_TILE,        // two 32-bit counters of the running launch: tiles handed
                  // out (sweeps), blocks done; zero between launches
   NSCAL
@@ -90,7 +93,8 @@ struct Params {
   int N[3];           // ghost-extended points
   int pitch;          // row pitch (elements)
   int coord;          // 0: Cartesian, 2: spherical (batched kernels select on it)
-  int per[3];         // 1: the axis is periodic
+  int per[3];         // 1: the axis is periodic and its ghost layers repeat the active cells, in
+                      // the AB2 history too (gop_prepare looks)
   long long sj, sk;   // strides of j and k (stride of i is 1)
   long long fs;       // stride between fields
   const double* tab;  // [3][NTAB][tmax]

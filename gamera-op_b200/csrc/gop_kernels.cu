@@ -842,9 +842,11 @@ __global__ void k_turn(Params P) {
   turn_body(P);
 }
 
-// S_PSNZ <- 1 if p_S of either state buffer is nonzero at a point the AB2
-// stage reads (every point but the last plane of each axis)
-__global__ void k_ps_check(Params P) {
+// At the points the AB2 stage reads (every point but the last plane of each
+// axis): S_PSNZ <- 1 if p_S of either state buffer is nonzero; with an uploaded
+// history (in buffer 1) S_HISTG <- 1 if its velocities in the ghost layers of
+// the axes in P.per are not those of the cells the layers repeat
+__global__ void k_state_check(Params P, bool history) {
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
   bool nz = false;
@@ -853,6 +855,19 @@ __global__ void k_ps_check(Params P) {
     nz = P.Wbuf[0][x] != 0.0 || P.Wbuf[1][x] != 0.0;
   }
   if (__any_sync(0xffffffffu, nz) && (threadIdx.x & 31) == 0) P.scal[S_PSNZ] = 1.0;
+  if (!history) return;
+  bool other = false;
+  if (i < P.N[0] - 1 && j < P.N[1] - 1 && k < P.N[2] - 1) {
+    const int x[3] = {i, j, k};
+    for (int a = 0; a < 3; a++) {
+      if (!P.per[a] || (x[a] >= NGH && x[a] < NGH + P.n[a])) continue;
+      const double* h = P.Wbuf[1] + lin(P, i, j, k);
+      const long long s = (x[a] < NGH ? P.n[a] : -P.n[a]) * stride(P, a);
+      for (int m = V1; m <= V3; m++)
+        other = other || !(h[(long long)m * P.fs] == h[(long long)m * P.fs + s]);
+    }
+  }
+  if (__any_sync(0xffffffffu, other) && (threadIdx.x & 31) == 0) P.scal[S_HISTG] = 1.0;
 }
 
 template <int COORD, bool BG, typename R>
@@ -1122,10 +1137,10 @@ void launch_arm(const Params& P, double tstop, double budget, cudaStream_t st) {
   LAUNCH(k_arm, 1, 1, st, P, tstop, budget);
 }
 
-void launch_ps_check(const Params& P, cudaStream_t st) {
+void launch_state_check(const Params& P, bool history, cudaStream_t st) {
   const int nx = (P.N[0] - 1 + 31) / 32 * 32;
   const dim3 blk(std::min(nx, 256), 1, 1);
-  LAUNCH(k_ps_check, dim3((nx + blk.x - 1) / blk.x, P.N[1] - 1, P.N[2] - 1), blk, st, P);
+  LAUNCH(k_state_check, dim3((nx + blk.x - 1) / blk.x, P.N[1] - 1, P.N[2] - 1), blk, st, P, history);
 }
 
 template <typename R>

@@ -95,8 +95,10 @@ void launch_arm(const Params& P, double tstop, double budget, cudaStream_t st);
 // CFL dt (in the form and arithmetic of the step's own estimate) and
 // max|div B| of the current state
 void launch_dt(const Params& P, int coord, bool mixed, cudaStream_t st);
-// P.scal[S_PSNZ] <- 1 if p_S is nonzero in either state buffer (it must be 0 before)
-void launch_ps_check(const Params& P, cudaStream_t st);
+// P.scal[S_PSNZ] <- 1 if p_S is nonzero in either state buffer, and with an
+// uploaded history S_HISTG <- 1 if its periodic ghosts do not repeat its active
+// cells (both must be 0 before)
+void launch_state_check(const Params& P, bool history, cudaStream_t st);
 template <typename R>
 void launch_step_body(const Params& P, int coord, const Work<R>& w, cudaStream_t st,
                       const Tune& tune, const SweepSet* sw, const Hook& hook = Hook());

@@ -122,7 +122,10 @@ int gop_upload(gop_instance *h, const double *gas, const double *face_b,
 
 /* The start of solve() before its loop (src/solver_solve.c:25-99): ghost
  * fill, derived variables, and for a fresh start (restart == 0) the AB2
- * history copy and the initial CFL dt0. */
+ * history copy and the initial CFL dt0.  The ghosts of an uploaded history are
+ * taken as they are; where those of a periodic axis do not repeat its active
+ * cells, every step until the next gop_prepare reconstructs the edge velocities
+ * there (one launch more). */
 int gop_prepare(gop_instance *h, int restart);
 
 /* nsteps passes of the time loop (src/solver_solve.c:102-529).  Stops early

@@ -1121,6 +1121,7 @@ Tune::Tune() {
 dim3 launch_space(const Params& P, int slot) {
   if (slot == K_AB2) return dim3(P.N[0], P.N[1], P.N[2]);
   if (slot == K_UPDATE) return dim3(P.n[0], P.n[1], P.n[2]);
+  if (slot < K_EMF0 || slot > K_FLUX2) return dim3(0, 0, 0);
   const bool emf = slot < K_FLUX0;
   const int D = emf ? slot - K_EMF0 : slot - K_FLUX0;
   int cnt[3] = {P.n[0], P.n[1], P.n[2]};
@@ -1172,6 +1173,7 @@ template <typename R, bool BG>
 static void launch_slot_bg(const Params& P, int coord, const Work<R>& w, int slot, dim3 blk,
                            cudaStream_t st, bool pdl) {
   const dim3 sp = launch_space(P, slot);
+  if (sp.x == 0) return;
   const dim3 g = grid3(sp.x, sp.y, sp.z, blk);
   switch (slot) {
     case K_AB2:

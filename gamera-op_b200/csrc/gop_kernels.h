@@ -34,8 +34,8 @@ void count_launches(int64_t n);  // kernels run by graph replays
 // kernel groups of one step, for event timing
 enum Group : int { G_BEGIN = 0, G_AB2, G_C2C, G_EMF, G_FLUX, G_UPDATE, G_GHOST, G_END, NGROUP };
 
-// launch shapes of the tunable kernels: AB2, C2C x3, EMF x3, FLUX x3,
-// UPDATE
+// launch shapes of the tunable kernels: AB2, C2C x3 (places of gop_autotune's
+// result alone: their launch has one shape), EMF x3, FLUX x3, UPDATE
 enum TuneSlot : int { K_AB2 = 0, K_C2C0, K_C2C1, K_C2C2, K_EMF0, K_EMF1, K_EMF2,
                       K_FLUX0, K_FLUX1, K_FLUX2, K_UPDATE, NTUNE };
 struct Tune {
@@ -72,7 +72,8 @@ bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, con
 template <typename R>
 bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st);
 
-// points covered by the launch of one slot (x, y, z extents)
+// points covered by the launch of one slot (x, y, z extents); none for K_C2C0..2,
+// which are one launch of a fixed shape within launch_step_body
 dim3 launch_space(const Params& P, int slot);
 
 // launches one tunable kernel; pdl false: without programmatic dependent

@@ -142,12 +142,13 @@ __device__ __forceinline__ void cell_rate_divb(const Args& A, size_t c, size_t s
     bu[2] += f2[1];
   }
   // |v| + sqrt(cs^2 + va^2) with va^2 = v^2 ca^2 / (v^2 + ca^2), v^2 = b^2 /
-  // rho, over the common denominator; no number where the density or the
-  // pressure is negative, as the roots of the separate terms give
+  // rho, over the common denominator; no number where the density is not above
+  // zero or the pressure below it (but for both below without a field), as the
+  // roots of the separate terms give
   const double b2 = m1 * m1 + m2 * m2 + m3 * m3, r = A.ca2m * rho, q = fma(A.ca2m, rho, b2 * A.ca2s);
   const double num = A.gamma * p * q + b2 * r, den = rho * q;
   double f = num == 0.0 ? 0.0 : num * rsqrt(num * den);
-  if (!(rho > 0.0) || p < 0.0) f = nan("");
+  if (!(rho > 0.0 ? p >= 0.0 : rho < 0.0 && p <= 0.0 && b2 == 0.0)) f = nan("");
   rate = (sqrt(u * u + v * v + w * w) + f) * (R.il + R.il3 * id3);
   divb = fabs((bu[0] * R.d1u - bl[0] * R.d1l) + (bu[1] * R.d2u - bl[1] * R.d2l) +
               (bu[2] - bl[2]) * (R.d3 * id3));

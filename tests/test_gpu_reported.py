@@ -85,3 +85,31 @@ def test_cells_without_a_signal_speed_set_no_time_step(b, prec):
         dt.append(inst.stats()["dt0"])
         inst.close()
     assert dt[0] == dt[1]
+
+
+@pytest.mark.parametrize("rho,p", [(1.0, -0.5), (-1.0, 1.0), (-1.0, -0.5), (0.0, 1.0), (-1e-4, -1.0)])
+@pytest.mark.parametrize("b", [0.0, 0.3, 30.0])
+def test_the_device_states_step_is_the_instances(b, rho, p):
+    """gop_cfl_dt_noalloc skips and counts the cells that gop_prepare does (-rho and
+    -p without a field have the speed of rho and p).  Tolerance: some twenty
+    roundings of 1.1e-16 on either side."""
+    import ctypes as C
+
+    import gop
+    import torch
+
+    W, B = _state(1.0, 1.0, b)
+    W[(0,) + PATCH], W[(4,) + PATCH] = rho, p
+    inst = gop.Instance(N3, *[gop.grid_uniform(m, 0.0, 1.0) for m in N3])
+    inst.upload(W, B)
+    inst.prepare()
+    L = gop.lib()
+    L.gop_cfl_dt_noalloc.argtypes = [C.POINTER(gop.Desc)] + [C.c_void_p] * 6
+    dev = [torch.from_numpy(a).cuda() for a in (W, B)]
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    assert L.gop_cfl_dt_noalloc(C.byref(inst.desc), *[C.c_void_p(t.data_ptr()) for t in dev], None, None,
+                                C.c_void_p(out.data_ptr()),
+                                C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    dt0 = inst.stats()["dt0"]
+    inst.close()
+    assert abs(float(out[0]) - dt0) <= 1e-14 * dt0

@@ -146,8 +146,8 @@ __device__ __forceinline__ void cell_rate_divb(const Args& A, size_t c, size_t s
   // zero or the pressure below it (but for both below without a field), as the
   // roots of the separate terms give
   const double b2 = m1 * m1 + m2 * m2 + m3 * m3, r = A.ca2m * rho, q = fma(A.ca2m, rho, b2 * A.ca2s);
-  const double num = A.gamma * p * q + b2 * r, den = rho * q;
-  double f = num == 0.0 ? 0.0 : num * rsqrt(num * den);
+  const double num = A.gamma * p * q + b2 * r, t = num * (rho * q);
+  double f = t == 0.0 ? 0.0 : num * rsqrt(t);
   if (!(rho > 0.0 ? p >= 0.0 : rho < 0.0 && p <= 0.0 && b2 == 0.0)) f = nan("");
   rate = (sqrt(u * u + v * v + w * w) + f) * (R.il + R.il3 * id3);
   divb = fabs((bu[0] * R.d1u - bl[0] * R.d1l) + (bu[1] * R.d2u - bl[1] * R.d2l) +

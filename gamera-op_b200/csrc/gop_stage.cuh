@@ -32,9 +32,11 @@ __device__ __forceinline__ double max2(double a, double b) { return a > b || b !
 
 // sqrt(n / d) for n, d > 0 (zero for n = 0) as n rsqrt(n d): one special
 // function where the division and the root take two of about 25 instructions
-// each
+// each.  Zero too where n d underflows (the field far from a field loop is
+// 1e-160 and less, its square next to nothing).
 __device__ __forceinline__ double sqrt_ratio(double n, double d) {
-  return n == 0.0 ? 0.0 : n * rsqrt(n * d);
+  const double t = n * d;
+  return t == 0.0 ? 0.0 : n * rsqrt(t);
 }
 
 // The upper word of a density that is zero, negative, infinite or no number

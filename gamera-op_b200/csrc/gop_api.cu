@@ -372,7 +372,8 @@ namespace {
 // milliseconds, a quarter of a small request's whole time (64^3 mixed on B200:
 // create 4.0 -> 0.15 ms, destroy 1.2 -> 0.06 ms).  Beyond that much freed
 // memory goes back to the device at the next synchronisation, and all of it
-// when an allocation fails.  The pool is ordered by streams and safe from any
+// when an allocation of the library's fails or gop_release_memory asks for it
+// (for the other allocators of the process and of the device).  The pool is ordered by streams and safe from any
 // thread.
 constexpr uint64_t kPoolKeep = 2ull << 30;
 std::mutex g_pool_mu;
@@ -823,6 +824,20 @@ int gop_destroy(gop_instance* h) {
   prof_collect(h);
   for (cudaEvent_t e : h->pool) cudaEventDestroy(e);
   delete h;
+  return GOP_OK;
+}
+
+int gop_release_memory(void) {
+  int dev = 0;
+  cudaMemPool_t pool = nullptr;
+  CK(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (dev >= 0 && dev < 64) pool = g_pool[dev];
+  }
+  if (!pool) return GOP_OK;
+  CK(cudaDeviceSynchronize());  // what has been freed on a stream is free now
+  CK(cudaMemPoolTrimTo(pool, 0));
   return GOP_OK;
 }
 

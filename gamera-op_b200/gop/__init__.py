@@ -135,6 +135,12 @@ def fp64_peak_tflops(stream_ptr=None) -> float:
     return v.value
 
 
+def release_memory():
+    """Gives the memory kept of closed instances back to the device
+    (gop_release_memory)."""
+    _check(lib().gop_release_memory())
+
+
 def kernel_launches() -> int:
     return int(lib().gop_kernel_launches())
 

@@ -104,6 +104,13 @@ typedef struct gop_instance gop_instance;
 int gop_create(const gop_desc *desc, gop_instance **out);
 int gop_destroy(gop_instance *h);
 
+/* Gives back to the current device what the library keeps of freed instances
+ * (up to 2 GiB a device, so that the next gop_create need not map memory anew):
+ * for a host whose other allocations, or another process, want it.  Waits for
+ * the device's work.  The library does the same by itself when one of its own
+ * allocations fails. */
+int gop_release_memory(void);
+
 /* Device bytes gop_create would allocate for desc (admission control). */
 size_t gop_footprint(const gop_desc *desc);
 

@@ -1045,6 +1045,12 @@ static const dim3 kBlockCandidates[] = {dim3(32, 4, 2), dim3(32, 8, 1), dim3(32,
                                         dim3(8, 32, 1),  dim3(8, 4, 8)};
 static const int kNumBlockCandidates = sizeof(kBlockCandidates) / sizeof(kBlockCandidates[0]);
 
+// the update of this grid may run from tiles
+static bool update_tiles_apply(const gop_instance* h) {
+  return h->d.precision == GOP_PREC_MIXED ? update_sweep_applies<float>(h->sweep, h->P)
+                                          : update_sweep_applies<double>(h->sweep, h->P);
+}
+
 // one step's launches: the stages, the ghost fill with the turn to the next
 // step (the begin and end groups hold no launch of their own)
 static void enqueue_one_step(gop_instance* h, cudaStream_t st, const Hook& hook) {
@@ -1283,6 +1289,17 @@ int gop_autotune(gop_instance* h, int reps, int* chosen) {
     if (*sweep)
       for (int d = 0; d < 3; d++) pick[first + d] = ncand;
   }
+  // the update: the per-cell launch with its shape or the tiles, where they apply
+  if (update_tiles_apply(h)) {
+    float t_point = 0.f, t_tiles = 0.f;
+    CK(timed([&] { launch_point(K_UPDATE, h->tune.blk[K_UPDATE]); }, &t_point));
+    CK(timed([&] {
+      if (mixed) launch_update_sweep<float>(h->sweep, P, h->wf, h->st);
+      else launch_update_sweep<double>(h->sweep, P, h->wd, h->st);
+    }, &t_tiles));
+    h->tune.update_sweep = t_tiles < t_point;
+    if (h->tune.update_sweep) pick[K_UPDATE] = ncand;
+  }
   if (chosen)
     for (int t = 0; t < NTUNE; t++) chosen[t] = pick[t];
   drop_step_graph(h);  // the captured step has the old shapes
@@ -1492,7 +1509,7 @@ static int batch_build(gop_batch* b) {
 static int batch_pick_sweeps(gop_batch* b) {
   bool any = false;
   for (gop_instance* h : b->m)
-    any = any || h->tune.flux_sweep || h->tune.emf_sweep;
+    any = any || h->tune.flux_sweep || h->tune.emf_sweep || (h->tune.update_sweep && update_tiles_apply(h));
   if (!any || !b->graph) return GOP_OK;
   const size_t nm = b->m.size();
   std::vector<double*> saved(nm, nullptr);

@@ -70,6 +70,8 @@ bool launch_emf_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, con
 // the update from TMA-filled tiles; false as above, on small grids, and on
 // spherical ones with the pole ring average or on the mixed path
 template <typename R>
+bool update_sweep_applies(const SweepSet* sw, const Params& P);
+template <typename R>
 bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st);
 
 // points covered by the launch of one slot (x, y, z extents); none for K_C2C0..2,

@@ -1167,11 +1167,14 @@ static void launch_update_c(const SweepSet* sw, const Params& P, const Work<R>& 
   launch_persistent<UpdSweep<R, BG, COORD>, R>(k_update_sweep<R, BG, COORD>, sw, P, w, sw->upd, order, st);
 }
 template <typename R>
-bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
+bool update_sweep_applies(const SweepSet* sw, const Params& P) {
   if (!sw || P.ps_live || P.ring || (P.coord != 0 && sizeof(R) == 4)) return false;
   const int* nt = sw->upd.m[0].nt;
-  if ((long long)nt[0] * nt[1] * nt[2] < (long long)upd_tiles<R>() * sw->sms * UpdSweep<R, false, 0>::CTAS)
-    return false;
+  return (long long)nt[0] * nt[1] * nt[2] >= (long long)upd_tiles<R>() * sw->sms * UpdSweep<R, false, 0>::CTAS;
+}
+template <typename R>
+bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, cudaStream_t st) {
+  if (!update_sweep_applies<R>(sw, P)) return false;
   const bool bg = P.bg != nullptr;
   if (P.coord == 0) bg ? launch_update_c<R, true, 0>(sw, P, w, st) : launch_update_c<R, false, 0>(sw, P, w, st);
   else if constexpr (sizeof(R) == 8)
@@ -1179,6 +1182,7 @@ bool launch_update_sweep(const SweepSet* sw, const Params& P, const Work<R>& w, 
   return true;
 }
 #define GOP_INST(R)                                                                            \
+  template bool update_sweep_applies<R>(const SweepSet*, const Params&);                        \
   template bool launch_update_sweep<R>(const SweepSet*, const Params&, const Work<R>&, cudaStream_t); \
   template bool launch_flux_sweep<R>(const SweepSet*, const Params&, const Work<R>&,            \
                                      const int[3], cudaStream_t);                     \

@@ -161,7 +161,8 @@ int gop_get_stats(gop_instance *h, gop_stats *out);
  * tunable launches of a step on the instance's current state (after
  * gop_prepare; the state is not advanced) and keeps the fastest for the
  * following steps, and for the flux and the edge-EMF stage the tile-staged
- * sweep where that beats their three launches; then the order of the axes in
+ * sweep where that beats their three launches, for the update of a grid large
+ * enough its tiles where they beat the per-cell launch; then the order of the axes in
  * the flux stage and in the edge-EMF stage (each order a rotation of the axes;
  * they are independent, so no result changes), timing two whole steps per
  * rotation with the state restored after each.  reps: timed launches per
@@ -169,7 +170,7 @@ int gop_get_stats(gop_instance *h, gop_stats *out);
  * candidate index per launch (0 for the three centre-to-edge entries, which
  * are one launch of a fixed shape). */
 #define GOP_NTUNE 11
-#define GOP_TUNE_SWEEP 14 /* chosen[] value of a flux or EMF launch: the tile-staged sweep kernel */
+#define GOP_TUNE_SWEEP 14 /* chosen[] value of a flux, EMF or update launch: the tile-staged kernel */
 int gop_autotune(gop_instance *h, int reps, int *chosen);
 /* The launch orders the autotuner picked (axes, 3 ints each; may be NULL). */
 int gop_get_launch_order(gop_instance *h, int *flux_order, int *emf_order);
@@ -177,8 +178,9 @@ int gop_get_launch_order(gop_instance *h, int *flux_order, int *emf_order);
 /* Kernel choice for the face fluxes and edge EMFs: on (the default) runs
  * the tile-staged sweep kernels (shared-memory tiles filled by the Tensor
  * Memory Accelerator, persistent blocks) wherever they apply, and the update
- * in the same form on grids large enough, off the per-point kernels; both give the same results.  With the entropy channel
- * live the per-face flux kernels always run.  GOP_ENODEV if the sweep
+ * in the same form on grids large enough, off the per-point kernels; both
+ * give the same results, to a multiply-add contracted differently.  With the
+ * entropy channel live the per-face flux kernels always run.  GOP_ENODEV if the sweep
  * kernels could not be set up for this instance. */
 int gop_set_sweep(gop_instance *h, int on);
 
@@ -364,7 +366,7 @@ int gop_batch_set_stream(gop_batch *b, void *stream);
  * member of each class of equal grid shape, geometry and precision, copied
  * to the rest of the class, then captures the batch graph again; then
  * times replays of the batch step with those picks and with every member
- * on the per-point flux and EMF kernels (the tile-staged sweeps, picked
+ * on the per-point flux, EMF and update kernels (the tile-staged sweeps, picked
  * with each grid alone, share the SMs with the other members' kernels in
  * a batch) and keeps the faster (skipped without device memory for a copy
  * of every member's state).  chosen[GOP_NTUNE] (may be NULL) receives the

@@ -649,6 +649,8 @@ int gop_create(const gop_desc* desc, gop_instance** out) {
   *out = nullptr;
   int rc = check_desc(desc);
   if (rc) return rc;
+  if (layout_of(desc).fs >= kMaxField)
+    return fail(GOP_ENOMEM, "a field of %lld points exceeds the kernels' 32-bit offsets", layout_of(desc).fs);
   int dev = 0, count = 0;
   if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0)
     return fail(GOP_ENODEV, "no CUDA device");

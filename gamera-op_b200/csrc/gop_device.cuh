@@ -137,8 +137,9 @@ __device__ __forceinline__ long long lin(const Params& P, int i, int j, int k) {
   return (long long)k * P.sk + (long long)j * P.sj + i;
 }
 
-// the same in 32 bits: a field has fewer than 2^29 points (an instance holds
-// at least 432 bytes per point, so one of 2^29 would not fit a GPU of 232 GB)
+// the same in 32 bits: a field has fewer than 2^29 points (gop_create refuses
+// more: at 432 bytes per point and up an instance would hold 232 GB)
+constexpr long long kMaxField = 1LL << 29;
 __device__ __forceinline__ int lin32(const Params& P, int i, int j, int k) {
   return (k * P.N[1] + j) * P.pitch + i;
 }

@@ -59,7 +59,7 @@ int cudaDeviceSynchronize(void) { return 0; }
 int cudaMemPoolTrimTo(void *p, size_t n) { (void)n; note("trim", p, 0); return 0; }
 int cudaMallocFromPoolAsync(void **p, size_t n, void *pool, void *st) {
   (void)pool; (void)st;
-  *p = calloc(1, n);
+  *p = calloc(1, n >> 32 ? 16 : n); /* (a block of 4 GiB and more is never touched) */
   blocks[nblocks].p = *p;
   blocks[nblocks++].n = n;
   return *p ? 0 : 2;

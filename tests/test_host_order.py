@@ -155,3 +155,19 @@ def test_prepare_clears_what_a_failed_step_left(fake, restart):
         """, names=[sc[k] for k in ("S_STOP", "S_STEPS", "S_FLAGS", "S_PAR", "S_TILE")], count=sc["NSCAL"],
         restart=restart)
     assert left == [0.0] * 5
+
+
+@pytest.mark.parametrize("n,code", [((1000, 1000, 500), 0), ((1000, 1000, 540), -12), ((1280, 1280, 1280), -12),
+                                    ((4, 4, 2**25), -12)])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_fields_beyond_the_kernels_offsets_are_refused(fake, n, code, prec):
+    """The kernels index a field by 32-bit byte offsets: 2^29 points, ghosts and row
+    padding included, are too many, on a GPU with any memory."""
+    got = _run(fake, """
+        try:
+            gop.Instance(A["n"], *[np.linspace(1.0, 2.0, m + 9) for m in A["n"]], precision=A["prec"])
+            out = 0
+        except gop.GopError as e:
+            out = e.code
+        """, n=n, prec=prec)
+    assert got == code

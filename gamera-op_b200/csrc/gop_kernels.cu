@@ -92,7 +92,7 @@ __device__ __forceinline__ void begin_body(const Params& P) {
   }
   s[S_BUDGET] = s[S_BUDGET] - 1.0;
   const double dt = s[S_NEXT_DT];
-  if (!(dt > 0.0) || !isfinite(dt)) flag_numeric(P);
+  if ((!(dt > 0.0) || !isfinite(dt)) && s[S_FLAGS] == 0.0) s[S_FLAGS] = 1.0;  // (one thread: no atomic)
   s[S_DT] = dt;
   s[S_TIME] = s[S_TIME] + dt;
   s[S_CAB2] = 0.5 * dt / s[S_DT0];

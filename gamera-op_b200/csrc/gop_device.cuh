@@ -315,10 +315,11 @@ __device__ __forceinline__ bool is_zero(double x) {
 // below, ordered for the left state and not for the right one.
 // On B200, blast 256^3 FP64: flux stage 3.09 -> 2.56, EMF stage 1.88 -> 1.72 ms
 // per step.
-// POLE (faces along axis 1): the theta face on a pole has no area, its limiter
-// coefficients are infinite and q is, or is no number: nothing is taken off
-// then, whatever the signs (sgn dm + s1 = 0 times infinity is no number
-// either), and the state is the value held between l1 and l2.
+// POLE (faces along axis 1, one of which may lie on a pole): the theta face on
+// a pole has no area, the limiter's coefficients there are infinite and q is, or
+// is no number: nothing is taken off then, whatever the signs (sgn dm + s1 = 0
+// times infinity is no number either), and the state is the value held between
+// l1 and l2.
 template <bool RIGHT, bool POLE>
 __device__ __forceinline__ double pdm_side(double fi, double near, double opp, double d, double d1,
                                            bool neg, double ag) {
@@ -338,7 +339,7 @@ __device__ __forceinline__ double pdm_side(double fi, double near, double opp, d
   const bool beyond = RIGHT ? !(fi < bound) == neg : (fi <= bound) == neg;
   return off ? near : (beyond ? bound : fi);
 }
-template <int AXIS>
+template <bool POLE>
 __device__ __forceinline__ void recon_lr(const double v[8], const double lim[4],
                                          const FaceWeights<double>& W, double& L, double& Rr) {
   const double dm = lim[1] - lim[0], d1 = lim[2] - lim[1], dp = lim[3] - lim[2];
@@ -349,8 +350,8 @@ __device__ __forceinline__ void recon_lr(const double v[8], const double lim[4],
     fl = fma(v[t], W.wl[t], fl);
     fr = fma(v[7 - t], W.wr[t], fr);
   }
-  L = pdm_side<false, AXIS == 1>(fl, lim[1], lim[2], dm, d1, neg, W.cl1 * lim[1] + W.cl2 * lim[0]);
-  Rr = pdm_side<true, AXIS == 1>(fr, lim[2], lim[1], dp, d1, neg, W.cr1 * lim[2] + W.cr2 * lim[3]);
+  L = pdm_side<false, POLE>(fl, lim[1], lim[2], dm, d1, neg, W.cl1 * lim[1] + W.cl2 * lim[0]);
+  Rr = pdm_side<true, POLE>(fr, lim[2], lim[1], dp, d1, neg, W.cr1 * lim[2] + W.cr2 * lim[3]);
 }
 
 // FP32: min and max are one instruction each, and every rounding is the
@@ -364,7 +365,7 @@ __device__ __forceinline__ float pdm_limit(float fi, float near, float hi, float
   const float w = d == 0.0f ? 0.5f : (other ? 0.0f : 1.0f);
   return fmaf(-s, fmaxf(0.0f, fabsf(f - near) - w * q2), f);
 }
-template <int AXIS>
+template <bool POLE>
 __device__ __forceinline__ void recon_lr(const float v[8], const float lim[4],
                                          const FaceWeights<float>& W, float& L, float& Rr) {
   const float dm = lim[1] - lim[0], d1 = lim[2] - lim[1], dp = lim[3] - lim[2];

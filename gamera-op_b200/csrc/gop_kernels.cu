@@ -214,7 +214,7 @@ __device__ __forceinline__ void c2c_body(const Params& P, const Work<R>& wk, Pos
     line8<R, R>(wk.Wh + (size_t)(V1 + comp) * fs + x, s, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = W[(V1 + comp) * fs + (u - 2) * s];
-    recon_lr<p>(v, lim, Wt, L, Rr);
+    recon_lr<p == 1>(v, lim, Wt, L, Rr);
     wk.V[x + (size_t)(2 * D + cc) * fs] = R(0.5) * (L + Rr);
   }
 }
@@ -245,7 +245,7 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
       line8<R, R>(wk.V + (size_t)(2 * D + cc) * fs + x, sq, v);
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = v[u + 2];
-      recon_lr<q>(v, lim, Wt, L, Rr);
+      recon_lr<q == 1>(v, lim, Wt, L, Rr);
       vav[cc] = R(0.5) * (L + Rr);
     }
     // B_p along q
@@ -253,7 +253,7 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
     line8<R, R>(wk.Bh + (size_t)p * fs + x, sq, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = B[p * fs + (u - 2) * sq];
-    recon_lr<q>(v, lim, Wt, bpl, bpr);
+    recon_lr<q == 1>(v, lim, Wt, bpl, bpr);
   }
   {
     // B_q along p
@@ -263,7 +263,7 @@ __device__ __forceinline__ void emf_body(const Params& P, const Work<R>& wk, Pos
     line8<R, R>(wk.Bh + (size_t)q * fs + x, sp, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = B[q * fs + (u - 2) * sp];
-    recon_lr<p>(v, lim, Wt, bql, bqr);
+    recon_lr<p == 1>(v, lim, Wt, bql, bqr);
   }
   R b0p = R(0), b0q = R(0);
   if constexpr (BG) {  // B0 averaged along the edge (B0Aedge*)
@@ -307,7 +307,7 @@ __device__ __forceinline__ void flux_body(const Params& P, const Work<R>& wk, Po
     line8<R, R>(wk.Wh + (size_t)m * fs + x, s, v);
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = W[m * fs + (u - 2) * s];
-    recon_lr<D>(v, lim, Wt, L[m], Rt[m]);
+    recon_lr<D == 1>(v, lim, Wt, L[m], Rt[m]);
   }
 #pragma unroll
   for (int a = 0; a < 3; a++) {
@@ -316,7 +316,7 @@ __device__ __forceinline__ void flux_body(const Params& P, const Work<R>& wk, Po
     const R* ms = wk.Ms + (size_t)a * fs + x;
 #pragma unroll
     for (int u = 0; u < 4; u++) lim[u] = ms[(u - 2) * s];
-    recon_lr<D>(v, lim, Wt, mL[a], mR[a]);
+    recon_lr<D == 1>(v, lim, Wt, mL[a], mR[a]);
   }
   flux_out<R, D, BG, PSL>(P, wk, (int)x, D == 0 ? j : (D == 1 ? k : i), L, Rt, mL, mR,
                           lim_b<R>(P, wk)[x + D * fs]);

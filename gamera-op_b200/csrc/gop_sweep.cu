@@ -26,7 +26,8 @@
 // So the global-memory latency of tile n+1 overlaps the arithmetic of tile
 // n, and the stencil re-reads come from shared memory instead of L1.  The
 // per-point arithmetic is the per-point kernels' own (recon_lr, flux_out,
-// emf_finish), in the same order, so both forms give the same bits.
+// emf_finish), in the same order, so both forms give the same results (to a
+// multiply-add the compiler contracts in one and not in the other).
 //
 // Lanes always run along i (x, the TMA box's contiguous axis); a tile is 32
 // lanes x 8 or 16 rows, a warp's row along the stage's sweep axis or its
@@ -218,7 +219,7 @@ struct Gather {
   double rate = 0.0, divb = 0.0;
 };
 
-template <typename R, int D, bool BG>
+template <typename R, int D, bool BG, bool POLE>
 struct FluxStage {
   using F = FluxTile<D>;
   using Maps = FluxMaps;
@@ -280,7 +281,7 @@ struct FluxStage {
       for (int u = 0; u < 8; u++) v[u] = wh[f * F::SB + u * TS];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = wl[f * F::LB + u * TS];
-      recon_lr<D>(v, lim, Wt, L[f], Rt[f]);
+      recon_lr<POLE && D == 1>(v, lim, Wt, L[f], Rt[f]);
     }
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -289,7 +290,7 @@ struct FluxStage {
       for (int u = 0; u < 8; u++) v[u] = msh[a * F::SB + u * TS];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = ms[a * F::LB + u * TS];
-      recon_lr<D>(v, lim, Wt, mL[a], mR[a]);
+      recon_lr<POLE && D == 1>(v, lim, Wt, mL[a], mR[a]);
     }
     flux_out<R, D, BG, false>(P, wk, lin32(P, i, j, k), D == 0 ? j : (D == 1 ? k : i), L, Rt, mL, mR,
                               bn);
@@ -351,7 +352,7 @@ struct alignas(64) EmfMaps {
   uint64_t inv[2];
 };
 
-template <typename R, int D, bool BG>
+template <typename R, int D, bool BG, bool POLE>
 struct EmfStage {
   using E = EmfTile<D>;
   using Maps = EmfMaps;
@@ -453,7 +454,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = v0[cc * E::VF + u * tq];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = v[u + 2];
-      recon_lr<q>(v, lim, Wq, L, Rr);
+      recon_lr<POLE && q == 1>(v, lim, Wq, L, Rr);
       vav[cc] = R(0.5) * (L + Rr);
     }
     {  // B_p along q
@@ -462,7 +463,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = bp[u * tq];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = bpl[u * tq];
-      recon_lr<q>(v, lim, Wq, bpL, bpR);
+      recon_lr<POLE && q == 1>(v, lim, Wq, bpL, bpR);
     }
     {  // B_q along p
       R v[8], lim[4];
@@ -470,7 +471,7 @@ struct EmfStage {
       for (int u = 0; u < 8; u++) v[u] = bq[u * tp];
 #pragma unroll
       for (int u = 0; u < 4; u++) lim[u] = bql[u * tp];
-      recon_lr<p>(v, lim, Wp, bqL, bqR);
+      recon_lr<POLE && p == 1>(v, lim, Wp, bqL, bqR);
     }
     const int x = lin32(P, i, j, k);
     const size_t fs = P.fs;
@@ -488,14 +489,16 @@ struct EmfStage {
 
 // A stage's three sweeps as one launch: the stage of each axis, their tensor
 // maps, and the order in which the axes' tiles are taken.
-// MASK: the axes it is compiled for (bit d).
-template <typename R, bool EMF_, bool BG, unsigned MASK_>
+// MASK: the axes it is compiled for (bit d).  POLE: with the look at pole faces
+// (recon_lr), for grids with the pole ring average alone: those without have no
+// face without an area, and it costs the FP64 flux stage 1 to 2 % (128^3 325 -> 329 us).
+template <typename R, bool EMF_, bool BG, unsigned MASK_, bool POLE>
 struct Sweep {
   static constexpr bool EMF = EMF_, STATE = false;
   static constexpr unsigned MASK = MASK_;
   static constexpr bool H0 = MASK & 1, H1 = MASK >> 1 & 1, H2 = MASK >> 2 & 1;
   template <int D>
-  using Stage = typename std::conditional<EMF, EmfStage<R, D, BG>, FluxStage<R, D, BG>>::type;
+  using Stage = typename std::conditional<EMF, EmfStage<R, D, BG, POLE>, FluxStage<R, D, BG, POLE>>::type;
   using Maps = typename Stage<0>::Maps;
   static constexpr int max3(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
   // a slot holds the tile of any axis
@@ -686,13 +689,13 @@ __device__ __forceinline__ void sweep_run(const Params& P, const Work<R>& wk,
   if (!ok) P.scal[S_FLAGS] = 2.0;
 }
 
-template <typename R, bool EMF, bool BG, unsigned MASK>
+template <typename R, bool EMF, bool BG, unsigned MASK, bool POLE>
 __global__ void __launch_bounds__(kSweepThreads, (SweepCfg<R, EMF>::CTAS))
     k_sweep(Params P, Work<R> wk,
-            const __grid_constant__ SweepMaps<typename Sweep<R, EMF, BG, MASK>::Maps> maps) {
+            const __grid_constant__ SweepMaps<typename Sweep<R, EMF, BG, MASK, POLE>::Maps> maps) {
   pdl_enter();
   Gather none;
-  sweep_run<Sweep<R, EMF, BG, MASK>, R>(P, wk, maps, none);
+  sweep_run<Sweep<R, EMF, BG, MASK, POLE>, R>(P, wk, maps, none);
 }
 
 // ---------------------------------------------------------------- update
@@ -876,8 +879,8 @@ __global__ void __launch_bounds__(kSweepThreads, (UpdSweep<R, BG, COORD>::CTAS))
 
 template <typename R, unsigned MASK>
 constexpr bool smem_fits() {
-  using F = Sweep<R, false, false, MASK>;
-  using E = Sweep<R, true, false, MASK>;
+  using F = Sweep<R, false, false, MASK, false>;
+  using E = Sweep<R, true, false, MASK, false>;
   return (F::SMEM + 1024) * F::CTAS <= 228 * 1024 && (E::SMEM + 1024) * E::CTAS <= 228 * 1024;
 }
 static_assert(smem_fits<double, 7>() && smem_fits<double, 1>(), "FP64 sweep blocks per SM");
@@ -1040,10 +1043,16 @@ struct SweepSet {
   int sms = 0;
 };
 
+// the kernels that may have a face on a pole to look at
+template <typename R, unsigned MASK>
+constexpr bool kPole = sizeof(R) == 8 && (MASK >> 1 & 1);
 template <typename R, bool EMF, bool BG, unsigned MASK>
 static bool allow_smem() {
-  return cudaFuncSetAttribute(k_sweep<R, EMF, BG, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              Sweep<R, EMF, BG, MASK>::SMEM) == cudaSuccess;
+  constexpr bool pole = kPole<R, MASK>;
+  return cudaFuncSetAttribute(k_sweep<R, EMF, BG, MASK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              Sweep<R, EMF, BG, MASK, false>::SMEM) == cudaSuccess &&
+         (!pole || cudaFuncSetAttribute(k_sweep<R, EMF, BG, MASK, pole>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        Sweep<R, EMF, BG, MASK, pole>::SMEM) == cudaSuccess);
 }
 template <typename R, bool BG>
 static bool allow_smem() {
@@ -1107,7 +1116,11 @@ static void launch_persistent(K kern, const SweepSet* sw, const Params& P, const
 template <typename R, bool EMF, bool BG, unsigned MASK, class Maps>
 static void launch_mask(const SweepSet* sw, const Params& P, const Work<R>& w, const Maps& m,
                         const int order[3], cudaStream_t st) {
-  launch_persistent<Sweep<R, EMF, BG, MASK>, R>(k_sweep<R, EMF, BG, MASK>, sw, P, w, m, order, st);
+  constexpr bool pole = kPole<R, MASK>;
+  if (pole && P.ring)
+    launch_persistent<Sweep<R, EMF, BG, MASK, pole>, R>(k_sweep<R, EMF, BG, MASK, pole>, sw, P, w, m, order, st);
+  else
+    launch_persistent<Sweep<R, EMF, BG, MASK, false>, R>(k_sweep<R, EMF, BG, MASK, false>, sw, P, w, m, order, st);
 }
 // The axes of a stage in one launch, or (flux) one launch each where each
 // axis alone keeps the GPU busy for long: the kernels of one axis are about 3 %

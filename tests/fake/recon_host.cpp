@@ -30,7 +30,7 @@ static void lines(int n, const double* v, const double* lim, const double* w, do
     for (int t = 0; t < 4; t++) b[t] = (R)lim[t];
     for (int t = 0; t < 7; t++) W.wl[t] = (R)w[t], W.wr[t] = (R)w[7 + t];
     W.set_limiter((R)w[14], (R)w[15], (R)w[16], (R)w[17]);
-    gop::recon_lr<RECON_AXIS>(a, b, W, L, Rr);
+    gop::recon_lr<RECON_AXIS == 1>(a, b, W, L, Rr);
     out[0] = L, out[1] = Rr;
   }
 }

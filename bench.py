@@ -41,6 +41,8 @@ REF_BUDGET_S = 120  # seconds of timed steps the reference arm may spend
 # directions a group covers per step: the bytes and times below are of one
 # direction (the three go out in one launch or three, by stage and grid)
 GROUP_LAUNCHES = {"ab2": 1, "c2c": 3, "emf": 3, "flux": 3, "update": 1}
+# the kernel a group's time is spent in on a large grid
+GROUP_KERNEL = {"ab2": "k_ab2", "c2c": "k_c2c", "emf": "k_sweep", "flux": "k_sweep", "update": "k_update_sweep"}
 # thread-block shapes the library's autotuner chooses from (gop_autotune)
 BLOCK_CANDIDATES = ["32x4x2", "32x8x1", "32x1x8", "32x2x4", "64x2x2", "64x4x1", "64x1x4",
                     "128x2x1", "128x1x2", "32x4x1", "64x2x1", "256x1x1", "8x32x1", "8x4x8",
@@ -473,7 +475,7 @@ def main():
                    "launch_order": inst.launch_order()},
         "latency_ms": {"p50": round(float(np.percentile(durs, 50)), 4),
                        "p99": round(float(np.percentile(durs, 99)), 4)},
-        "roofline": {"bound": "hbm", "kernel": f"k_{dom}", "achieved": round(achieved, 2),
+        "roofline": {"bound": "hbm", "kernel": GROUP_KERNEL[dom], "achieved": round(achieved, 2),
                      "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
                      "traffic": tr, "peak_kind": peak_kind,
                      "algorithmic_bytes_per_launch": alg,

@@ -52,7 +52,7 @@ __device__ __forceinline__ double no_number() { return __hiloint2double(0x7ff800
 // FP64: over the common denominator rho (b2 + ca^2 rho) it is one reciprocal
 // root.  The reference's order (src/solver_func.c:1005-1018) takes three
 // roots, a reciprocal root and a division per state.  Blast 256^3 on B200:
-// flux stage 2.56 -> 2.34 ms per step, the EMFs' form of it 1.72 -> 1.58 ms.
+// flux stage 2.56 -> 2.35 ms per step, the EMFs' form of it 1.72 -> 1.58 ms.
 // What decides whether there is a speed is what the separate roots decide by:
 // no number for a negative pressure, however strong the field, nor for a
 // density of zero or below (but for -rho and -p without a field, whose ratio

@@ -1,7 +1,7 @@
 """A restart from an AB2 history whose periodic ghost layers do not repeat its
 active cells (a history kept without its ghosts, say): gop_prepare fills the
 ghosts of the state, not of the history, so the first step takes what was
-uploaded, as the reference does.  Against the checker; and by the launches of a
+uploaded, as the reference does.  Against the oracle; and by the launches of a
 step, that a history with its ghosts filled costs no more than none.
 
 Tolerance: one step takes each value through fewer than a thousand roundings of

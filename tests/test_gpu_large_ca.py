@@ -1,12 +1,12 @@
 """A Boris speed of light far above every signal (no limit in effect, as a user
 asks for who wants the plain Alfven speed).
 
-Against the checker, which evaluates the reference's separate roots, on Cartesian
+Against the oracle, which evaluates the reference's separate roots, on Cartesian
 grids: the state after two steps, their time, and the CFL step of the same state in
 device memory.  Tolerance: as for one step of states without ties (fewer than a
 thousand roundings of 1.1e-16, amplified less than tenfold: 1e-12 relative L1),
 twice.  (On a spherical grid the limiter jumps where a slope is zero, so rough
-states differ from the checker's by more than roundings.)
+states differ from the oracle's by more than roundings.)
 
 Against itself, on either kind of grid: above about 1e20 nothing is left of the
 limit in 53 bits, so powers of two give the same bits."""
@@ -68,7 +68,7 @@ def _run(n, coord, ca, sweep):
 @pytest.mark.parametrize("sweep", [True, False])
 @pytest.mark.parametrize("n", [(16, 12, 9), (64, 56, 64)])
 @pytest.mark.parametrize("ca", [10.0, 1e30, 1e80, 1e100, 1e150])
-def test_as_the_checker(oracle_mod, ca, n, sweep):
+def test_as_the_oracle(oracle_mod, ca, n, sweep):
     xs, W, B = _case(n, 0)
     ref = oracle_mod.Oracle(n, *xs, ca=ca)
     ref.set_state(W, B)

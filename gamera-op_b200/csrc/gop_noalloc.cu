@@ -43,7 +43,7 @@ constexpr int kThreads = 256;
 struct Args {
   int n[3], N[3];
   int sph;
-  double gamma, cfl;
+  double gamma, cfl, ca;
   double ca2m, ca2s;  // ca^2 = ca2m / ca2s (split_ca2)
   const double* gas;  // [6][NI][NJ][NK], k fastest (reference layout)
   const double* fb;   // [3][NI][NJ][NK]
@@ -142,13 +142,16 @@ __device__ __forceinline__ void cell_rate_divb(const Args& A, size_t c, size_t s
     bu[2] += f2[1];
   }
   // |v| + sqrt(cs^2 + va^2) with va^2 = v^2 ca^2 / (v^2 + ca^2), v^2 = b^2 /
-  // rho, over the common denominator; no number where the density is not above
-  // zero or the pressure below it (but for both below without a field), as the
-  // roots of the separate terms give
+  // rho, over the common denominator; by the separate roots (which decide whether
+  // there is a speed) where the density or the pressure is not above zero or
+  // the product leaves the range of a double
   const double b2 = m1 * m1 + m2 * m2 + m3 * m3, r = A.ca2m * rho, q = fma(A.ca2m, rho, b2 * A.ca2s);
   const double num = A.gamma * p * q + b2 * r, t = num * (rho * q);
-  double f = t == 0.0 ? 0.0 : num * rsqrt(t);
-  if (!(rho > 0.0 ? p >= 0.0 : rho < 0.0 && p <= 0.0 && b2 == 0.0)) f = nan("");
+  double f = num * rsqrt(t);
+  if (!(t >= DBL_MIN && t <= DBL_MAX && rho > 0.0 && p >= 0.0)) {
+    const double vs = sqrt(A.gamma * p / rho), va = sqrt(b2 / rho), ve = va * A.ca / sqrt(va * va + A.ca * A.ca);
+    f = sqrt(vs * vs + ve * ve);
+  }
   rate = (sqrt(u * u + v * v + w * w) + f) * (R.il + R.il3 * id3);
   divb = fabs((bu[0] * R.d1u - bl[0] * R.d1l) + (bu[1] * R.d2u - bl[1] * R.d2l) +
               (bu[2] - bl[2]) * (R.d3 * id3));
@@ -299,7 +302,8 @@ extern "C" int gop_cfl_dt_noalloc(const gop_desc* desc, const double* gas, const
   A.sph = desc->coord == GOP_COORD_SPHERICAL;
   A.gamma = desc->gamma != 0 ? desc->gamma : 5.0 / 3.0;
   A.cfl = desc->cfl != 0 ? desc->cfl : 0.3;
-  gop::split_ca2(desc->ca != 0 ? desc->ca : 10.0, A.ca2m, A.ca2s);
+  A.ca = desc->ca != 0 ? desc->ca : 10.0;
+  gop::split_ca2(A.ca, A.ca2m, A.ca2s);
   A.gas = gas;
   A.fb = face_b;
   A.b0 = b0;

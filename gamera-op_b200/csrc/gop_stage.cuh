@@ -30,22 +30,27 @@ __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
 // comparison and a select, where fmax(double) is twice that)
 __device__ __forceinline__ double max2(double a, double b) { return a > b || b != b ? a : b; }
 
-// sqrt(n / d) for n, d > 0 (zero for n = 0) as n rsqrt(n d): one special
-// function where the division and the root take two of about 25 instructions
-// each.  Zero too where n d underflows (the field far from a field loop is
-// 1e-160 and less, its square next to nothing).
-__device__ __forceinline__ double sqrt_ratio(double n, double d) {
-  const double t = n * d;
-  return t == 0.0 ? 0.0 : n * rsqrt(t);
-}
+// Speeds over a common denominator: sqrt(n / d) for n, d > 0 as n rsqrt(n d), one
+// special function where the division and the root take two of about 25
+// instructions each.  What is out of the ordinary -- a density or pressure not
+// above zero, infinite or no number, a product n d that leaves the range of a
+// double -- goes to the reference's separate roots, in a branch that is as good as
+// never taken.
 
-// The upper word of a density that is zero, negative, infinite or no number
-// (one comparison: below zero wraps round), where a speed over a common
-// denominator may have a value that the reference's separate roots do not have
+// a product that is zero, subnormal, infinite, negative or no number (one
+// comparison of the upper word: below the least normal it wraps round)
+__device__ __forceinline__ bool odd_product(double t) {
+  return (unsigned)(__double2hiint(t) - 0x00100000) >= 0x7fe00000u;
+}
+// a density that is zero, negative, infinite or no number
 __device__ __forceinline__ bool odd_density(double rho) {
   return (unsigned)(__double2hiint(rho) - 1) >= 0x7fefffffu;
 }
-__device__ __forceinline__ double no_number() { return __hiloint2double(0x7ff80000, 0); }
+// the Boris-limited Alfven speed of sqrt(v2), v2 = b^2 / rho
+__device__ __forceinline__ double alfven_apart(const Params& P, double v2) {
+  const double va = sqrt(v2);
+  return va * P.ca * rsqrt(va * va + P.ca2);
+}
 
 // Fast magnetosonic speed sqrt(cs^2 + va^2) with the Boris-limited Alfven
 // speed va^2 = v^2 ca^2 / (v^2 + ca^2), v^2 = b2 / rho, from gp = gamma p, in
@@ -53,15 +58,15 @@ __device__ __forceinline__ double no_number() { return __hiloint2double(0x7ff800
 // root.  The reference's order (src/solver_func.c:1005-1018) takes three
 // roots, a reciprocal root and a division per state.  Blast 256^3 on B200:
 // flux stage 2.56 -> 2.35 ms per step, the EMFs' form of it 1.72 -> 1.58 ms.
-// What decides whether there is a speed is what the separate roots decide by:
-// no number for a negative pressure, however strong the field, nor for a
-// density of zero or below (but for -rho and -p without a field, whose ratio
-// is that of rho and p).
 __device__ __forceinline__ double fast_speed(const Params& P, double gp, double rho, double b2) {
   const double r = P.ca2m * rho, q = fma(b2, P.ca2s, r);
-  double v = sqrt_ratio(gp * q + b2 * r, rho * q);
-  if (odd_density(rho) || __double2hiint(gp) < 0)
-    if (!(rho > 0.0 ? gp >= 0.0 : rho < 0.0 && gp <= 0.0 && b2 == 0.0)) v = no_number();
+  const double n = gp * q + b2 * r, t = n * (rho * q);
+  double v = n * rsqrt(t);
+  // (p < 0 in a strong field, and rho < 0 with it, leave t positive)
+  if (odd_product(t) || (__double2hiint(rho) | __double2hiint(gp)) < 0) {
+    const double ir = 1.0 / rho, cs = sqrt(gp * ir), ve = alfven_apart(P, b2 * ir);
+    v = sqrt(cs * cs + ve * ve);
+  }
   return v;
 }
 
@@ -232,12 +237,13 @@ __device__ __forceinline__ R emf_finish(const Params& P, R vp, R vq, R bpl, R bp
   R e = -(vp * bq - vq * bp);
   R vz;
   if constexpr (sizeof(R) == 8) {
-    // Boris-limited Alfven speed as in fast_speed, cs = 0.  The half-step
-    // densities are extrapolated and may be negative: no speed then, as
-    // sqrt(b^2 / rho) has none, but for b = 0.
+    // Boris-limited Alfven speed as in fast_speed, cs = 0.  (The half-step
+    // densities are extrapolated and may be negative.)  Zero where n d underflows,
+    // as it does without a field and far from a field loop, where b is 1e-160.
     const R b2 = bp * bp + bq * bq;
-    R va = sqrt_ratio(b2 * P.ca2m, fma(R(0.25) * P.ca2m, rho4, b2 * P.ca2s));
-    if (odd_density(rho4) && !(rho4 > 0.0 || (rho4 < 0.0 && b2 == 0.0))) va = no_number();
+    const R n = b2 * P.ca2m, t = n * fma(R(0.25) * P.ca2m, rho4, b2 * P.ca2s);
+    R va = t == R(0) ? R(0) : n * rsq(t);
+    if (odd_density(rho4)) va = alfven_apart(P, b2 / (R(0.25) * rho4));
     vz = va + sqrt(vp * vp + vq * vq);
   } else {
     const R ca = (R)P.ca;

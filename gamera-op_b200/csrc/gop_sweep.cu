@@ -1126,7 +1126,7 @@ static void launch_mask(const SweepSet* sw, const Params& P, const Work<R>& w, c
 // axis alone keeps the GPU busy for long: the kernels of one axis are about 3 %
 // faster per tile (a third of the code, registers left over), which beats the
 // two waves and fills saved from about 128 tiles per resident block on.  Blast
-// on B200, flux stage per step, one launch / three: FP64 128^3 326 / 335 us,
+// on B200, flux stage per step, one launch / three: FP64 128^3 321 / 335 us,
 // 192^3 1048 / 1022, 256^3 2443 / 2350; FP32 216 / 226, 693 / 681, 1616 / 1560.
 // EMF tiles are shorter and gain by the common launch at every size (FP32
 // 128^3 120 / 137, 256^3 854 / 851).

@@ -136,6 +136,13 @@ __device__ __forceinline__ double cfl_cart(const Params& P, const double il[3], 
   return (double)(vc * (T)il[0] + vc * (T)il[1] + vc * (T)il[2]);
 }
 
+// alf = b^2 / (rho ca^2) and perp = 1 / (1 + alf) by one division
+__device__ __forceinline__ void boris(const Params& P, double rho, double bsq, double& alf, double& perp) {
+  const double rc = rho * P.ca2m, bs = bsq * P.ca2s, q = fma(bsq, P.ca2s, rc), t = rc * q, inv = 1.0 / t;
+  alf = bs * q * inv;
+  perp = rc * rc * inv;
+}
+
 // What a cell's update reads, from global memory: the fluxes of its faces,
 // the EMFs of its edges, its face field and its state
 template <typename R>
@@ -308,10 +315,8 @@ __device__ __forceinline__ void update_cart(const Params& P, const Reader& in, i
   {
     const RA bsq = (RA)(mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
     RA alf, perp;
-    if constexpr (sizeof(RA) == 8) {  // b^2 / (rho ca^2) and 1 / (1 + that) by one division
-      const double rc = rho * P.ca2m, bs = bsq * P.ca2s, q = fma(bsq, P.ca2s, rc), inv = 1.0 / (rc * q);
-      alf = bs * q * inv;
-      perp = rc * rc * inv;
+    if constexpr (sizeof(RA) == 8) {
+      boris(P, rho, bsq, alf, perp);
     } else {
       alf = bsq / ((RA)rho * (RA)P.ca2);
       perp = RA(1) / (RA(1) + alf);
@@ -514,10 +519,7 @@ __device__ __forceinline__ void update_sph(const Params& P, const Work<double>& 
   const R mr[3] = {(R)mt[0], (R)mt[1], (R)mt[2]};
   const R bsq = mr[0] * mr[0] + mr[1] * mr[1] + mr[2] * mr[2];
   R alf, perp;
-  // b^2 / (rho ca^2) and 1 / (1 + that) by one division
-  const double rc = rho * P.ca2m, bs = bsq * P.ca2s, q = fma(bsq, P.ca2s, rc), inv = 1.0 / (rc * q);
-  alf = bs * q * inv;
-  perp = rc * rc * inv;
+  boris(P, rho, bsq, alf, perp);
   const R rdt = (R)dt;
   const R drho = -rdt * du[0];
   const R dva = alf * drho;
